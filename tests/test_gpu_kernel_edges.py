@@ -1,0 +1,96 @@
+"""GPU tests of kernels at the sizes where their tiles, chunks and remainders
+begin and end, bit-exact against the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def sg():
+    from synaptogenesis_gb300 import syngen
+    assert syngen.get_gpus(), "no CUDA GPU visible"
+    syngen.set_warnings(False)
+    return syngen
+
+
+def layer(name, model, rows, cols, **more):
+    return dict({"name": name, "neural model": model, "rows": rows, "columns": cols}, **more)
+
+
+def connection(name, source, to, kind, **more):
+    return dict({"name": name, "from layer": source, "to layer": to, "type": kind,
+                 "plastic": False, "opcode": "add", "myelinated": True}, **more)
+
+
+def network(layers, connections):
+    return {"structures": [{"name": "s", "type": "parallel", "layers": layers}],
+            "connections": connections}
+
+
+def run_both(sg, net_dict, inject, steps, keys, learning=False, args=None):
+    """The keys' arrays after ``steps`` on the GPU and on the oracle, started
+    from the same injected arrays; a key is (layer, name) or (connection, name)
+    with a leading "matrix"."""
+    from oracle.oracle import OracleNetwork
+    net, onet = sg.Network(net_dict), OracleNetwork(net_dict)
+    net.build_state()
+
+    def gpu(key):
+        if key[0] == "matrix":
+            return net.get_weight_matrix(key[1], key[2]).to_np_array()
+        return net.get_neuron_data("s", key[0], key[1]).to_np_array()
+
+    def cpu(key):
+        return onet.get_weight_matrix(key[1], key[2]) if key[0] == "matrix" \
+            else onet.get_neuron_data(*key)
+
+    for key, values in inject.items():
+        values = np.asarray(values)
+        for dst in (gpu(key), cpu(key)):
+            assert dst.size == values.size, key
+            dst.view(values.dtype)[:] = values
+    with sg.Engine(net, None, dict({"learning flag": learning}, **(args or {}))) as eng:
+        eng.step(steps)
+    for _ in range(steps):
+        onet.step(learning=learning)
+    return {k: (gpu(k).copy().view(np.uint32), np.asarray(cpu(k)).copy().view(np.uint32))
+            for k in keys}
+
+
+def assert_equal(results):
+    for key, (got, want) in results.items():
+        bad = np.flatnonzero(got != want)
+        assert bad.size == 0, (key, bad.size, bad[:3], got[bad[:3]], want[bad[:3]])
+
+
+# chunks of 256 sources, two in registers and one in shared memory ahead of the
+# one being summed; sums by 16 sources; bands of 8 destinations
+@pytest.mark.parametrize("sources,dests", [
+    (1, 1), (15, 7), (17, 8), (255, 9), (256, 7), (257, 8), (512, 17), (769, 3), (1025, 33), (1281, 5),
+    (40, 4873)])
+@pytest.mark.parametrize("model,delay", [("relay", 0), ("game_of_life", 5)])
+def test_dense_base_activator(sg, sources, dests, model, delay):
+    rng = np.random.default_rng(sources * 7 + dests)
+    net = network([layer("a", model, 1, sources), layer("b", "relay", 1, dests)],
+                  [connection("c", "a", "b", "fully connected", delay=delay, opcode="sub")])
+    words = rng.standard_normal(sources).astype(np.float32).view(np.uint32) if model == "relay" \
+        else rng.integers(0, 2**32, sources, dtype=np.uint64).astype(np.uint32)
+    inject = {("a", "output"): words,
+              ("matrix", "c", "weights"): rng.standard_normal(sources * dests).astype(np.float32)}
+    assert_equal(run_both(sg, net, inject, 1, [("b", "input"), ("b", "output")]))
+
+
+@pytest.mark.parametrize("window", [(0, 1, 0, 1), (1, 12, 2, 13), (3, 20, 1, 16)])
+def test_dense_base_activator_subset(sg, window):
+    rng = np.random.default_rng(sum(window))
+    r0, r1, c0, c1 = window
+    net = network([layer("a", "relay", 20, 17), layer("b", "relay", 20, 17)],
+                  [connection("c", "a", "b", "subset", **{"subset config": {
+                      "from row start": r0, "from row end": r1, "from column start": c0,
+                      "from column end": c1, "to row start": r0, "to row end": r1,
+                      "to column start": c0, "to column end": c1}})])
+    n = ((r1 - r0) * (c1 - c0)) ** 2
+    inject = {("a", "output"): rng.standard_normal(20 * 17).astype(np.float32).view(np.uint32),
+              ("matrix", "c", "weights"): rng.standard_normal(n).astype(np.float32)}
+    assert_equal(run_both(sg, net, inject, 1, [("b", "input")]))
