@@ -94,3 +94,28 @@ def test_dense_base_activator_subset(sg, window):
     inject = {("a", "output"): rng.standard_normal(20 * 17).astype(np.float32).view(np.uint32),
               ("matrix", "c", "weights"): rng.standard_normal(n).astype(np.float32)}
     assert_equal(run_both(sg, net, inject, 1, [("b", "input")]))
+
+
+# 128 source rows a CTA, 4 a thread; bands of 8 destinations
+@pytest.mark.parametrize("sources,dests", [(1, 1), (31, 9), (33, 8), (128, 7), (129, 17), (300, 3)])
+@pytest.mark.parametrize("opcode", ["add", "sub"])
+def test_dense_izhikevich_learning(sg, sources, dests, opcode):
+    rng = np.random.default_rng(sources + dests)
+    n = sources * dests
+    net = network([layer("a", "izhikevich", 1, sources, params="regular"),
+                   layer("b", "izhikevich", 1, dests, params="fast")],
+                  [connection("c", "a", "b", "fully connected", opcode=opcode, plastic=True)])
+    draw = lambda lo, hi, m: rng.uniform(lo, hi, m).astype(np.float32)    # noqa: E731
+    inject = {("a", "output"): rng.integers(0, 2**32, sources, dtype=np.uint64).astype(np.uint32),
+              ("a", "voltage"): draw(-70, 40, sources), ("b", "voltage"): draw(-70, 40, dests),
+              ("b", "post trace"): draw(0, 0.004, dests),
+              ("b", "time since spike"): rng.integers(0, 33, dests).astype(np.int32),
+              ("matrix", "c", "weights"): np.where(rng.random(n) < 0.2, 0, draw(0, 0.5, n)),
+              ("matrix", "c", "presyn trace"): draw(0, 0.004, n),
+              ("matrix", "c", "weight derivatives"): draw(-1e-3, 1e-3, n),
+              ("matrix", "c", "short term R"): draw(0.5, 1, n),
+              ("matrix", "c", "short term w"): draw(0.2, 0.8, n)}
+    inject[("matrix", "c", "weights")] = inject[("matrix", "c", "weights")].astype(np.float32)
+    keys = [("matrix", "c", k) for k in ("weights", "presyn trace", "weight derivatives",
+                                         "short term R", "short term w", "short trace")]
+    assert_equal(run_both(sg, net, inject, 3, keys + [("b", "voltage")], learning=True))
