@@ -98,7 +98,7 @@ struct StepArgs {
 
 // Trace decays of the "add" (AMPA, NMDA) and "sub" (GABA-A, GABA-B) activators.
 constexpr float kAmpaTau = 0.8f, kNmdaTau = 0.993f, kGabaaTau = 0.833f, kGababTau = 0.993f;
-constexpr int kFcUnroll = 4;
+constexpr int kConvUnroll = 8;
 constexpr int kMaxThreads = 256;
 
 // Wrapped coordinate for x in [-n, 2n) (the field is checked against the
@@ -110,7 +110,16 @@ __device__ __forceinline__ float relay_value(const InstDev& I, long long t, int 
                                                                                     : 0.0f;
 }
 
-__global__ void __launch_bounds__(kMaxThreads) k_batch_step(StepArgs A) {
+// kFcUnroll slots of a lane are loaded while as many are summed, OCC CTAs to an
+// SM.  HBM bounds a batch that fills the GPU, so what counts is bytes in flight:
+// 64 instances of 16..128 a side take 2.74 ms a step with 8 slots and 2 CTAs
+// (6.0 TB/s without padding), 2.97 with 16 and 1, 3.43 with 4 and 3, and took
+// 3.41 with 4 slots whose trace stores held back the next loads.  With no more
+// units than SMs a second CTA has nothing to do and the loads' latency is the
+// bound: 12 instances of 16..48 take 41 us a step with 16 slots, 48 with 8, and
+// took 66.
+template <int kFcUnroll, int OCC>
+__global__ void __launch_bounds__(kMaxThreads, OCC) k_batch_step(StepArgs A) {
     extern __shared__ uint32_t sm[];
     __shared__ int s_unit;
     __shared__ long long s_t;
@@ -152,23 +161,37 @@ __global__ void __launch_bounds__(kMaxThreads) k_batch_step(StepArgs A) {
             {
                 const float* ew = A.conv_ew + g * I.K * 32 + lane;
                 float2* ct = A.conv_tr + g * I.K * 32 + lane;
-                int k = 0;
-                for (int kr = 0; kr < I.field; ++kr) {
-                    const float* rrow = relay + (tr + kr) * I.cols;
-                    for (int kc = 0; kc < I.field; ++kc, ++k) {
-                        float spike = rrow[wrap1(col - h + kc, I.cols)];
-                        float weight = __ldg(ew + k * 32);
-                        float2 x = ct[k * 32];
-                        float st = x.x + (spike * weight * I.gconv);
+                const float* rrow = relay + tr * I.cols;
+                for (int k0 = 0, kc = 0; k0 < I.K; k0 += kConvUnroll) {
+                    float spike[kConvUnroll], weight[kConvUnroll];
+                    float2 x[kConvUnroll];
+#pragma unroll
+                    for (int j = 0; j < kConvUnroll; ++j) {
+                        if (k0 + j >= I.K) break;
+                        spike[j] = rrow[wrap1(col - h + kc, I.cols)];
+                        weight[j] = __ldg(ew + (k0 + j) * 32);
+                        x[j] = ct[(k0 + j) * 32];
+                        if (++kc == I.field) {
+                            kc = 0;
+                            rrow += I.cols;
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < kConvUnroll; ++j) {
+                        if (k0 + j >= I.K) break;
+                        const float st = x[j].x + (spike[j] * weight[j] * I.gconv);
                         s_sum += st;
-                        float lt = x.y + (spike * weight * I.gconv);
+                        const float lt = x[j].y + (spike[j] * weight[j] * I.gconv);
                         l_sum += lt;
-                        ct[k * 32] = make_float2(st * kAmpaTau, lt * kNmdaTau);
+                        ct[(k0 + j) * 32] = make_float2(st * kAmpaTau, lt * kNmdaTau);
                     }
                 }
             }
 
-            // recurrent fully connected, "sub": GABA-A (short) and GABA-B (long)
+            // recurrent fully connected, "sub": GABA-A (short) and GABA-B
+            // (long).  The next kFcUnroll slots are loaded before this lot is
+            // summed and stored: the loads are the bound, and the compiler
+            // may not move them over the trace stores itself.
             float f_sum = 0.0f, fl_sum = 0.0f;
             {
                 const long long base = A.group_base[g];
@@ -176,38 +199,36 @@ __global__ void __launch_bounds__(kMaxThreads) k_batch_step(StepArgs A) {
                 const uint2* in = A.fc_in + base * 32 + lane;
                 float2* trp = A.fc_tr + base * 32 + lane;
                 const float gf = I.gfc;
-                int s = 0;
-                for (; s + kFcUnroll <= slots; s += kFcUnroll) {
-                    uint2 x[kFcUnroll];
-                    float2 y[kFcUnroll];
+                uint2 x[2][kFcUnroll];
+                float2 y[2][kFcUnroll];
+                auto load = [&](int s, uint2 (&xx)[kFcUnroll], float2 (&yy)[kFcUnroll]) {
+#pragma unroll
+                    for (int j = 0; j < kFcUnroll; ++j)
+                        if (s + j < slots) {
+                            xx[j] = __ldg(in + (long long)(s + j) * 32);
+                            yy[j] = trp[(long long)(s + j) * 32];
+                        }
+                };
+                auto use = [&](int s, const uint2 (&xx)[kFcUnroll], const float2 (&yy)[kFcUnroll]) {
 #pragma unroll
                     for (int j = 0; j < kFcUnroll; ++j) {
-                        x[j] = __ldg(in + (long long)(s + j) * 32);
-                        y[j] = trp[(long long)(s + j) * 32];
-                    }
-#pragma unroll
-                    for (int j = 0; j < kFcUnroll; ++j) {
-                        uint32_t word = sm[x[j].x & 0x07FFFFFFu];
-                        float spike = (float)((word << (x[j].x >> 27)) >> 31);
-                        float weight = __uint_as_float(x[j].y);
-                        float st = y[j].x + (spike * weight * gf);
+                        if (s + j >= slots) break;
+                        const uint32_t word = sm[xx[j].x & 0x07FFFFFFu];
+                        const float spike = (float)((word << (xx[j].x >> 27)) >> 31);
+                        const float weight = __uint_as_float(xx[j].y);
+                        const float st = yy[j].x + (spike * weight * gf);
                         f_sum += st;
-                        float lt = y[j].y + (spike * weight * gf);
+                        const float lt = yy[j].y + (spike * weight * gf);
                         fl_sum += lt;
                         trp[(long long)(s + j) * 32] = make_float2(st * kGabaaTau, lt * kGababTau);
                     }
-                }
-                for (; s < slots; ++s) {
-                    uint2 x = __ldg(in + (long long)s * 32);
-                    float2 y = trp[(long long)s * 32];
-                    uint32_t word = sm[x.x & 0x07FFFFFFu];
-                    float spike = (float)((word << (x.x >> 27)) >> 31);
-                    float weight = __uint_as_float(x.y);
-                    float st = y.x + (spike * weight * gf);
-                    f_sum += st;
-                    float lt = y.y + (spike * weight * gf);
-                    fl_sum += lt;
-                    trp[(long long)s * 32] = make_float2(st * kGabaaTau, lt * kGababTau);
+                };
+                load(0, x[0], y[0]);
+                for (int s = 0; s < slots; s += 2 * kFcUnroll) {
+                    load(s + kFcUnroll, x[1], y[1]);
+                    use(s, x[0], y[0]);
+                    load(s + 2 * kFcUnroll, x[0], y[0]);
+                    use(s + kFcUnroll, x[1], y[1]);
                 }
             }
 
@@ -216,8 +237,8 @@ __global__ void __launch_bounds__(kMaxThreads) k_batch_step(StepArgs A) {
             const int local = gr * I.cols + col;
             const long long nid = I.neuron_off + local;
             float voltage = A.v[nid], recovery = A.u[nid];
-            iz_integrate(voltage, recovery, 0.0f + s_sum, 0.0f + l_sum, 0.0f + f_sum,
-                         0.0f + fl_sum, 0.0f, 0.0f, I.a, I.b);
+            iz_integrate_ff(voltage, recovery, 0.0f + s_sum, 0.0f + l_sum, 0.0f + f_sum,
+                            0.0f + fl_sum, 0.0f, 0.0f, I.a, I.b);
             unsigned int spike = voltage >= 30.0;
             words_out[nid] = (sm[local] >> 1) | (spike << 31);
             A.v[nid] = spike ? I.c : voltage;
@@ -600,8 +621,6 @@ class Batch {
         words_cap_ = (max_n_ + 3) / 4 * 4;
         smem_ = (size_t)(words_cap_ + (tile_rows + max_field_ - 1) * max_cols_) * 4;
         if ((int)smem_ > smem_optin_) throw SgError("batch: instance too large for shared memory");
-        SG_CUDA(cudaFuncSetAttribute(k_batch_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem_));
         units_h_.clear();
         for (size_t i = 0; i < inst_.size(); ++i) {
             const InstDev& I = inst_[i];
@@ -623,9 +642,15 @@ class Batch {
         }
         SG_CUDA(cudaMemcpyAsync(d_units_, units_h_.data(), units_h_.size() * sizeof(Unit),
                                 cudaMemcpyHostToDevice, stream_));
+        kernel_ = (int)units_h_.size() <= num_sms_ ? k_batch_step<16, 1> : k_batch_step<8, 2>;
+        // the limit is the function's, shared by every batch of the process:
+        // always the largest, or a smaller batch would lower it for a larger one
+        cudaFuncAttributes fa;
+        SG_CUDA(cudaFuncGetAttributes(&fa, kernel_));
+        SG_CUDA(cudaFuncSetAttribute(kernel_, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     smem_optin_ - (int)fa.sharedSizeBytes));
         int per_sm = 0;
-        SG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_step, threads_,
-                                                              smem_));
+        SG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel_, threads_, smem_));
         if (per_sm < 1) throw SgError("batch: step kernel does not fit on an SM");
         grid_ = (int)std::min<long long>((long long)units_h_.size(), (long long)per_sm * num_sms_);
         if (graph_) {
@@ -659,14 +684,14 @@ class Batch {
     }
 
     void launch() {
-        k_batch_step<<<grid_, threads_, smem_, stream_>>>(args());
+        kernel_<<<grid_, threads_, smem_, stream_>>>(args());
         SG_LAUNCH_CHECK();
     }
 
     void capture() {
         cudaGraph_t g;
         SG_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-        for (int i = 0; i < kGraphSteps; ++i) k_batch_step<<<grid_, threads_, smem_, stream_>>>(args());
+        for (int i = 0; i < kGraphSteps; ++i) kernel_<<<grid_, threads_, smem_, stream_>>>(args());
         SG_CUDA(cudaStreamEndCapture(stream_, &g));
         cudaError_t e = cudaGraphInstantiate(&graph_, g, 0);
         cudaGraphDestroy(g);
@@ -721,6 +746,7 @@ class Batch {
     int max_n_ = 0, max_cols_ = 0, max_rows_ = 0, max_field_ = 0, max_cblocks_ = 0, K_ = 0;
     int tile_rows_ = 0, tile_cblocks_ = 0, threads_ = 0, grid_ = 0, words_cap_ = 0;
     size_t smem_ = 0, units_cap_ = 0;
+    void (*kernel_)(StepArgs) = nullptr;
     int device_ = 0, num_sms_ = 0, smem_optin_ = 0;
     cudaStream_t stream_ = nullptr;
     cudaGraphExec_t graph_ = nullptr;

@@ -119,3 +119,28 @@ def test_dense_izhikevich_learning(sg, sources, dests, opcode):
     keys = [("matrix", "c", k) for k in ("weights", "presyn trace", "weight derivatives",
                                          "short term R", "short term w", "short trace")]
     assert_equal(run_both(sg, net, inject, 3, keys + [("b", "voltage")], learning=True))
+
+
+def test_batches_side_by_side(sg):
+    """Batches of few and many work units (the two forms of the step kernel)
+    and of different shared-memory sizes, alive together and captured late:
+    each equals itself run alone."""
+    from synaptogenesis_gb300 import batching
+    made = [([batching.instance(s, 40 + s, rows=s, cols=c) for s, c in sides], tile)
+            for sides, tile in (([(61, 97), (16, 16), (128, 70)], (1, 1)), ([(20, 33), (5, 9)], (2, 2)))]
+
+    def read(b, insts):
+        return [b.read(i, k).view(np.uint32) for i in range(len(insts))
+                for k in ("voltage", "recovery", "output")]
+
+    alone = []
+    for insts, tile in made:
+        with sg.Batch(insts, tile=tile) as b:
+            b.step(70)
+            alone.append(read(b, insts))
+    together = [sg.Batch(insts, tile=tile) for insts, tile in made]
+    for b in together:
+        b.step(70)
+    for b, (insts, _), want in zip(together, made, alone):
+        assert all(np.array_equal(x, y) for x, y in zip(read(b, insts), want))
+        b.close()
