@@ -505,14 +505,19 @@ constexpr int kPlaneHY = kPlaneTY + 2 * kPlaneK;
 constexpr int kPlaneHX = kPlaneTX + 2;
 constexpr size_t kPlaneSmem = (size_t)(2 + kPlaneK) * kPlaneHY * kPlaneHX * sizeof(uint32_t);
 
+// A row of a plane is ceil(cols / 32) words, padded to `pitch`; the bits of a
+// last, partial word past the row's end, and the padding, are zero.
+
 // Words of one row segment (32 cells) -> the 32 plane words of the segment.
-__global__ void k_gol_words_to_planes(int rows, int W, const uint32_t* __restrict__ words,
+__global__ void k_gol_words_to_planes(int rows, int cols, int pitch,
+                                      const uint32_t* __restrict__ words,
                                       uint32_t* __restrict__ planes) {
     const long long seg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    if (seg >= (long long)rows * W) return;
-    const uint32_t w = words[seg * 32 + lane];
-    const size_t plane_words = (size_t)rows * W;
+    if (seg >= (long long)rows * pitch) return;
+    const int r = (int)(seg / pitch), c = (int)(seg - (long long)r * pitch) * 32 + lane;
+    const uint32_t w = c < cols ? words[(size_t)r * cols + c] : 0u;
+    const size_t plane_words = (size_t)rows * pitch;
     uint32_t mine = 0;
 #pragma unroll
     for (int p = 0; p < 32; ++p) {
@@ -525,38 +530,43 @@ __global__ void k_gol_words_to_planes(int rows, int W, const uint32_t* __restric
 // Planes after T steps -> words; and, if T > 0, the input register of the
 // last step: the weighted count of the neighbours' newest bits one step
 // earlier (plane T + 30).
-__global__ void k_gol_planes_to_words(int rows, int W, long long T,
+__global__ void k_gol_planes_to_words(int rows, int cols, int pitch, long long T,
                                       const uint32_t* __restrict__ planes,
                                       uint32_t* __restrict__ words, float* __restrict__ input_out,
                                       unsigned mask9) {
+    const int W = (cols + 31) / 32;
     const long long seg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (seg >= (long long)rows * W) return;
-    const size_t plane_words = (size_t)rows * W;
-    const uint32_t pw = planes[(size_t)((T + lane) % kPlaneRing) * plane_words + seg];
+    const int r = (int)(seg / W), x = (int)(seg - (long long)r * W);
+    const int last = (cols - 1) & 31;                     // the row's last bit in its last word
+    const size_t plane_words = (size_t)rows * pitch;
+    const uint32_t pw = planes[(size_t)((T + lane) % kPlaneRing) * plane_words +
+                               (size_t)r * pitch + x];
     uint32_t word = 0;
 #pragma unroll
     for (int p = 0; p < 32; ++p) word |= ((__shfl_sync(0xFFFFFFFFu, pw, p) >> lane) & 1u) << p;
-    words[seg * 32 + lane] = word;
+    const int c = x * 32 + lane;
+    if (c >= cols) return;
+    words[(size_t)r * cols + c] = word;
     if (T == 0 || !input_out) return;
-    const int r = (int)(seg / W), x = (int)(seg - (long long)r * W);
     const uint32_t* prev = planes + (size_t)((T + 30) % kPlaneRing) * plane_words;
     uint32_t c0 = 0, c1 = 0, c2 = 0, c3 = 0;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         int rr = r + k - 1;
         rr = rr < 0 ? rr + rows : (rr >= rows ? rr - rows : rr);
-        const int xl = x == 0 ? W - 1 : x - 1, xr = x == W - 1 ? 0 : x + 1;
-        const uint32_t n = prev[(size_t)rr * W + x];
-        const uint32_t wv = (n << 1) | (prev[(size_t)rr * W + xl] >> 31);
-        const uint32_t ev = (n >> 1) | (prev[(size_t)rr * W + xr] << 31);
+        const uint32_t* row = prev + (size_t)rr * pitch;
+        const uint32_t n = row[x];
+        const uint32_t wv = (n << 1) | (x == 0 ? (row[W - 1] >> last) & 1u : row[x - 1] >> 31);
+        const uint32_t ev = (n >> 1) | (x == W - 1 ? (row[0] & 1u) << last : row[x + 1] << 31);
         if (mask9 & (1u << (k * 3 + 0))) csa_add(c0, c1, c2, c3, wv);
         if (mask9 & (1u << (k * 3 + 1))) csa_add(c0, c1, c2, c3, n);
         if (mask9 & (1u << (k * 3 + 2))) csa_add(c0, c1, c2, c3, ev);
     }
     const unsigned cnt = ((c0 >> lane) & 1u) | (((c1 >> lane) & 1u) << 1) |
                          (((c2 >> lane) & 1u) << 2) | (((c3 >> lane) & 1u) << 3);
-    input_out[seg * 32 + lane] = (float)cnt;
+    input_out[(size_t)r * cols + c] = (float)cnt;
 }
 
 // Neighbour count of 32 cells (bit-sliced, bits c0..c3) from the three rows'
@@ -706,9 +716,8 @@ __global__ void __launch_bounds__(kPlaneThreads) k_gol_planes_steps(int rows, in
 }
 
 // ---------------------------------------------------------------------------
-// game_of_life on bit planes, full-width strips: boards whose rows are 32, 64
-// or 128 words (1024, 2048 or 4096 cells) wide, counting the 8 outer cells or
-// all 9 cells of the 3x3 block.
+// game_of_life on bit planes, full-width strips: boards up to 4096 cells wide,
+// counting the 8 outer cells or all 9 cells of the 3x3 block.
 //
 // A CTA advances K steps (K <= 31) of a band of ty board rows plus K halo rows
 // above and below, one band per SM.  Each warp holds R consecutive band rows
@@ -732,6 +741,15 @@ __global__ void __launch_bounds__(kPlaneThreads) k_gol_planes_steps(int rows, in
 // 16 warps, registers permitting).
 __host__ __device__ constexpr int strip_rows(int wpl) { return wpl >= 4 ? 4 : 2; }
 __host__ __device__ constexpr int strip_max_warps(int rpw) { return rpw >= 4 ? 16 : 32; }
+// words a lane holds for a row of `cols` <= kStripCols cells, and a row's words
+// in the planes: whole lanes, so that a lane's words are one aligned vector
+constexpr int kStripCols = 4096;
+__host__ __device__ constexpr int strip_wpl(int cols) {
+    return cols <= 1024 ? 1 : (cols <= 2048 ? 2 : 4);
+}
+__host__ __device__ constexpr int strip_pitch(int cols) {
+    return ((cols + 31) / 32 + strip_wpl(cols) - 1) / strip_wpl(cols) * strip_wpl(cols);
+}
 constexpr int kStripDepth = 4;       // steps ahead the oldest-bit plane is copied
 
 template <int WPL>
@@ -810,17 +828,56 @@ struct StripRow {
     uint32_t s3[WPL], c3[WPL], s2[WPL], c2[WPL];
 };
 
-// Horizontal sums of one row held across the warp.
-template <int MODE, int WPL>
-__device__ __forceinline__ void strip_sums(const uint32_t (&v)[WPL], int lane, StripRow<WPL>& r) {
-    const uint32_t wi = __shfl_sync(0xFFFFFFFFu, v[WPL - 1], (lane + 31) & 31);
+// Where a row that does not fill the warp's 32 * WPL words ends: its last word
+// (lane, index within the lane), the bits of that word in use, and, per word of
+// this lane, the bits in use (`valid`) and the row's last cell (`end`).
+template <int WPL>
+struct StripEnd {
+    int lane, word, bits;
+    uint32_t valid[WPL], end[WPL];
+};
+template <int WPL>
+__device__ __forceinline__ StripEnd<WPL> strip_end(int cols, int lane) {
+    StripEnd<WPL> e;
+    const int last = (cols - 1) / 32;
+    e.lane = last / WPL;
+    e.word = last - e.lane * WPL;
+    e.bits = cols - 32 * last;
+#pragma unroll
+    for (int j = 0; j < WPL; ++j) {
+        const int w = lane * WPL + j;
+        e.valid[j] = w < last ? ~0u : (w == last ? ~0u >> (32 - e.bits) : 0u);
+        e.end[j] = w == last ? 1u << (e.bits - 1) : 0u;
+    }
+    return e;
+}
+
+// Horizontal sums of one row held across the warp.  In a row that does not
+// fill the warp (RAGGED) the first cell's west neighbour is the last cell, and
+// the last cell's east neighbour the first; bits past the end are zero in v and
+// garbage in the sums, which nothing reads before they are masked.
+template <int MODE, int WPL, bool RAGGED>
+__device__ __forceinline__ void strip_sums(const uint32_t (&v)[WPL], int lane,
+                                           const StripEnd<WPL>& end, StripRow<WPL>& r) {
+    uint32_t wi = __shfl_sync(0xFFFFFFFFu, v[WPL - 1], (lane + 31) & 31);
     const uint32_t ei = __shfl_sync(0xFFFFFFFFu, v[0], (lane + 1) & 31);
+    uint32_t first = 0;                                      // all ones if the first cell is set
+    if (RAGGED) {
+        uint32_t lw = v[0];
+#pragma unroll
+        for (int j = 1; j < WPL; ++j)
+            if (end.word == j) lw = v[j];
+        lw = __shfl_sync(0xFFFFFFFFu, lw, end.lane);
+        if (lane == 0) wi = lw << (32 - end.bits);
+        first = 0u - (__shfl_sync(0xFFFFFFFFu, v[0], 0) & 1u);
+    }
 #pragma unroll
     for (int j = 0; j < WPL; ++j) {
         const uint32_t west = j == 0 ? wi : v[j > 0 ? j - 1 : 0];
         const uint32_t east = j == WPL - 1 ? ei : v[j < WPL - 1 ? j + 1 : 0];
         const uint32_t a = __funnelshift_l(west, v[j], 1);   // west neighbours: (v << 1) | (west >> 31)
-        const uint32_t b = __funnelshift_r(v[j], east, 1);   // east neighbours: (v >> 1) | (east << 31)
+        uint32_t b = __funnelshift_r(v[j], east, 1);         // east neighbours: (v >> 1) | (east << 31)
+        if (RAGGED) b |= first & end.end[j];
         r.s3[j] = a ^ v[j] ^ b;
         r.c3[j] = maj3(a, v[j], b);
         if (MODE == 1) {
@@ -830,11 +887,12 @@ __device__ __forceinline__ void strip_sums(const uint32_t (&v)[WPL], int lane, S
     }
 }
 
-template <int MODE, bool CONWAY, int WPL, int R>
+template <int MODE, bool CONWAY, int WPL, int R, bool RAGGED>
 __global__ void __launch_bounds__(strip_max_warps(R) * 32) k_gol_strips_steps(
-    int rows, int ty, long long T0, int K, uint32_t* __restrict__ planes, unsigned smask,
+    int rows, int cols, int ty, long long T0, int K, uint32_t* __restrict__ planes, unsigned smask,
     unsigned bmask) {
-    constexpr int W = 32 * WPL, XN = 2 * WPL;
+    constexpr int XN = 2 * WPL;
+    const int W = RAGGED ? strip_pitch(cols) : 32 * WPL;
     extern __shared__ uint4 strip_smem[];
     // [2][warps + 2][2][32][XN]: warp w publishes in slot w + 1; slots 0 and
     // warps + 1 stay zero (nothing above the first warp or below the last)
@@ -856,6 +914,8 @@ __global__ void __launch_bounds__(strip_max_warps(R) * 32) k_gol_strips_steps(
             for (int k = 0; k < 2 * XN; ++k)
                 xch[b * slots + (size_t)slot * 2 * 32 * XN + (size_t)k * 32 + lane] = 0u;
     }
+    const StripEnd<WPL> end = strip_end<WPL>(cols, lane);
+    const bool in_row = !RAGGED || lane * WPL < W;
     const size_t plane_words = (size_t)rows * W;
     const int r0 = blockIdx.x * ty, tile_n = min(ty, rows - r0);
     const int hb0 = warp * R;                 // first band row of this warp; band row K is board row r0
@@ -876,9 +936,13 @@ __global__ void __launch_bounds__(strip_max_warps(R) * 32) k_gol_strips_steps(
         const uint32_t* newest = planes + (size_t)((t0 + 31) & (kPlaneRing - 1)) * plane_words;
         uint32_t v[R][WPL];
 #pragma unroll
-        for (int q = 0; q < R; ++q) strip_ld<WPL>(newest + off[q], v[q]);
+        for (int q = 0; q < R; ++q) {
 #pragma unroll
-        for (int q = 0; q < R; ++q) strip_sums<MODE, WPL>(v[q], lane, cur[q]);
+            for (int j = 0; j < WPL; ++j) v[q][j] = 0u;
+            if (in_row) strip_ld<WPL>(newest + off[q], v[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < R; ++q) strip_sums<MODE, WPL, RAGGED>(v[q], lane, end, cur[q]);
     }
     // the cells' oldest bits: plane T0 + s at step s
     // The cells' oldest bits, plane T0 + s at step s, come through a ring of
@@ -888,7 +952,7 @@ __global__ void __launch_bounds__(strip_max_warps(R) * 32) k_gol_strips_steps(
     uint32_t* oring = xch + 2 * slots + (size_t)lane * WPL;       // [depth][warps * R][32][WPL]
     const size_t oslot = (size_t)nw * R * 32 * WPL;
     auto fetch_oldest = [&](int s) {
-        if (s < K) {
+        if (s < K && in_row) {
             const uint32_t* p = planes + (size_t)((t0 + s) & (kPlaneRing - 1)) * plane_words;
             uint32_t* d = oring + (size_t)(s % kStripDepth) * oslot + (size_t)hb0 * 32 * WPL;
 #pragma unroll
@@ -962,19 +1026,20 @@ __global__ void __launch_bounds__(strip_max_warps(R) * 32) k_gol_strips_steps(
                     }
                     nl[j] = (Od[q][j] & S) | (~Od[q][j] & B);
                 }
+                if (RAGGED) nl[j] &= end.valid[j];
             }
             // the new row q - 1 is no longer read as an old row: store it and
             // take its sums
             if (q > 0) {
-                if (tile_rows & (1u << (q - 1))) strip_st<WPL>(out + off[q - 1], prev);
-                strip_sums<MODE, WPL>(prev, lane, cur[q - 1]);
+                if (in_row && (tile_rows & (1u << (q - 1)))) strip_st<WPL>(out + off[q - 1], prev);
+                strip_sums<MODE, WPL, RAGGED>(prev, lane, end, cur[q - 1]);
             }
 #pragma unroll
             for (int j = 0; j < WPL; ++j) prev[j] = nl[j];
         }
         {
-            if (tile_rows & (1u << (R - 1))) strip_st<WPL>(out + off[R - 1], prev);
-            strip_sums<MODE, WPL>(prev, lane, cur[R - 1]);
+            if (in_row && (tile_rows & (1u << (R - 1)))) strip_st<WPL>(out + off[R - 1], prev);
+            strip_sums<MODE, WPL, RAGGED>(prev, lane, end, cur[R - 1]);
         }
         // buffer (s + 1) & 1 was last read before this step's barrier
         publish((s + 1) & 1);
@@ -1056,8 +1121,11 @@ class GameOfLifeModel : public Model {
             swap->scratch = true;
             ls.internal["output swap"] = swap;
             const Connection& c = *l.inputs[0];
-            if (c.delay == 0 && c.arbor.wrap && l.cols % 32 == 0) {
-                Array* planes = st.add_array("planes", 'u', (size_t)kPlaneRing * (l.size / 32));
+            if (c.delay == 0 && c.arbor.wrap && (l.cols % 32 == 0 || l.cols <= kStripCols)) {
+                Array* planes = st.add_array(
+                    "planes", 'u',
+                    (size_t)kPlaneRing * l.rows *
+                        (l.cols <= kStripCols ? strip_pitch(l.cols) : l.cols / 32));
                 planes->scratch = true;
                 ls.internal["planes"] = planes;
             }
@@ -1080,22 +1148,27 @@ class GameOfLifeModel : public Model {
     static size_t strip_smem_bytes(int warps, int rpw, int wpl) {
         return ((size_t)(warps + 2) * 256 + (size_t)kStripDepth * warps * rpw * 32) * wpl * 4;
     }
-    static long advance_strips(int rows, int W, int mode, bool conway, long n, uint32_t* planes,
+    static long advance_strips(int rows, int cols, int mode, bool conway, long n, uint32_t* planes,
                                unsigned smask, unsigned bmask, cudaStream_t s) {
-        using Kernel = void (*)(int, int, long long, int, uint32_t*, unsigned, unsigned);
-        const int wpl = W / 32;
+        using Kernel = void (*)(int, int, int, long long, int, uint32_t*, unsigned, unsigned);
+        const int wpl = strip_wpl(cols);
+        const int ragged = cols == 1024 * wpl ? 0 : 1;
         const int rpw = strip_rows(wpl), max_warps = strip_max_warps(rpw);
         const int wi = wpl == 1 ? 0 : (wpl == 2 ? 1 : 2);
-#define SG_STRIPS(M, C)                                                                  \
-    {k_gol_strips_steps<M, C, 1, strip_rows(1)>, k_gol_strips_steps<M, C, 2, strip_rows(2)>, \
-     k_gol_strips_steps<M, C, 4, strip_rows(4)>}
-        static const Kernel kernels[2][2][3] = {{SG_STRIPS(1, false), SG_STRIPS(1, true)},
-                                                {SG_STRIPS(2, false), SG_STRIPS(2, true)}};
+#define SG_STRIPS(M, C)                                                                          \
+    {{k_gol_strips_steps<M, C, 1, strip_rows(1), false>,                                         \
+      k_gol_strips_steps<M, C, 2, strip_rows(2), false>,                                         \
+      k_gol_strips_steps<M, C, 4, strip_rows(4), false>},                                        \
+     {k_gol_strips_steps<M, C, 1, strip_rows(1), true>,                                          \
+      k_gol_strips_steps<M, C, 2, strip_rows(2), true>,                                          \
+      k_gol_strips_steps<M, C, 4, strip_rows(4), true>}}
+        static const Kernel kernels[2][2][2][3] = {{SG_STRIPS(1, false), SG_STRIPS(1, true)},
+                                                   {SG_STRIPS(2, false), SG_STRIPS(2, true)}};
 #undef SG_STRIPS
-        const Kernel kernel = kernels[mode - 1][conway ? 1 : 0][wi];
+        const Kernel kernel = kernels[mode - 1][conway ? 1 : 0][ragged][wi];
         const size_t max_smem = strip_smem_bytes(max_warps, rpw, wpl);
-        static bool configured[2][2][3] = {};
-        bool& cfg = configured[mode - 1][conway ? 1 : 0][wi];
+        static bool configured[2][2][2][3] = {};
+        bool& cfg = configured[mode - 1][conway ? 1 : 0][ragged][wi];
         if (!cfg) {
             SG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)max_smem));
@@ -1126,7 +1199,8 @@ class GameOfLifeModel : public Model {
             attr[0].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            SG_CUDA(cudaLaunchKernelEx(&cfg, kernel, rows, ty, (long long)T, K, planes, smask, bmask));
+            SG_CUDA(cudaLaunchKernelEx(&cfg, kernel, rows, cols, ty, (long long)T, K, planes, smask,
+                                       bmask));
             ++launches;
             T += K;
         }
@@ -1139,7 +1213,12 @@ class GameOfLifeModel : public Model {
         if (!fusable_shape(l) || !ls.internal.count("planes")) return false;
         const ConnState& cs = *st.conn_state(l.inputs[0]);
         auto bm = cs.params.find("bits mask");
-        return bm != cs.params.end() && bm->second >= 0.0f;
+        return bm != cs.params.end() && bm->second >= 0.0f &&
+               (l.cols % 32 == 0 || plane_mode((unsigned)bm->second) != 0);
+    }
+    // counting kernel of a 0/1 mask: 1 the 8 outer neighbours, 2 all 9, 0 others
+    static int plane_mode(unsigned mask9) {
+        return (mask9 & 0x1EFu) == 0x1EFu ? ((mask9 & 0x10u) ? 2 : 1) : 0;
     }
     long advance_alone(State& st, LayerState& ls, long n, cudaStream_t s) const override {
         const Layer& l = *ls.layer;
@@ -1147,22 +1226,28 @@ class GameOfLifeModel : public Model {
         const unsigned mask9 = (unsigned)cs.params.at("bits mask");
         const unsigned smask = count_mask((int)ls.params.at("smin"), (int)ls.params.at("smax"));
         const unsigned bmask = count_mask((int)ls.params.at("bmin"), (int)ls.params.at("bmax"));
-        const int W = l.cols / 32;
         uint32_t* planes = ls.internal.at("planes")->du();
         uint32_t* words = ls.output->du();
+        // the B3/S23 rule is its own instance of either kernel
+        const int mode = plane_mode(mask9);
+        const bool conway = smask == count_mask(2, 3) && bmask == count_mask(3, 3);
+        // Strips wherever a row fits a warp.  Time per step against the tile
+        // kernel (aligned widths): 0.40 / 0.52 us at 500 x 320, 0.58 / 0.92 at
+        // 1500 x 1504, 0.38 / 0.63 at 32 x 32; against the per-step word
+        // kernel, the only other path for ragged widths: 0.40 / 5.0 us at
+        // 500 x 333, 0.58 / 33 at 1500 x 1500, 0.78 / 15 at 300 x 3000.
+        const bool strips = mode != 0 && l.cols <= kStripCols;
+        const int W = (l.cols + 31) / 32, pitch = strips ? strip_pitch(l.cols) : W;
         const long long segs = (long long)l.rows * W;
         long launches = 0;
-        k_gol_words_to_planes<<<blocks_for(segs * 32, 256), 256, 0, s>>>(l.rows, W, words, planes);
+        k_gol_words_to_planes<<<blocks_for((long)l.rows * pitch * 32, 256), 256, 0, s>>>(
+            l.rows, l.cols, pitch, words, planes);
         SG_LAUNCH_CHECK();
         ++launches;
-        // counting kernel: the 8 outer neighbours, all 9, or any other 0/1
-        // mask; the B3/S23 rule as its own instance
-        const int mode = (mask9 & 0x1EFu) == 0x1EFu ? ((mask9 & 0x10u) ? 2 : 1) : 0;
-        const bool conway = smask == count_mask(2, 3) && bmask == count_mask(3, 3);
-        if (mode != 0 && (W == 32 || W == 64 || W == 128)) {
-            launches += advance_strips(l.rows, W, mode, conway, n, planes, smask, bmask, s);
+        if (strips) {
+            launches += advance_strips(l.rows, l.cols, mode, conway, n, planes, smask, bmask, s);
             k_gol_planes_to_words<<<blocks_for(segs * 32, 256), 256, 0, s>>>(
-                l.rows, W, n, planes, words, ls.input->df(), mask9);
+                l.rows, l.cols, pitch, n, planes, words, ls.input->df(), mask9);
             SG_LAUNCH_CHECK();
             return launches + 1;
         }
@@ -1201,7 +1286,7 @@ class GameOfLifeModel : public Model {
             T += K;
         }
         k_gol_planes_to_words<<<blocks_for(segs * 32, 256), 256, 0, s>>>(
-            l.rows, W, T, planes, words, ls.input->df(), mask9);
+            l.rows, l.cols, W, T, planes, words, ls.input->df(), mask9);
         SG_LAUNCH_CHECK();
         return launches + 1;
     }
@@ -1209,16 +1294,15 @@ class GameOfLifeModel : public Model {
         return fusable_shape(*c.to) && !ctx.is_input(*c.to);
     }
     // After every upload: can the bit-sliced kernel run this layer?  (3x3
-    // convolutional kernel of 0/1 weights, stride and spacing 1, offset -1,
-    // whole 32-cell row segments.)
+    // convolutional kernel of 0/1 weights, stride and spacing 1, offset -1; the
+    // per-step kernel also wants whole 32-cell row segments.)
     void prepare_device(State& st, ConnState& cs, cudaStream_t) const override {
         const Connection& c = *cs.conn;
         cs.params["bits mask"] = -1.0f;
         if (!fusable_shape(*c.to) || !c.convolutional) return;
         const Arbor& a = c.arbor;
         if (a.row_field != 3 || a.col_field != 3 || a.row_stride != 1 || a.col_stride != 1 ||
-            a.row_spacing != 1 || a.col_spacing != 1 || a.row_offset != -1 || a.col_offset != -1 ||
-            c.to->cols % 32 != 0)
+            a.row_spacing != 1 || a.col_spacing != 1 || a.row_offset != -1 || a.col_offset != -1)
             return;
         const float* w = cs.weights->hf();
         unsigned mask = 0;
@@ -1236,7 +1320,7 @@ class GameOfLifeModel : public Model {
             ConnState& cs = *st.conn_state(l.inputs[0]);
             Array* swap = ls.internal.at("output swap");
             auto bm = cs.params.find("bits mask");
-            if (bm != cs.params.end() && bm->second >= 0.0f) {
+            if (l.cols % 32 == 0 && bm != cs.params.end() && bm->second >= 0.0f) {
                 int strips = (l.cols / 32 + 31) / 32;
                 dim3 grid(strips, blocks_for(l.rows, kTileRows));
                 k_gol_bits_tile<<<grid, 256, 0, ctx.stream>>>(

@@ -144,3 +144,23 @@ def test_batches_side_by_side(sg):
     for b, (insts, _), want in zip(together, made, alone):
         assert all(np.array_equal(x, y) for x, y in zip(read(b, insts), want))
         b.close()
+
+
+# rows across a warp: 1, 2 or 4 words a lane up to 1024, 2048 and 4096 cells, a
+# last word of any number of bits; whole runs of 12 steps a launch
+@pytest.mark.parametrize("rows,cols,diagonal,low,high", [
+    (1, 1, False, 2, 3), (5, 2, True, 2, 3), (3, 31, False, 2, 3), (40, 33, False, 1, 4),
+    (7, 63, True, 3, 4), (200, 333, False, 2, 3), (19, 1000, False, 2, 3), (9, 1023, True, 2, 5),
+    (8, 1025, False, 2, 3), (6, 1056, False, 2, 3), (11, 1999, True, 3, 4), (5, 2049, False, 2, 3),
+    (4, 2080, False, 1, 3), (3, 4095, False, 2, 3)])
+def test_gol_whole_runs_on_ragged_boards(sg, rows, cols, diagonal, low, high):
+    net = network([layer("b", "game_of_life", rows, cols, survival_min=low, survival_max=high,
+                         birth_min=3, birth_max=3)],
+                  [connection("c", "b", "b", "convergent", convolutional=True, **{
+                      "weight config": {"type": "flat", "weight": 1.0, "diagonal": diagonal},
+                      "arborized config": {"field size": 3, "wrap": True}})])
+    words = np.random.default_rng(rows * cols).integers(0, 2**32, rows * cols,
+                                                       dtype=np.uint64).astype(np.uint32)
+    for steps in (1, 12, 37):
+        assert_equal(run_both(sg, net, {("b", "output"): words}, steps,
+                              [("b", "output"), ("b", "input")]))
