@@ -319,7 +319,7 @@ def rate_workload():
                 "steps of N(0,1) input, MSE to U(0,1) targets (seed 4), checkpoint every 10",
         "unit": "sequence-timesteps/s",
         "dtype": "f32",
-        "kernel": "k_rate_fused (forward pass: one launch for all timesteps; time per timestep)",
+        "kernel": "k_rate_layer (forward pass: a launch per layer and chunk of timesteps; time per timestep)",
         "cpu_seconds": 12.0,
         "rate": True,
     }

@@ -259,7 +259,8 @@ void sg_batch_destroy(SG_BATCH batch);
  *   y        [steps][batch][outputs] (optional output)
  *   loss     one float
  * The workspace (sg_rate_workspace_bytes, device memory owned by the caller)
- * keeps the forward pass's checkpoints (v every `checkpoint` steps) for the
+ * keeps the forward pass's checkpoints (v every `checkpoint` steps, or fewer of
+ * them in small networks, whose longer segments stay in cache) for the
  * backward pass, which recomputes each segment from its checkpoint and runs
  * the hand-written adjoint back through it.  d_weights, d_readout, d_tau (and
  * d_x, or NULL) receive grad_loss * dloss/d(parameter).  Work is asynchronous

@@ -29,17 +29,26 @@
 //   dR[o][i]   = sum_{t,b} gy[t][o] r_{L-1}[t][i]
 //   dtau_l     = -(dt / tau_l^2) sum_{t,b,i} lambda_l[t][i] d_l[t][i]
 //   dx[t]      = a_0 lambda_0[t]
-// The forward pass stores v every `checkpoint` steps; the backward pass
-// recomputes each segment's states from its checkpoint (bit-identical: the
-// same kernel on the same inputs), then runs the adjoint back through it.
-// Every sum has a fixed order, and every gradient accumulator takes one
-// timestep's sum at a time, so results are deterministic and do not depend on
-// the checkpoint stride.
+// The forward pass stores v every few steps (at least `checkpoint` apart); the
+// backward pass recomputes each segment's states from its checkpoint
+// (bit-identical: the same kernels on the same inputs), then runs the adjoint
+// back through it.  Every sum has a fixed order, and every gradient accumulator
+// takes one timestep's sum at a time, so results are deterministic and do not
+// depend on the checkpoint stride.
+//
+// A layer reads only the layer below, one step earlier, and its own state is
+// pointwise in time, so a stretch of steps is run layer by layer and not step
+// by step: one launch takes a layer through every step of a segment, all of its
+// stencils independent but for the pointwise recurrence, which stays in
+// registers.  The adjoint runs the same way from the last layer down.  Before, a
+// tile's layers ran step by step in one CTA with a barrier per step, recomputing
+// halos, and the adjoint took a launch per step: forward and adjoint of 3 x 64x64
+// layers, field 5, batch 64, 100 steps took 4.55 ms; 1.76 ms like this (4 x 30x45,
+// batch 5, 37 steps: 0.56 and 0.34 ms).
 //
 // Layout on the device: the convergent weights are transposed once per call
 // into the workspace as [layer][k][neuron], so that consecutive threads
-// (consecutive neurons) read consecutive weights; the readout is reduced per
-// 256-neuron block inside the step kernel and finished at the end.
+// (consecutive neurons) read consecutive weights.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -61,20 +70,37 @@ constexpr int kTauBlocks = 64;
 constexpr int kBlock = 256;
 
 struct Dims {
-    int L, rows, cols, N, field, h, K, O, B, T, k, nseg, nchunk, bg;
+    int L, rows, cols, N, field, K, O, B, T, k, nseg, chunk;
     float dt;
-    long long S;   // L * B * N
+    long long BN, S;   // B * N, L * B * N
+    long long G;       // gradient elements: (L - 1) * N * K weights, then O * N of the readout
 };
 
 // The rate network is checked against an FP64 restatement (not a bit-exact
-// reference), so it uses the fast exponential and a correctly rounded
-// reciprocal (relative error a few units in the last place), and explicit
-// fused multiply-adds in its sums; every kernel is deterministic, so the
-// backward pass recomputes the forward states bit for bit.
-__device__ __forceinline__ float sigmoid(float v) { return __frcp_rn(1.0f + __expf(-v)); }
+// reference), so it uses the fast exponential, a reciprocal by one Newton step
+// (relative error a few units in the last place in all) and explicit fused
+// multiply-adds in its sums; every kernel is deterministic, so the backward pass
+// recomputes the forward states bit for bit.
+__device__ __forceinline__ float sigmoid(float v) {
+    float e, y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(v * -1.44269504f));
+    const float d = 1.0f + e;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+    // (an infinite d, v below -88, has a zero reciprocal and no correction)
+    return d > 1.0e38f ? y : __fmaf_rn(y, __fmaf_rn(-d, y, 1.0f), y);
+}
+
+// Launches follow one another closely (programmatic dependents): a kernel waits
+// here for the one before it, which has waited for its own predecessor, so what
+// was written two launches ago or earlier may be read before the wait.
+__device__ __forceinline__ void wait_for_previous() {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
 
 // wt[l][k][i] = w[l][i][k]
 __global__ void k_rate_transpose(Dims D, const float* __restrict__ w, float* __restrict__ wt) {
+    wait_for_previous();
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)(D.L - 1) * D.N * D.K) return;
     const long long per = (long long)D.N * D.K;
@@ -84,435 +110,341 @@ __global__ void k_rate_transpose(Dims D, const float* __restrict__ w, float* __r
     wt[idx] = w[l * per + (long long)i * D.K + k];
 }
 
-// One forward timestep: grid (tiles of 16 x 16 neurons, layers, groups of
-// D.bg batch elements).  A thread keeps its neuron's field x field weights
-// (and, in the last layer, its readout weights) in registers; per batch
-// element the CTA stages the source rates of its tile plus the kernel's halo
-// (zero outside the layer: a skipped source adds w * 0) in shared memory,
-// double-buffered, with the next element's halo fetched into registers while
-// the current one is summed.  Tiles of the last layer reduce their readout
-// contributions (fixed tree) into ypart[b][tile][o].
-constexpr int kTileSide = 16;
-constexpr int kMaxBatchGroup = 8;
+// ---------------------------------------------------------------------------
+// Stencil tiles.  A CTA of kTileWarps warps owns a tile of 32 columns; a thread
+// owns PY neurons of one column in consecutive rows, so that the PY + F - 1
+// window rows it reads serve F x F terms of every one of them: (PY + F - 1) F
+// shared-memory reads for PY F F multiply-adds (0.6 per term at 5 x 5 and
+// PY = 2, where a neuron a thread needs 1).  Instruction issue is what bounds
+// these kernels, at half its rate for want of warps: at 5 x 5, two rows (72
+// registers, 7 CTAs an SM) took 13.9 us a 10-step launch where four (151, 3 CTAs)
+// took 20.1, though four issue fewer instructions.  Everything else in the loop over items (batch element, timestep) is
+// kept short: offsets within a layer are 32-bit and worked out once, added to
+// bases that are the same for the whole CTA; windows (tile plus halo) come in
+// with cp.async, 16 bytes at a time where the layer's rows allow it (V = 4),
+// kTileDepth - 1 items ahead, and the part of a window outside the layer (a
+// skipped source adds w * 0) is zeroed once and never copied.
+// ---------------------------------------------------------------------------
+constexpr int kTileWarps = 4;
+constexpr int kTileThreads = 32 * kTileWarps;
+constexpr int kTileDepth = 4;
 
-// Source window of a tile: element e of the (16 + 2h)^2 halo, zero outside.
-// A thread copies elements threadIdx.x + q * kBlock; their plane offsets
-// (-1 outside the layer) and shared-memory slots (-1 past the window) are the
-// same for every batch element and are worked out once.
-template <int F>
-struct Halo {
-    static constexpr int H = F / 2, SIDE = kTileSide + 2 * H, COUNT = SIDE * SIDE;
-    static constexpr int PER = (COUNT + kBlock - 1) / kBlock;
-    // row pitch = 16 (mod 32): the two tile rows a warp reads hit disjoint banks
-    static constexpr int PITCH = SIDE <= 16 ? 16 : 48;
-    int off[PER], slot[PER];
-    __device__ Halo(const Dims& D, int ty0, int tx0) {
+constexpr int tile_py(int field) { return field <= 3 ? 8 : (field <= 7 ? 2 : 1); }
+
+// CTAs an SM should hold of the forward kernel: up to 50 weights fit in 72
+// registers, and seven CTAs are one wave of 1024 (3 x 64x64, batch 64: 13.9 us a
+// 10-step launch against 14.9 with five).
+constexpr int tile_ctas(int field, int py) { return field * field * py <= 50 ? 7 : 1; }
+
+template <int F, int PY, int V>
+struct Tile {
+    static constexpr int H = F / 2, TY = PY * kTileWarps, WY = TY + 2 * H;
+    // columns left of the tile in a window row: whole pieces of V
+    static constexpr int LEFT = (H + V - 1) / V * V, WX = 32 + 2 * LEFT;
+    static constexpr int COUNT = WY * WX, PIECES = COUNT / V;
+    static constexpr int PER = (PIECES + kTileThreads - 1) / kTileThreads;
+    int y0, x0, lane, row;                   // the tile; this thread's column, first row in it
+    unsigned off[PER];                       // pieces this thread copies,
+    unsigned copies;                         // those that lie in the layer,
+    unsigned rows_ok;                        // rows of this thread that do,
+    unsigned own[PY];                        // and its neurons (0 for the others)
+
+    __device__ Tile(const Dims& D, float (*win)[COUNT]) {
+        const int tiles_x = (D.cols + 31) / 32;
+        y0 = blockIdx.x / tiles_x * TY;
+        x0 = blockIdx.x % tiles_x * 32;
+        lane = threadIdx.x & 31;
+        row = (threadIdx.x >> 5) * PY;
+        rows_ok = copies = 0;
 #pragma unroll
-        for (int q = 0; q < PER; ++q) {
-            const int e = threadIdx.x + q * kBlock;
-            const int sy = e / SIDE, sx = e - sy * SIDE;
-            const int r = ty0 - H + sy, c = tx0 - H + sx;
-            slot[q] = e < COUNT ? sy * PITCH + sx : -1;
-            off[q] = (r >= 0 && r < D.rows && c >= 0 && c < D.cols) ? r * D.cols + c : -1;
+        for (int q = 0; q < PY; ++q) {
+            const bool in = x0 + lane < D.cols && y0 + row + q < D.rows;
+            if (in) rows_ok |= 1u << q;
+            own[q] = in ? (unsigned)((y0 + row + q) * D.cols + x0 + lane) : 0u;
+        }
+#pragma unroll
+        for (int e = 0; e < PER; ++e) {
+            const int n = threadIdx.x + e * kTileThreads;
+            const int r = y0 - H + n / (WX / V), c = x0 - LEFT + n % (WX / V) * V;
+            const bool in = n < PIECES && r >= 0 && r < D.rows && c >= 0 && c < D.cols;
+            if (in) copies |= 1u << e;
+            off[e] = in ? (unsigned)(r * D.cols + c) : 0u;
+            if (n < PIECES && !in)
+                for (int s = 0; s < kTileDepth; ++s)
+#pragma unroll
+                    for (int j = 0; j < V; ++j) win[s][n * V + j] = 0.0f;
         }
     }
-    __device__ void fetch(const float* plane, float scale, float (&reg)[PER]) const {
+    __device__ bool ok(int q) const { return rows_ok >> q & 1u; }
+    // one commit group per call, also past the last item (!more)
+    __device__ void fetch(float* win, const float* plane, bool more) const {
+        if (more) {
 #pragma unroll
-        for (int q = 0; q < PER; ++q)
-            reg[q] = (slot[q] >= 0 && off[q] >= 0) ? scale * plane[off[q]] : 0.0f;
+            for (int e = 0; e < PER; ++e)
+                if (copies >> e & 1u) {
+                    const unsigned dst = (unsigned)__cvta_generic_to_shared(
+                        win + (threadIdx.x + e * kTileThreads) * V);
+                    if (V == 4)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
+                                     "l"(plane + off[e]) : "memory");
+                    else
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst),
+                                     "l"(plane + off[e]) : "memory");
+                }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    __device__ void stage(const float (&reg)[PER], float* dst) const {
-#pragma unroll
-        for (int q = 0; q < PER; ++q)
-            if (slot[q] >= 0) dst[slot[q]] = reg[q];
+    // the oldest item's window has landed for every thread, and every thread
+    // has read the window before it
+    __device__ void wait() const {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kTileDepth - 2) : "memory");
+        __syncthreads();
+    }
+    // this thread's corner of a window: the source of its row 0, kernel (0, 0)
+    __device__ const float* corner(const float* win) const {
+        return win + row * WX + lane + LEFT - H;
     }
 };
 
-template <int F>
-__global__ void __launch_bounds__(kBlock) k_rate_step(
-    Dims D, const float* __restrict__ x_t, const float* wt, const float* wo,
-    const float* __restrict__ tau, const float* __restrict__ v_prev,
-    const float* __restrict__ r_prev, float* __restrict__ v_new, float* __restrict__ r_new,
-    float* __restrict__ d_out, float* __restrict__ ypart) {
-    using W = Halo<F>;
-    __shared__ float src[2][W::SIDE][W::PITCH];
-    __shared__ float red[kBlock / 32][kMaxOutputs];
-    const int tiles_x = (D.cols + kTileSide - 1) / kTileSide;
-    const int tile = blockIdx.x, l = blockIdx.y;
-    const int ty0 = (tile / tiles_x) * kTileSide, tx0 = (tile % tiles_x) * kTileSide;
-    const int tr = threadIdx.x / kTileSide, tc = threadIdx.x % kTileSide;
-    const int ir = ty0 + tr, ic = tx0 + tc;
-    const bool ok = ir < D.rows && ic < D.cols;
-    const int i = ir * D.cols + ic;
-    const bool readout = ypart && l == D.L - 1;
+// One layer l >= 1 through nt steps (c + 1 .. c + nt) for a group of batch
+// elements: grid (tiles, batch groups).  src: the rates of layer l - 1 at steps
+// c .. c + nt - 1, `src_t` floats apart; r: this layer's rates at c .. c + nt.
+struct LayerArgs {
+    const float* src;
+    long long src_t;
+    float* r;
+    long long r_t;
+    float* d;                // drives of steps c + 1 .. c + nt, S apart, or null
+    const float* v0;         // [B][N] at step c, or null (zero)
+    float* v1;               // at step c + nt, or null
+    float* ckpt;             // checkpoints of this layer, S apart, or null
+    int c, nt, bg;
+};
+
+template <int F, int PY, int V>
+__global__ void __launch_bounds__(kTileThreads, tile_ctas(F, PY)) k_rate_layer(Dims D, int l, LayerArgs A,
+                                                             const float* __restrict__ wt,
+                                                             const float* __restrict__ tau) {
+    using W = Tile<F, PY, V>;
+    __shared__ __align__(16) float win[kTileDepth][W::COUNT];
+    const W tile(D, win);
     const float a = D.dt / __ldg(tau + l);
-    // plain loads: kept in registers across the batch loop's barriers
-    float wk[F * F];
+    // weights of neurons outside the layer are neuron 0's; nothing they give is stored
+    float wk[PY][F * F];
+    const float* wl = wt + (long long)(l - 1) * F * F * D.N;
 #pragma unroll
-    for (int k = 0; k < F * F; ++k)
-        wk[k] = (l >= 1 && ok) ? wt[((long long)(l - 1) * F * F + k) * D.N + i] : 0.0f;
-    float wov[kMaxOutputs];
+    for (int k = 0; k < F * F; ++k, wl += D.N)
 #pragma unroll
-    for (int o = 0; o < kMaxOutputs; ++o)
-        wov[o] = (readout && ok && o < D.O) ? wo[(long long)o * D.N + i] : 0.0f;
-    const int b0 = blockIdx.z * D.bg, b1 = min(D.B, b0 + D.bg);
-    const float* rp = l >= 1 ? r_prev + (long long)(l - 1) * D.B * D.N : nullptr;
-    const W halo(D, ty0, tx0);
-    float pre[W::PER];
-    if (l >= 1) halo.fetch(rp + (long long)b0 * D.N, 1.0f, pre);
-    for (int b = b0, buf = 0; b < b1; ++b, buf ^= 1) {
-        if (l >= 1) halo.stage(pre, &src[buf][0][0]);
-        const long long idx = ((long long)l * D.B + b) * D.N + i;
-        const float vp = ok ? v_prev[idx] : 0.0f;
-        float I = (ok && l == 0) ? __ldg(x_t + (long long)b * D.N + i) : 0.0f;
-        __syncthreads();
-        if (l >= 1 && b + 1 < b1) halo.fetch(rp + (long long)(b + 1) * D.N, 1.0f, pre);
-        float rn = 0.0f;
-        if (ok) {
-            if (l >= 1) {
-                // one partial sum per kernel row (independent chains), rows
-                // added in order
-                float part[F];
-#pragma unroll
-                for (int kr = 0; kr < F; ++kr) {
-                    part[kr] = 0.0f;
-#pragma unroll
-                    for (int kc = 0; kc < F; ++kc)
-                        part[kr] = __fmaf_rn(wk[kr * F + kc], src[buf][tr + kr][tc + kc], part[kr]);
-                }
-#pragma unroll
-                for (int kr = 0; kr < F; ++kr) I += part[kr];
-            }
-            const float d = -vp + I;
-            const float vn = vp + a * d;
-            v_new[idx] = vn;
-            rn = sigmoid(vn);
-            r_new[idx] = rn;
-            if (d_out) d_out[idx] = d;
+        for (int q = 0; q < PY; ++q) wk[q][k] = __ldg(wl + tile.own[q]);
+    wait_for_previous();
+    const int b0 = blockIdx.y * A.bg, b1 = min(D.B, b0 + A.bg);
+    const float* src = A.src + (long long)b0 * D.N;          // the next item to fetch
+    int pb = b0, pt = 0, slot = 0;
+    auto fetch = [&](int into) {
+        tile.fetch(win[into], src, pb < b1);
+        src += A.src_t;
+        if (++pt == A.nt) {
+            pt = 0;
+            ++pb;
+            src += D.N - A.nt * A.src_t;
         }
-        if (readout) {
-            // butterfly transpose reduction: after the exchanges with lanes
-            // 16, 8, 4, 2 apart a lane holds one output's partial sum of 32
-            // lanes' contributions -- output lane >> 1 -- and the exchange
-            // with the neighbour completes it (16 shuffles for 16 outputs)
-            const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-            float c[kMaxOutputs];
+    };
 #pragma unroll
-            for (int o = 0; o < kMaxOutputs; ++o) c[o] = wov[o] * rn;
+    for (int s = 0; s < kTileDepth - 1; ++s) fetch(s);
+    for (int b = b0; b < b1; ++b) {
+        const float* v0 = A.v0 ? A.v0 + (long long)b * D.N : nullptr;
+        float* r = A.r + (long long)b * D.N;
+        float* dd = A.d ? A.d + (long long)b * D.N : nullptr;
+        float v[PY];
 #pragma unroll
-            for (int half = kMaxOutputs / 2; half >= 1; half /= 2) {
-                const bool up = lane & (2 * half);
+        for (int q = 0; q < PY; ++q) {
+            v[q] = v0 ? v0[tile.own[q]] : 0.0f;
+            if (tile.ok(q)) r[tile.own[q]] = sigmoid(v[q]);
+        }
+        int mark = D.k - A.c % D.k;                          // steps to the next checkpoint
+        for (int tt = 1; tt <= A.nt; ++tt) {
+            tile.wait();
+            fetch((slot + kTileDepth - 1) % kTileDepth);
+            const float* x = tile.corner(win[slot]);
+            slot = (slot + 1) % kTileDepth;
+            float I[PY];
 #pragma unroll
-                for (int j = 0; j < half; ++j) {
-                    const float send = up ? c[j] : c[j + half];
-                    const float keep = up ? c[j + half] : c[j];
-                    c[j] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, 2 * half);
+            for (int q = 0; q < PY; ++q) I[q] = 0.0f;
+#pragma unroll
+            for (int wr = 0; wr < PY + F - 1; ++wr) {
+                float xr[F];
+#pragma unroll
+                for (int kc = 0; kc < F; ++kc) xr[kc] = x[wr * W::WX + kc];
+#pragma unroll
+                for (int q = 0; q < PY; ++q) {
+                    const int kr = wr - q;
+                    if (kr < 0 || kr >= F) continue;
+#pragma unroll
+                    for (int kc = 0; kc < F; ++kc) I[q] = __fmaf_rn(wk[q][kr * F + kc], xr[kc], I[q]);
                 }
             }
-            const float y_lane = c[0] + __shfl_xor_sync(0xFFFFFFFFu, c[0], 1);
-            if ((lane & 1) == 0 && (lane >> 1) < D.O) red[warp][lane >> 1] = y_lane;
-            __syncthreads();
-            if (threadIdx.x < D.O) {
-                float y = 0.0f;
-                for (int w = 0; w < kBlock / 32; ++w) y += red[w][threadIdx.x];
-                ypart[((long long)b * D.nchunk + tile) * D.O + threadIdx.x] = y;
-            }
-        }
-    }
-}
-
-// Many timesteps of one batch element on one 16 x 16 tile in one launch.
-// A layer's own state is pointwise in time and layer l at step t reads layer
-// l-1 at step t-1 within +-h, so the tile of the last layer for any number
-// of steps needs layer l over the tile plus (L-1-l) h on each side and
-// nothing else: the CTA keeps v and r of those regions (and the stencil
-// weights of layers >= 1 over them) in shared memory and advances them step
-// by step with no global exchange.  Halo neurons are computed exactly as
-// their owners compute them (same inputs, same operations), so each CTA's
-// tile neurons equal those of any other split -- and the backward pass's
-// recompute from a checkpoint reproduces the forward states bit for bit.
-//   mode 0 (forward): steps 1..T from v = 0; writes the checkpoints
-//     (t % k == 0, t < T) and the per-tile readout partials ypart.
-//   mode 1 (recompute): nt steps from the checkpointed v at step c; writes
-//     the segment's r (steps c..c+nt) and drives d, which is all the adjoint
-//     kernels read.
-// The input of the next step is fetched with cp.async during the current one.
-struct FusedRegions {
-    int L, H;
-    __device__ __host__ int side(int l) const { return kTileSide + 2 * (L - 1 - l) * H; }
-    __device__ __host__ int off(int l) const {      // float offset of region l
-        int o = 0;
-        for (int m = 0; m < l; ++m) o += side(m) * side(m);
-        return o;
-    }
-    __device__ __host__ int total() const { return off(L); }
-    __device__ __host__ int woff(int l, int K) const {   // weights of layers 1..l-1
-        int o = 0;
-        for (int m = 1; m < l; ++m) o += K * side(m) * side(m);
-        return o;
-    }
-};
-
-template <int F>
-__host__ __device__ inline size_t fused_smem_floats(int L) {
-    const FusedRegions R{L, F / 2};
-    const int s0 = R.side(0);
-    // v, r (two buffers), input (two buffers), weights, readout weights of
-    // the tile, readout partials, a_l, and two per-position tables (32-bit ints)
-    return (size_t)3 * R.total() + 2 * s0 * s0 + R.woff(L, F * F) +
-           kMaxOutputs * kBlock + 2 * (kBlock / 32) * kMaxOutputs + L + 2 * R.total();
-}
-
-__device__ __forceinline__ void cp_async_f32_zfill(float* dst, const float* src, bool valid) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
-                     (unsigned)__cvta_generic_to_shared(dst)),
-                 "l"(src), "r"(valid ? 4 : 0)
-                 : "memory");
-}
-
-constexpr int kOwnBit = 1 << 30;
-
-template <int F>
-__global__ void __launch_bounds__(kBlock) k_rate_fused(
-    Dims D, int mode, int c, int nt, const float* __restrict__ x, const float* __restrict__ wt,
-    const float* __restrict__ wo, const float* __restrict__ tau, const float* __restrict__ v0,
-    float* __restrict__ ckpt, float* __restrict__ ypart, float* __restrict__ seg_r,
-    float* __restrict__ seg_d) {
-    constexpr int H = F / 2, K = F * F;
-    extern __shared__ float fs[];
-    const FusedRegions R{D.L, H};
-    const int tot = R.total(), s0 = R.side(0);
-    // weights first, then v, r[2], x[2], readout weights,
-    // readout partials, a_l, tables
-    float* ws = fs;                                          // [k][position], layers >= 1
-    float* vs = ws + R.woff(D.L, K);
-    float* rs = vs + tot;
-    float* xs = vs + 3 * tot;
-    float* ows = xs + 2 * s0 * s0;                           // [O][256] readout weights
-    float* red = ows + kMaxOutputs * kBlock;                 // [2][8][16]
-    float* as = red + 2 * (kBlock / 32) * kMaxOutputs;       // dt / tau_l
-    // per region position: its global index, with kOwnBit for tile neurons,
-    // or -1 outside the layer; and the offset of its stencil window in the
-    // previous layer's region
-    int* info = reinterpret_cast<int*>(as + D.L);
-    int* sbase = info + tot;
-    const int tiles_x = (D.cols + kTileSide - 1) / kTileSide;
-    const int tile = blockIdx.x, b = blockIdx.y;
-    const int ty0 = (tile / tiles_x) * kTileSide, tx0 = (tile % tiles_x) * kTileSide;
-    const int tid = threadIdx.x;
-    const long long S = D.S;
-
-    // tables, initial state, weights
-    for (int l = 0, o = 0, op = 0, sp = 0, wofs = 0; l < D.L; ++l) {
-        const int sd = R.side(l), q = (D.L - 1 - l) * H;
-        for (int p = tid; p < sd * sd; p += kBlock) {
-            const int py = p / sd, px = p - py * sd;
-            const int gy = ty0 - q + py, gx = tx0 - q + px;
-            const bool in = gy >= 0 && gy < D.rows && gx >= 0 && gx < D.cols;
-            const int gi = in ? gy * D.cols + gx : -1;
-            const bool own = py >= q && py < q + kTileSide && px >= q && px < q + kTileSide;
-            info[o + p] = in ? (gi | (own ? kOwnBit : 0)) : -1;
-            sbase[o + p] = l >= 1 ? op + py * sp + px : 0;
-            const long long gl = ((long long)l * D.B + b) * D.N + gi;
-            const float v = (in && v0) ? v0[gl] : 0.0f;
-            const float r = in ? sigmoid(v) : 0.0f;
-            vs[o + p] = v;
-            rs[o + p] = r;
-            rs[tot + o + p] = 0.0f;
-            if (mode == 1 && in && own) seg_r[gl] = r;
-            if (l >= 1) {
+            r += A.r_t;
 #pragma unroll
-                for (int k = 0; k < K; ++k)
-                    ws[wofs + k * sd * sd + p] =
-                        in ? __ldg(wt + ((long long)(l - 1) * K + k) * D.N + gi) : 0.0f;
+            for (int q = 0; q < PY; ++q) {
+                I[q] -= v[q];
+                v[q] = v[q] + a * I[q];
+                if (tile.ok(q)) r[tile.own[q]] = sigmoid(v[q]);
             }
-            if (l == D.L - 1) {                               // the tile itself: p = tid
-                for (int k = 0; k < kMaxOutputs; ++k)
-                    ows[k * kBlock + p] = (in && k < D.O) ? __ldg(wo + (long long)k * D.N + gi) : 0.0f;
+            if (dd) {
+#pragma unroll
+                for (int q = 0; q < PY; ++q)
+                    if (tile.ok(q)) dd[tile.own[q]] = I[q];
+                dd += D.S;
+            }
+            if (--mark == 0) {
+                mark = D.k;
+                const int t = A.c + tt;
+                if (A.ckpt && t < D.T)
+#pragma unroll
+                    for (int q = 0; q < PY; ++q)
+                        if (tile.ok(q))
+                            A.ckpt[t / D.k * D.S + (long long)b * D.N + tile.own[q]] = v[q];
             }
         }
-        op = o;
-        sp = sd;
-        o += sd * sd;
-        if (l >= 1) wofs += K * sd * sd;
+        if (A.v1)
+#pragma unroll
+            for (int q = 0; q < PY; ++q)
+                if (tile.ok(q)) A.v1[(long long)b * D.N + tile.own[q]] = v[q];
     }
-    for (int l = tid; l < D.L; l += kBlock) as[l] = D.dt / __ldg(tau + l);
+}
+
+// Layer 0, driven by x alone: a thread per (batch element, neuron).
+constexpr int kAhead = 10;                   // timesteps whose loads are in flight
+
+__global__ void __launch_bounds__(kBlock) k_rate_input(Dims D, LayerArgs A,
+                                                       const float* __restrict__ x,
+                                                       const float* __restrict__ tau) {
+    const long long i = (long long)blockIdx.x * kBlock + threadIdx.x;
+    wait_for_previous();
+    if (i >= D.BN) return;
+    const float a = D.dt / __ldg(tau);
+    float v = A.v0 ? A.v0[i] : 0.0f;
+    A.r[i] = sigmoid(v);
+    const float* xt = x + (long long)A.c * D.BN + i;
+    for (int t0 = 0; t0 < A.nt; t0 += kAhead) {
+        float in[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            in[u] = t0 + u < A.nt ? __ldg(xt + (t0 + u) * D.BN) : 0.0f;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int tt = t0 + u + 1, t = A.c + tt;
+            if (tt > A.nt) break;
+            const float d = in[u] - v;
+            v = v + a * d;
+            A.r[tt * A.r_t + i] = sigmoid(v);
+            if (A.d) A.d[(tt - 1) * D.S + i] = d;
+            if (A.ckpt && t % D.k == 0 && t < D.T) A.ckpt[t / D.k * D.S + i] = v;
+        }
+    }
+    if (A.v1) A.v1[i] = v;
+}
+
+// y[t][b][o] = sum_i R[o][i] r[t][b][i] and the squared error of (t, b), for
+// rows (t, b) of a chunk.  A CTA takes kReadRows rows, so that a readout weight
+// read from L2 serves all of them, and its warps a slice of the neurons each (V
+// consecutive ones to a lane).  A lane sums its neurons in order, a butterfly
+// adds the lanes, and the warps are added in order.
+constexpr int kReadRows = 8;
+
+// Sums c[] over the warp: of C = 2 * HALF sums a lane keeps half, exchanging the
+// other half with the lane M away, and so on down to the neighbour.
+template <int HALF, int M = 16, int C>
+__device__ __forceinline__ void butterfly(float (&c)[C], int lane) {
+    if constexpr (M >= 1) {
+        const bool up = lane & M;
+#pragma unroll
+        for (int e = 0; e < HALF; ++e) {
+            const float send = up ? c[e] : c[e + HALF];
+            const float keep = up ? c[e + HALF] : c[e];
+            c[e] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, M);
+        }
+        butterfly<HALF / 2, M / 2>(c, lane);
+    }
+}
+
+template <int V>
+__device__ __forceinline__ void load_row(const float* p, float (&v)[V]) {
+    if constexpr (V == 4) {
+        const float4 t = *reinterpret_cast<const float4*>(p);
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+        v[0] = *p;
+    }
+}
+
+template <int V>
+__global__ void __launch_bounds__(kBlock, 1) k_rate_readout(Dims D, int c, int nt,
+                                                            const float* __restrict__ r,
+                                                            long long r_t,
+                                                            const float* __restrict__ wo,
+                                                            const float* __restrict__ target,
+                                                            float* __restrict__ y,
+                                                            float* __restrict__ loss_tb) {
+    constexpr int C = kReadRows * kMaxOutputs, STEP = 32 * V;
+    __shared__ float red[kBlock / 32][C];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long rows = (long long)nt * D.B, row0 = (long long)blockIdx.x * kReadRows;
+    const float* src[kReadRows];
+#pragma unroll
+    for (int j = 0; j < kReadRows; ++j) {
+        const long long row = min(row0 + j, rows - 1);
+        src[j] = r + (row / D.B + 1) * r_t + row % D.B * D.N;
+    }
+    float acc[C];
+#pragma unroll
+    for (int e = 0; e < C; ++e) acc[e] = 0.0f;
+    wait_for_previous();
+    const int steps = (D.N + STEP - 1) / STEP, per = (steps + kBlock / 32 - 1) / (kBlock / 32);
+    const int k1 = min(D.N, (warp + 1) * per * STEP);
+    for (int k = warp * per * STEP + lane * V; k < k1; k += STEP) {
+        float rv[kReadRows][V];
+#pragma unroll
+        for (int j = 0; j < kReadRows; ++j) load_row<V>(src[j] + k, rv[j]);
+#pragma unroll
+        for (int o = 0; o < kMaxOutputs; ++o) {
+            if (o >= D.O) break;
+            float wv[V];
+#pragma unroll
+            for (int q = 0; q < V; ++q) wv[q] = __ldg(wo + (long long)o * D.N + k + q);
+#pragma unroll
+            for (int j = 0; j < kReadRows; ++j)
+#pragma unroll
+                for (int q = 0; q < V; ++q)
+                    acc[j * kMaxOutputs + o] = __fmaf_rn(wv[q], rv[j][q], acc[j * kMaxOutputs + o]);
+        }
+    }
+    butterfly<C / 2>(acc, lane);                             // sums C / 32 * lane and on
+#pragma unroll
+    for (int e = 0; e < C / 32; ++e) red[warp][lane * (C / 32) + e] = acc[e];
     __syncthreads();
-    {
-        const float* xt = x + ((long long)c * D.B + b) * D.N;
-        for (int p = tid; p < s0 * s0; p += kBlock) {
-            const int code = info[p];
-            cp_async_f32_zfill(&xs[p], code >= 0 ? xt + (code & (kOwnBit - 1)) : xt, code >= 0);
-        }
-        asm volatile("cp.async.commit_group;\ncp.async.wait_all;\n" ::: "memory");
+    if (threadIdx.x >= C) return;
+    const int j = threadIdx.x / kMaxOutputs, o = threadIdx.x % kMaxOutputs;
+    const long long tb = (long long)c * D.B + row0 + j;
+    float err = 0.0f;
+    if (row0 + j < rows && o < D.O) {
+        float sum = 0.0f;
+#pragma unroll
+        for (int q = 0; q < kBlock / 32; ++q) sum += red[q][threadIdx.x];
+        y[tb * D.O + o] = sum;
+        err = sum - target[tb % D.B * D.O + o];
+        err *= err;
     }
-    __syncthreads();
-
-    // The last layer's region is the tile itself: thread tid owns position
-    // tid, whose weights (small fields) it keeps in registers.
-    constexpr bool kRegLast = F <= 5;
-    float wlast[kRegLast ? K : 1];
-    if (kRegLast && D.L >= 2) {
-        const float* wl = ws + R.woff(D.L - 1, K) + tid;
 #pragma unroll
-        for (int k = 0; k < (kRegLast ? K : 1); ++k) wlast[k] = wl[k * kTileSide * kTileSide];
-    }
-    // Layer 1, when it is not the last: the weights of the thread's first
-    // position (p = tid) in registers too, the other positions' from shared
-    // memory.
-    constexpr bool kRegMid = F <= 5;
-    float wmid[kRegMid ? K : 1];
-    if (kRegMid && D.L >= 3) {
-        const int sd1 = R.side(1);
-        const float* wl = ws + R.woff(1, K) + tid;
-#pragma unroll
-        for (int k = 0; k < (kRegMid ? K : 1); ++k) wmid[k] = wl[k * sd1 * sd1];
-    }
-    const int lane = tid & 31, warp = tid >> 5;
-    for (int tt = 1; tt <= nt; ++tt) {
-        const int t = c + tt, cur = (tt - 1) & 1;
-        const float* r_old = rs + cur * tot;
-        float* r_new = rs + (cur ^ 1) * tot;
-        const float* x_cur = xs + cur * s0 * s0;
-        if (tt < nt) {                                       // next step's input
-            const float* xt = x + ((long long)t * D.B + b) * D.N;
-            float* xn = xs + (cur ^ 1) * s0 * s0;
-            for (int p = tid; p < s0 * s0; p += kBlock) {
-                const int code = info[p];
-                cp_async_f32_zfill(&xn[p], code >= 0 ? xt + (code & (kOwnBit - 1)) : xt, code >= 0);
-            }
-            asm volatile("cp.async.commit_group;\n" ::: "memory");
-        }
-        const bool store_ckpt = mode == 0 && t % D.k == 0 && t < D.T;
-        float r_last = 0.0f;                                  // tile neuron of the last layer
-        for (int l = 0, o = 0, wofs = 0; l < D.L; ++l) {
-            const int sd = R.side(l), sd2 = sd * sd, sp = sd + 2 * H;
-            const float a = as[l];
-            for (int p = tid; p < sd2; p += kBlock) {
-                const int code = info[o + p];
-                if (code < 0) continue;
-                float I;
-                if (l == 0) {
-                    I = x_cur[p];
-                } else {
-                    // one partial sum per kernel row, rows added in order
-                    const float* src = r_old + sbase[o + p];
-                    const float* wl = ws + wofs + p;
-                    float part[F];
-                    if (kRegLast && l == D.L - 1) {
-#pragma unroll
-                        for (int kr = 0; kr < F; ++kr) {
-                            part[kr] = 0.0f;
-#pragma unroll
-                            for (int kc = 0; kc < F; ++kc)
-                                part[kr] = __fmaf_rn(wlast[kRegLast ? kr * F + kc : 0],
-                                                     src[kr * sp + kc], part[kr]);
-                        }
-                    } else if (kRegMid && l == 1 && p == tid) {
-#pragma unroll
-                        for (int kr = 0; kr < F; ++kr) {
-                            part[kr] = 0.0f;
-#pragma unroll
-                            for (int kc = 0; kc < F; ++kc)
-                                part[kr] = __fmaf_rn(wmid[kRegMid ? kr * F + kc : 0],
-                                                     src[kr * sp + kc], part[kr]);
-                        }
-                    } else {
-#pragma unroll
-                        for (int kr = 0; kr < F; ++kr) {
-                            part[kr] = 0.0f;
-#pragma unroll
-                            for (int kc = 0; kc < F; ++kc)
-                                part[kr] = __fmaf_rn(wl[(kr * F + kc) * sd2], src[kr * sp + kc],
-                                                     part[kr]);
-                        }
-                    }
-                    I = 0.0f;
-#pragma unroll
-                    for (int kr = 0; kr < F; ++kr) I += part[kr];
-                }
-                const float vp = vs[o + p];
-                const float d = -vp + I;
-                const float vn = vp + a * d;
-                const float rn = sigmoid(vn);
-                vs[o + p] = vn;
-                r_new[o + p] = rn;
-                if (code & kOwnBit) {
-                    const long long gl = ((long long)l * D.B + b) * D.N + (code & (kOwnBit - 1));
-                    if (mode == 1) {
-                        seg_r[tt * S + gl] = rn;
-                        seg_d[(tt - 1) * S + gl] = d;
-                    } else if (store_ckpt) {
-                        ckpt[(long long)(t / D.k) * S + gl] = vn;
-                    }
-                    if (l == D.L - 1) r_last = rn;
-                }
-            }
-            o += sd2;
-            if (l >= 1) wofs += K * sd2;
-        }
-        if (mode == 0) {
-            // readout of the tile's last-layer neurons (thread tid owns
-            // position tid of the 16 x 16 region): butterfly transpose
-            // reduction per warp, warps added in order
-            float cv[kMaxOutputs];
-#pragma unroll
-            for (int q = 0; q < kMaxOutputs; ++q) cv[q] = ows[q * kBlock + tid] * r_last;
-#pragma unroll
-            for (int half = kMaxOutputs / 2; half >= 1; half /= 2) {
-                const bool up = lane & (2 * half);
-#pragma unroll
-                for (int j = 0; j < half; ++j) {
-                    const float send = up ? cv[j] : cv[j + half];
-                    const float keep = up ? cv[j + half] : cv[j];
-                    cv[j] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, 2 * half);
-                }
-            }
-            const float y_lane = cv[0] + __shfl_xor_sync(0xFFFFFFFFu, cv[0], 1);
-            float* rd = red + cur * (kBlock / 32) * kMaxOutputs;
-            if ((lane & 1) == 0 && (lane >> 1) < D.O) rd[warp * kMaxOutputs + (lane >> 1)] = y_lane;
-        }
-        asm volatile("cp.async.wait_all;\n" ::: "memory");
-        __syncthreads();
-        if (mode == 0 && tid < D.O) {
-            const float* rd = red + cur * (kBlock / 32) * kMaxOutputs;
-            float y = 0.0f;
-            for (int w = 0; w < kBlock / 32; ++w) y += rd[w * kMaxOutputs + tid];
-            ypart[(((long long)(t - 1) * D.B + b) * D.nchunk + tile) * D.O + tid] = y;
-        }
-    }
-}
-
-// r = sigmoid(v) for a whole state (checkpoint reload / initial state).
-__global__ void k_rate_rates(long long S, const float* __restrict__ v, float* __restrict__ r) {
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx < S) r[idx] = sigmoid(v[idx]);
-}
-
-// y[t][b][o] = sum of the blocks' partial readouts (block order) and the
-// squared error of each (t, b).
-__global__ void k_rate_finish(Dims D, const float* __restrict__ ypart,
-                              const float* __restrict__ target, float* __restrict__ y,
-                              float* __restrict__ loss_tb) {
-    long long tb = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (tb >= (long long)D.T * D.B) return;
-    const int b = (int)(tb % D.B);
-    const float* yp = ypart + tb * D.nchunk * D.O;
-    float e = 0.0f;
-    for (int o = 0; o < D.O; ++o) {
-        float s = 0.0f;
-        for (int c = 0; c < D.nchunk; ++c) s += yp[(long long)c * D.O + o];
-        y[tb * D.O + o] = s;
-        const float diff = s - target[(long long)b * D.O + o];
-        e += diff * diff;
-    }
-    loss_tb[tb] = e;
+    for (int m = kMaxOutputs / 2; m >= 1; m /= 2) err += __shfl_xor_sync(0xFFFFFFFFu, err, m);
+    if (o == 0 && row0 + j < rows) loss_tb[tb] = err;
 }
 
 // loss = sum over (t, b) of the squared errors / (T B O): 256 strided
 // partial sums reduced in a fixed tree.
 __global__ void __launch_bounds__(256) k_rate_loss(Dims D, const float* __restrict__ loss_tb,
                                                    float* __restrict__ loss) {
+    wait_for_previous();
     __shared__ float sm[256];
     const int tid = threadIdx.x;
     float s = 0.0f;
@@ -529,259 +461,411 @@ __global__ void __launch_bounds__(256) k_rate_loss(Dims D, const float* __restri
 // gy[t][b][o] = gscale * (y - target), for every step.
 __global__ void k_rate_gy(Dims D, float gscale, const float* __restrict__ y,
                           const float* __restrict__ target, float* __restrict__ gy) {
+    wait_for_previous();
     long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (long long)D.T * D.B * D.O) return;
     const long long bo = e % ((long long)D.B * D.O);
     gy[e] = gscale * (y[e] - target[bo]);
 }
 
-// Adjoint of one timestep, grid like the step kernel: lambda[t] from
-// lambda[t+1] (the next layer's inputs at t+1 read the rates of t).  Neuron i
-// of layer l feeds destinations j = i + h - (kr, kc) of layer l+1; the thread
-// keeps those field x field weights (zero where j is outside the layer) in
-// registers, and per batch element the CTA stages a_{l+1} * lambda_{l+1}[t+1]
-// of its tile plus halo in shared memory, double-buffered like the step.
-template <int F>
-__global__ void __launch_bounds__(kBlock) k_rate_lambda(
-    Dims D, const float* wt, const float* wo, const float* __restrict__ tau,
-    const float* __restrict__ gy_t, const float* __restrict__ r_t,
-    const float* __restrict__ lam_next, float* __restrict__ lam, float* __restrict__ dx_t) {
-    using W = Halo<F>;
+// ---------------------------------------------------------------------------
+// Adjoint of one layer through a segment's steps, last first.  What the layer
+// below and the weight gradients read is P_l[t] = a_l lambda_l[t], so that is
+// what is stored (P[tt - 1] for step c + tt; for layer 0 it is dx).  lambda
+// itself and the sum of lambda d over time stay in registers and cross segments
+// in `lam` and `lamd` ([B][N] of this layer).
+// ---------------------------------------------------------------------------
+struct AdjointArgs {
+    const float* r;          // this layer's rates at c .. c + nt, S apart
+    const float* d;          // its drives, S apart
+    const float* next;       // P_{l+1} of steps c + 1 .. c + nt, S apart
+    const float* next_carry; // P_{l+1} of step c + nt + 1
+    bool first;              // nothing is carried yet: the carries are zero (next_carry is)
+    float* P;                // P_l, P_t apart, or null
+    long long P_t;
+    float* carry;            // P_l of step c + 1 again, for the segment before, or null
+    float *lam, *lamd;
+    int nt, bg;
+};
+
+struct AdjointNeuron {
+    float lam, lamd;
+    __device__ float step(float r, float d, float g, float a) {
+        lam = r * (1.0f - r) * g + (1.0f - a) * lam;
+        lamd = __fmaf_rn(lam, d, lamd);
+        return a * lam;
+    }
+};
+
+// Neuron i of layer l feeds destinations j = i + h - (kr, kc) of layer l + 1:
+// the thread keeps those weights, zero where j lies outside the layer.
+template <int F, int PY, int V>
+__global__ void __launch_bounds__(kTileThreads, tile_ctas(F, PY) > 1 ? 6 : 1) k_rate_adjoint(Dims D, int l, AdjointArgs A,
+                                                               const float* __restrict__ wt,
+                                                               const float* __restrict__ tau) {
+    using W = Tile<F, PY, V>;
     constexpr int H = W::H;
-    __shared__ float P[2][W::SIDE][W::PITCH];
-    const int tiles_x = (D.cols + kTileSide - 1) / kTileSide;
-    const int tile = blockIdx.x, l = blockIdx.y;
-    const int ty0 = (tile / tiles_x) * kTileSide, tx0 = (tile % tiles_x) * kTileSide;
-    const int tr = threadIdx.x / kTileSide, tc = threadIdx.x % kTileSide;
-    const int ir = ty0 + tr, ic = tx0 + tc;
-    const bool ok = ir < D.rows && ic < D.cols;
-    const int i = ir * D.cols + ic;
-    const bool last = l == D.L - 1;
+    __shared__ __align__(16) float win[kTileDepth][W::COUNT];
+    const W tile(D, win);
     const float a = D.dt / __ldg(tau + l);
-    const float a1 = last ? 0.0f : D.dt / __ldg(tau + l + 1);
-    float wk[F * F];
+    float wk[PY][F * F];
+    const float* wl = wt + (long long)l * F * F * D.N;
 #pragma unroll
-    for (int kr = 0; kr < F; ++kr)
+    for (int k = 0; k < F * F; ++k, wl += D.N) {
+        const int jc = tile.x0 + tile.lane + H - k % F;
+        const bool col = jc >= 0 && jc < D.cols;
 #pragma unroll
-        for (int kc = 0; kc < F; ++kc) {
-            const int jr = ir + H - kr, jc = ic + H - kc;
-            wk[kr * F + kc] = (!last && ok && jr >= 0 && jr < D.rows && jc >= 0 && jc < D.cols)
-                                  ? wt[((long long)l * F * F + kr * F + kc) * D.N + jr * D.cols + jc]
-                                  : 0.0f;
+        for (int q = 0; q < PY; ++q) {
+            const int jr = tile.y0 + tile.row + q + H - k / F;
+            wk[q][k] = 0.0f;
+            if (col && jr >= 0 && jr < D.rows) wk[q][k] = __ldg(wl + (unsigned)(jr * D.cols + jc));
         }
+    }
+    wait_for_previous();
+    const int b0 = blockIdx.y * A.bg, b1 = min(D.B, b0 + A.bg);
+    int pb = b0, pt = A.nt, slot = 0;                        // the next item to fetch
+    auto fetch = [&](int into) {
+        const float* src = (pt == A.nt ? A.next_carry : A.next + pt * D.S) + (long long)pb * D.N;
+        tile.fetch(win[into], src, pb < b1);
+        if (--pt == 0) { pt = A.nt; ++pb; }
+    };
+#pragma unroll
+    for (int s = 0; s < kTileDepth - 1; ++s) fetch(s);
+    for (int b = b0; b < b1; ++b) {
+        const long long bn = (long long)b * D.N;
+        const float *r = A.r + A.nt * D.S + bn, *dd = A.d + (A.nt - 1) * D.S + bn;
+        float* P = A.P ? A.P + (A.nt - 1) * A.P_t + bn : nullptr;
+        AdjointNeuron n[PY];
+        float p[PY];
+#pragma unroll
+        for (int q = 0; q < PY; ++q) {
+            n[q].lam = A.first ? 0.0f : (A.lam + bn)[tile.own[q]];
+            n[q].lamd = A.first ? 0.0f : (A.lamd + bn)[tile.own[q]];
+        }
+        float rn[PY], dn[PY];                                // the next step's, loaded ahead
+#pragma unroll
+        for (int q = 0; q < PY; ++q) {
+            rn[q] = r[tile.own[q]];
+            dn[q] = dd[tile.own[q]];
+        }
+        for (int tt = A.nt; tt >= 1; --tt) {
+            float rv[PY], dv[PY];
+            if (tt > 1) {
+                r -= D.S;
+                dd -= D.S;
+            }
+#pragma unroll
+            for (int q = 0; q < PY; ++q) {
+                rv[q] = rn[q];
+                dv[q] = dn[q];
+                rn[q] = r[tile.own[q]];
+                dn[q] = dd[tile.own[q]];
+            }
+            tile.wait();
+            fetch((slot + kTileDepth - 1) % kTileDepth);
+            const float* x = tile.corner(win[slot]);
+            slot = (slot + 1) % kTileDepth;
+            float g[PY];
+#pragma unroll
+            for (int q = 0; q < PY; ++q) g[q] = 0.0f;
+            // window rows from the last, so that kernel rows come in order
+#pragma unroll
+            for (int wr = PY + F - 2; wr >= 0; --wr) {
+                float xr[F];
+#pragma unroll
+                for (int kc = 0; kc < F; ++kc) xr[kc] = x[wr * W::WX + 2 * H - kc];
+#pragma unroll
+                for (int q = 0; q < PY; ++q) {
+                    const int kr = q + 2 * H - wr;
+                    if (kr < 0 || kr >= F) continue;
+#pragma unroll
+                    for (int kc = 0; kc < F; ++kc) g[q] = __fmaf_rn(wk[q][kr * F + kc], xr[kc], g[q]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < PY; ++q) p[q] = n[q].step(rv[q], dv[q], g[q], a);
+            if (P) {
+#pragma unroll
+                for (int q = 0; q < PY; ++q)
+                    if (tile.ok(q)) P[tile.own[q]] = p[q];
+                P -= A.P_t;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < PY; ++q) {
+            if (!tile.ok(q)) continue;
+            (A.lam + bn)[tile.own[q]] = n[q].lam;
+            (A.lamd + bn)[tile.own[q]] = n[q].lamd;
+            if (A.carry) (A.carry + bn)[tile.own[q]] = p[q];
+        }
+    }
+}
+
+// The last layer, driven by the readout: grid (blocks of neurons, batch).
+// dloss/dy of kTopSteps steps at a time is kept in shared memory.
+constexpr int kTopSteps = 32;
+
+__global__ void __launch_bounds__(kBlock) k_rate_adjoint_top(Dims D, AdjointArgs A,
+                                                             const float* __restrict__ wo,
+                                                             const float* __restrict__ gy,
+                                                             const float* __restrict__ tau) {
+    __shared__ __align__(16) float gs[kTopSteps][kMaxOutputs];
+    const int i = blockIdx.x * kBlock + threadIdx.x, b = blockIdx.y;
+    const bool ok = i < D.N;
+    const unsigned own = ok ? i : 0;
+    const long long bn = (long long)b * D.N;
+    const float a = D.dt / __ldg(tau + D.L - 1);
     float wov[kMaxOutputs];
 #pragma unroll
-    for (int o = 0; o < kMaxOutputs; ++o)
-        wov[o] = (last && ok && o < D.O) ? wo[(long long)o * D.N + i] : 0.0f;
-    const int b0 = blockIdx.z * D.bg, b1 = min(D.B, b0 + D.bg);
-    const float* ln = last ? nullptr : lam_next + (long long)(l + 1) * D.B * D.N;
-    const W halo(D, ty0, tx0);
-    // launched as a programmatic dependent of the previous step's adjoint:
-    // the weights above are loaded while it drains; nothing it writes is
-    // read before it has completed
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    float pre[W::PER];
-    if (!last) halo.fetch(ln + (long long)b0 * D.N, a1, pre);
-    for (int b = b0, buf = 0; b < b1; ++b, buf ^= 1) {
-        if (!last) halo.stage(pre, &P[buf][0][0]);
-        const long long idx = ((long long)l * D.B + b) * D.N + i;
-        const float r = ok ? r_t[idx] : 0.0f;
-        const float own = ok ? lam_next[idx] : 0.0f;
+    for (int o = 0; o < kMaxOutputs; ++o) wov[o] = o < D.O ? __ldg(wo + (long long)o * D.N + own) : 0.0f;
+    wait_for_previous();
+    AdjointNeuron n{A.first ? 0.0f : (A.lam + bn)[own], A.first ? 0.0f : (A.lamd + bn)[own]};
+    const float *r = A.r + A.nt * D.S + bn, *d = A.d + (A.nt - 1) * D.S + bn;
+    float* P = A.P ? A.P + (A.nt - 1) * A.P_t + bn : nullptr;
+    float p = 0.0f;
+    for (int t1 = A.nt; t1 >= 1; t1 -= kTopSteps) {
+        const int steps = min(kTopSteps, t1);
+        float rv[kAhead], dv[kAhead];
+        auto load = [&](int u0) {
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (u0 + u < steps) {
+                    rv[u] = r[own];
+                    dv[u] = d[own];
+                    r -= D.S;
+                    d -= D.S;
+                }
+        };
+        load(0);                                             // in flight while gs is staged
         __syncthreads();
-        if (!last && b + 1 < b1) halo.fetch(ln + (long long)(b + 1) * D.N, a1, pre);
-        if (ok) {
-            float g = 0.0f;
-            if (last) {
+        for (int e = threadIdx.x; e < steps * kMaxOutputs; e += kBlock) {
+            const int u = e / kMaxOutputs, o = e % kMaxOutputs;
+            gs[u][o] = o < D.O ? __ldg(gy + ((long long)(t1 - u - 1) * D.B + b) * D.O + o) : 0.0f;
+        }
+        __syncthreads();
+        for (int u0 = 0; u0 < steps; u0 += kAhead) {
+            if (u0 > 0) load(u0);
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                if (u0 + u >= steps) break;
+                float g = 0.0f;
 #pragma unroll
                 for (int o = 0; o < kMaxOutputs; ++o)
-                    if (o < D.O) g += wov[o] * __ldg(gy_t + (long long)b * D.O + o);
-            } else {
-                float part[F];
-#pragma unroll
-                for (int kr = 0; kr < F; ++kr) {
-                    part[kr] = 0.0f;
-#pragma unroll
-                    for (int kc = 0; kc < F; ++kc)
-                        part[kr] = __fmaf_rn(wk[kr * F + kc], P[buf][tr + 2 * H - kr][tc + 2 * H - kc],
-                                             part[kr]);
+                    if (o < D.O) g = __fmaf_rn(wov[o], gs[u0 + u][o], g);
+                p = n.step(rv[u], dv[u], g, a);
+                if (P) {
+                    if (ok) P[own] = p;
+                    P -= A.P_t;
                 }
-#pragma unroll
-                for (int kr = 0; kr < F; ++kr) g += part[kr];
             }
-            const float lv = r * (1.0f - r) * g + (1.0f - a) * own;
-            lam[idx] = lv;
-            if (l == 0 && dx_t) dx_t[(long long)b * D.N + i] = a * lv;
         }
-    }
-}
-
-// The dR kernel below takes the batch in kGroups groups of thread warps,
-// kUnroll elements' loads in flight at a time.
-constexpr int kGroups = 8;
-constexpr int kUnroll = 8;
-
-// dW, staged: grid (tiles, layers >= 1, timesteps of the segment).  Thread
-// j of a 16 x 16 tile of layer l holds its F x F sums over the batch, in
-// batch order, of lambda_l[t][j] times the source rates of t-1 in its window;
-// per batch element the CTA stages the window (tile plus halo, zero outside
-// the layer) in shared memory, double-buffered with the next element fetched
-// into registers.  The step's totals go to part[tt][l-1][j][k], and
-// k_rate_dw_acc adds the steps latest first into dW: a fixed order that does
-// not depend on where the segments start.
-template <int F>
-__global__ void __launch_bounds__(kBlock) k_rate_dw_staged(Dims D, const float* __restrict__ seg_lam,
-                                                          const float* __restrict__ seg_r,
-                                                          float* __restrict__ part) {
-    using W = Halo<F>;
-    constexpr int K = F * F;
-    __shared__ float win[2][W::SIDE][W::PITCH];
-    const int tiles_x = (D.cols + kTileSide - 1) / kTileSide;
-    const int tile = blockIdx.x, l = 1 + blockIdx.y, tt = blockIdx.z;
-    const int ty0 = (tile / tiles_x) * kTileSide, tx0 = (tile % tiles_x) * kTileSide;
-    const int tr = threadIdx.x / kTileSide, tc = threadIdx.x % kTileSide;
-    const int jr = ty0 + tr, jc = tx0 + tc;
-    const bool ok = jr < D.rows && jc < D.cols;
-    const int j = jr * D.cols + jc;
-    const float* lam = seg_lam + (long long)tt * D.S + (long long)l * D.B * D.N;
-    const float* rp = seg_r + (long long)tt * D.S + (long long)(l - 1) * D.B * D.N;
-    const W halo(D, ty0, tx0);
-    float acc[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) acc[k] = 0.0f;
-    float pre[W::PER];
-    halo.fetch(rp, 1.0f, pre);
-    float lv = ok ? lam[j] : 0.0f;
-    for (int b = 0, buf = 0; b < D.B; ++b, buf ^= 1) {
-        halo.stage(pre, &win[buf][0][0]);
-        const float lcur = lv;
-        __syncthreads();
-        if (b + 1 < D.B) {
-            halo.fetch(rp + (long long)(b + 1) * D.N, 1.0f, pre);
-            lv = ok ? lam[(long long)(b + 1) * D.N + j] : 0.0f;
-        }
-#pragma unroll
-        for (int kr = 0; kr < F; ++kr)
-#pragma unroll
-            for (int kc = 0; kc < F; ++kc)
-                acc[kr * F + kc] = __fmaf_rn(lcur, win[buf][tr + kr][tc + kc], acc[kr * F + kc]);
     }
     if (!ok) return;
-    float* out = part + (((long long)tt * (D.L - 1) + (l - 1)) * D.N + j) * K;
-#pragma unroll
-    for (int k = 0; k < K; ++k) out[k] = acc[k];
+    (A.lam + bn)[own] = n.lam;
+    (A.lamd + bn)[own] = n.lamd;
+    if (A.carry) (A.carry + bn)[own] = p;
 }
 
-// dW[l-1][j][k] += a_l * part[tt] for the segment's steps, latest first.
-__global__ void k_rate_dw_acc(Dims D, int nt, const float* __restrict__ tau,
-                              const float* __restrict__ part, float* __restrict__ dw) {
-    const long long per = (long long)D.N * D.K, n = (long long)(D.L - 1) * per;
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n) return;
-    const float a = D.dt / __ldg(tau + 1 + (int)(e / per));
-    float acc = dw[e];
-    for (int tt = nt - 1; tt >= 0; --tt) acc += a * part[(long long)tt * n + e];
-    dw[e] = acc;
-}
-
-// dR, the same scheme: grid (tiles of 32 neurons i, timesteps), a CTA covers
-// its 32 neurons for every output with 8 groups of batch elements, the step's
-// total goes to part[tt][o][i] and k_rate_dwo_acc adds the steps latest first.
-__global__ void __launch_bounds__(kBlock) k_rate_dwo(Dims D, int t0, const float* __restrict__ gy,
-                                                    const float* __restrict__ seg_r,
-                                                    float* __restrict__ part) {
-    __shared__ float gsum[kGroups][32][kMaxOutputs + 1];
-    const int il = threadIdx.x & 31, g = threadIdx.x >> 5;
-    const int i = blockIdx.x * 32 + il, tt = blockIdx.y;
-    const bool ok = i < D.N;
-    const int bpg = (D.B + kGroups - 1) / kGroups;
-    const int b0 = g * bpg, b1 = min(D.B, b0 + bpg);
-    const int t = t0 + tt + 1;                          // 1-based step
-    const float* gt = gy + (long long)(t - 1) * D.B * D.O;
-    float st[kMaxOutputs];
+// dW of one timestep: grid (tiles, layers >= 1, timesteps of the segment).  A
+// thread holds the F x F sums over the batch, in batch order, of its PY neurons'
+// P_l[t] times the source rates of t - 1 in their windows.  The step's totals go
+// to part[tt][l-1][k][j], and k_rate_dw_acc adds the steps latest first: a fixed
+// order that does not depend on where the segments start.
+template <int F, int PY, int V>
+__global__ void __launch_bounds__(kTileThreads) k_rate_dw(Dims D, const float* __restrict__ seg_P,
+                                                          const float* __restrict__ seg_r,
+                                                          float* __restrict__ part) {
+    using W = Tile<F, PY, V>;
+    __shared__ __align__(16) float win[kTileDepth][W::COUNT];
+    __shared__ float own[kTileDepth][PY][kTileThreads];      // each thread its own P
+    const W tile(D, win);
+    const int l = 1 + blockIdx.y, tt = blockIdx.z;
+    const float* P = seg_P + tt * D.S + l * D.BN;
+    const float* r = seg_r + tt * D.S + (l - 1) * D.BN;
+    wait_for_previous();
+    float acc[PY][F * F];
 #pragma unroll
-    for (int o = 0; o < kMaxOutputs; ++o) st[o] = 0.0f;
-    if (ok) {
-        const float* r = seg_r + (long long)(tt + 1) * D.S + (long long)(D.L - 1) * D.B * D.N + i;
-        for (int bb = b0; bb < b1; bb += kUnroll) {
-            float rv[kUnroll];
+    for (int q = 0; q < PY; ++q)
 #pragma unroll
-            for (int u = 0; u < kUnroll; ++u) rv[u] = bb + u < b1 ? r[(long long)(bb + u) * D.N] : 0.0f;
+        for (int k = 0; k < F * F; ++k) acc[q][k] = 0.0f;
+    auto fetch = [&](int into, bool more) {
+        if (more)
 #pragma unroll
-            for (int u = 0; u < kUnroll; ++u) {
-                if (bb + u >= b1) break;
+            for (int q = 0; q < PY; ++q)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                                 (unsigned)__cvta_generic_to_shared(&own[into][q][threadIdx.x])),
+                             "l"(P + tile.own[q]) : "memory");
+        tile.fetch(win[into], r, more);
+        P += D.N;
+        r += D.N;
+    };
 #pragma unroll
-                for (int o = 0; o < kMaxOutputs; ++o)
-                    if (o < D.O) st[o] = __fmaf_rn(__ldg(gt + (long long)(bb + u) * D.O + o), rv[u], st[o]);
+    for (int s = 0; s < kTileDepth - 1; ++s) fetch(s, s < D.B);
+    for (int b = 0, slot = 0; b < D.B; ++b) {
+        tile.wait();
+        fetch((slot + kTileDepth - 1) % kTileDepth, b + kTileDepth - 1 < D.B);
+        float p[PY];
+#pragma unroll
+        for (int q = 0; q < PY; ++q) p[q] = own[slot][q][threadIdx.x];
+        const float* x = tile.corner(win[slot]);
+        slot = (slot + 1) % kTileDepth;
+#pragma unroll
+        for (int wr = 0; wr < PY + F - 1; ++wr) {
+            float xr[F];
+#pragma unroll
+            for (int kc = 0; kc < F; ++kc) xr[kc] = x[wr * W::WX + kc];
+#pragma unroll
+            for (int q = 0; q < PY; ++q) {
+                const int kr = wr - q;
+                if (kr < 0 || kr >= F) continue;
+#pragma unroll
+                for (int kc = 0; kc < F; ++kc)
+                    acc[q][kr * F + kc] = __fmaf_rn(p[q], xr[kc], acc[q][kr * F + kc]);
             }
         }
     }
+    float* out = part + tt * D.G + (long long)(l - 1) * F * F * D.N;
 #pragma unroll
-    for (int o = 0; o < kMaxOutputs; ++o) gsum[g][il][o] = st[o];
-    __syncthreads();
-    if (g == 0 && ok) {
+    for (int q = 0; q < PY; ++q)
 #pragma unroll
-        for (int o = 0; o < kMaxOutputs; ++o) {
-            if (o >= D.O) break;
-            float tot = 0.0f;
-            for (int q = 0; q < kGroups; ++q) tot += gsum[q][il][o];
-            part[((long long)tt * D.O + o) * D.N + i] = tot;
+        for (int k = 0; k < F * F; ++k)
+            if (tile.ok(q)) out[(long long)k * D.N + tile.own[q]] = acc[q][k];
+}
+
+// acc[e] += part[tt][e] for the segment's steps, latest first (the first segment
+// starts from zero): weight gradients [l-1][k][i], then dR [o][i].
+__global__ void k_rate_acc(Dims D, int nt, bool first, const float* __restrict__ part,
+                           float* __restrict__ acc) {
+    wait_for_previous();
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= D.G) return;
+    float s = first ? 0.0f : acc[e];
+    for (int t1 = nt - 1; t1 >= 0; t1 -= kAhead) {
+        float v[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) v[u] = t1 - u >= 0 ? part[(t1 - u) * D.G + e] : 0.0f;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (t1 - u >= 0) s += v[u];
+    }
+    acc[e] = s;
+}
+
+// The finished sums: dw[l][i][k] = acc[l][k][i], and dR.
+__global__ void k_rate_out(Dims D, const float* __restrict__ acc, float* __restrict__ dw,
+                           float* __restrict__ dwo) {
+    wait_for_previous();
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long per = (long long)D.N * D.K, weights = (D.L - 1) * per;
+    if (idx >= D.G) return;
+    if (idx >= weights) {
+        dwo[idx - weights] = acc[idx];
+        return;
+    }
+    const int l = (int)(idx / per), rem = (int)(idx - l * per), i = rem / D.K, k = rem - i * D.K;
+    dw[idx] = acc[l * per + (long long)k * D.N + i];
+}
+
+// dR, the same scheme: grid (blocks of neurons, timesteps).  A thread sums V
+// consecutive neurons for every output over the batch in order, kUnroll elements'
+// rates in flight; the step's dloss/dy is staged kReadoutBatch elements at a time.
+// The step's total goes to part[tt][o][i], and k_rate_acc adds the steps latest
+// first.
+constexpr int kUnroll = 16;
+constexpr int kReadoutBatch = 64;
+constexpr int kReadoutThreads = 64;
+
+template <int V>
+__global__ void __launch_bounds__(kReadoutThreads) k_rate_dwo(Dims D, const float* __restrict__ gy,
+                                                             const float* __restrict__ seg_r,
+                                                             float* __restrict__ part) {
+    __shared__ __align__(16) float gs[kReadoutBatch][kMaxOutputs];
+    const int i = (blockIdx.x * kReadoutThreads + threadIdx.x) * V, tt = blockIdx.y;
+    const bool ok = i < D.N;
+    const float* r = seg_r + (tt + 1) * D.S + (D.L - 1) * D.BN + (ok ? i : 0);
+    const float* gt = gy + (long long)tt * D.B * D.O;
+    float st[kMaxOutputs][V];
+#pragma unroll
+    for (int o = 0; o < kMaxOutputs; ++o)
+#pragma unroll
+        for (int q = 0; q < V; ++q) st[o][q] = 0.0f;
+    wait_for_previous();
+    for (int b0 = 0; b0 < D.B; b0 += kReadoutBatch) {
+        const int nb = min(kReadoutBatch, D.B - b0);
+        __syncthreads();
+        for (int e = threadIdx.x; e < nb * kMaxOutputs; e += kReadoutThreads) {
+            const int b = e / kMaxOutputs, o = e % kMaxOutputs;
+            gs[b][o] = o < D.O ? __ldg(gt + (long long)(b0 + b) * D.O + o) : 0.0f;
+        }
+        __syncthreads();
+        for (int b = 0; b < nb; b += kUnroll) {
+            float rv[kUnroll][V];
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u)
+                if (b + u < nb) load_row<V>(r + (long long)(b0 + b + u) * D.N, rv[u]);
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) {
+                if (b + u >= nb) break;
+#pragma unroll
+                for (int o = 0; o < kMaxOutputs; ++o)
+                    if (o < D.O)
+#pragma unroll
+                        for (int q = 0; q < V; ++q)
+                            st[o][q] = __fmaf_rn(gs[b + u][o], rv[u][q], st[o][q]);
+            }
         }
     }
+    if (!ok) return;
+#pragma unroll
+    for (int o = 0; o < kMaxOutputs; ++o)
+        if (o < D.O)
+#pragma unroll
+            for (int q = 0; q < V; ++q) part[tt * D.G + (long long)o * D.N + i + q] = st[o][q];
 }
 
-__global__ void k_rate_dwo_acc(Dims D, int nt, const float* __restrict__ part,
-                               float* __restrict__ dwo) {
-    const long long n = (long long)D.O * D.N;
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n) return;
-    float acc = dwo[e];
-    for (int tt = nt - 1; tt >= 0; --tt) acc += part[(long long)tt * n + e];
-    dwo[e] = acc;
-}
-
-// Partial sums of lambda * d per (timestep, layer): grid (kTauBlocks, L, nt),
-// each block a fixed strided slice of the batch x neurons reduced in a fixed
-// tree, written to part[t][l][block].
-__global__ void __launch_bounds__(256) k_rate_dtau_partial(Dims D, int t0,
-                                                           const float* __restrict__ seg_lam,
-                                                           const float* __restrict__ seg_d,
+// Per layer, sum of lamd over batch and neurons: grid (kTauBlocks, L), each
+// block a fixed strided slice reduced in a fixed tree.
+__global__ void __launch_bounds__(256) k_rate_dtau_partial(Dims D, const float* __restrict__ lamd,
                                                            float* __restrict__ part) {
+    wait_for_previous();
     __shared__ float sm[256];
-    const int l = blockIdx.y, tt = blockIdx.z, tid = threadIdx.x;
-    const long long per = (long long)D.B * D.N;
-    const long long off = (long long)tt * D.S + (long long)l * per;
+    const int l = blockIdx.y, tid = threadIdx.x;
+    const float* from = lamd + l * D.BN;
     float acc = 0.0f;
-    for (long long e = (long long)blockIdx.x * 256 + tid; e < per; e += (long long)gridDim.x * 256)
-        acc += seg_lam[off + e] * seg_d[off + e];
+    for (long long e = (long long)blockIdx.x * 256 + tid; e < D.BN; e += (long long)gridDim.x * 256)
+        acc += from[e];
     sm[tid] = acc;
     __syncthreads();
     for (int s = 128; s > 0; s >>= 1) {
         if (tid < s) sm[tid] += sm[tid + s];
         __syncthreads();
     }
-    if (tid == 0) part[((long long)(t0 + tt) * D.L + l) * kTauBlocks + blockIdx.x] = sm[0];
+    if (tid == 0) part[(long long)l * kTauBlocks + blockIdx.x] = sm[0];
 }
 
-// dtau_l = -(dt / tau_l^2) * sum over timesteps (latest first) of the step
-// sums; each step sum adds its blocks' partials in block order.
+// dtau_l = -(dt / tau_l^2) * sum of the layer's partials in block order.
 __global__ void __launch_bounds__(256) k_rate_dtau_final(Dims D, const float* __restrict__ tau,
                                                          const float* __restrict__ part,
-                                                         float* __restrict__ step_sums,
                                                          float* __restrict__ dtau) {
-    for (int e = threadIdx.x; e < D.T * D.L; e += blockDim.x) {
-        float st = 0.0f;
-        for (int q = 0; q < kTauBlocks; ++q) st += part[(long long)e * kTauBlocks + q];
-        step_sums[e] = st;
-    }
-    __syncthreads();
-    const int l = threadIdx.x;
+    wait_for_previous();
+    const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= D.L) return;
     float s = 0.0f;
-    for (int t = D.T - 1; t >= 0; --t) s += step_sums[(long long)t * D.L + l];
+    for (int q = 0; q < kTauBlocks; ++q) s += part[(long long)l * kTauBlocks + q];
     const float tv = __ldg(tau + l);
     dtau[l] = s * (-D.dt / (tv * tv));
 }
+
+// A segment's state of up to this many bytes stays in L2 and costs less than
+// the launches of shorter segments: small networks are not cut up more finely.
+constexpr long long kSegmentBytes = 64ll << 20;
+constexpr long long kChunkBytes = 64ll << 20;
+
+// States ([L][B][N]) of the segment buffers: lambda, sum of lambda d and two
+// carries, then rates [k+1], drives [k] and adjoints [k].  The forward pass keeps
+// two layers' chunks there.
+long long carry_states(const Dims& D) { return std::max(D.k + 1, 4); }
+long long chunk_states(const Dims& D) { return carry_states(D) + 3ll * D.k + 1; }
 
 Dims make_dims(const SgRateShape& s) {
     if (s.layers < 1 || s.rows < 1 || s.cols < 1 || s.batch < 1 || s.steps < 1 ||
@@ -801,33 +885,36 @@ Dims make_dims(const SgRateShape& s) {
     D.cols = s.cols;
     D.N = s.rows * s.cols;
     D.field = s.field;
-    D.h = s.field / 2;
     D.K = s.field * s.field;
     D.O = s.outputs;
     D.B = s.batch;
     D.T = s.steps;
-    D.k = s.checkpoint;
-    D.nseg = (s.steps + s.checkpoint - 1) / s.checkpoint;
-    D.nchunk = ((D.rows + kTileSide - 1) / kTileSide) * ((D.cols + kTileSide - 1) / kTileSide);
-    // batch elements per CTA: the largest group that still gives four CTAs
-    // per SM (152 SMs), fewer halo and weight reloads per element
-    D.bg = 1;
-    for (int g = kMaxBatchGroup; g > 1; g >>= 1)
-        if ((long long)D.nchunk * D.L * ((D.B + g - 1) / g) >= 4 * 152) { D.bg = g; break; }
     D.dt = s.dt;
-    D.S = (long long)D.L * D.B * D.N;
+    D.BN = (long long)D.B * D.N;
+    D.S = D.L * D.BN;
+    // per step: rates, drives, adjoints and the weight gradients' totals
+    D.G = (long long)(D.L - 1) * D.N * D.K + (long long)D.O * D.N;
+    const long long step_bytes = 4 * (3 * D.S + D.G);
+    D.k = (int)std::max<long long>(std::min(s.checkpoint, D.T),
+                                   std::min<long long>({kSegmentBytes / step_bytes, D.T, 65535}));
+    D.nseg = (D.T + D.k - 1) / D.k;
+    // forward: two layers' rates of a chunk of steps at a time, within the
+    // segment buffers of the backward pass and (mostly) L2; chunks alike
+    const long long fit = std::min(chunk_states(D) * D.L / 2, kChunkBytes / (8 * D.BN)) - 1;
+    const long long most = std::max<long long>(1, std::min<long long>(fit, D.T));
+    D.chunk = (int)((D.T + (D.T + most - 1) / most - 1) / ((D.T + most - 1) / most));
     return D;
 }
 
-// Workspace layout (floats): checkpoints [nseg][S], segment states v, r
-// [k+1][S], drives d and adjoints lambda [k][S], the lambda carried across
-// segments [S], outputs y [T][B][O] and their partial sums, squared errors
-// [T][B], dloss/dy [T][B][O], tau partials, transposed weights, and the
-// per-step weight and readout gradient totals of one segment.
+// Workspace layout (floats): checkpoints [nseg][S]; v at a chunk's end [S]; the
+// segment buffers (chunk_states); outputs y [T][B][O], squared errors [T][B],
+// dloss/dy [T][B][O], tau partials, transposed weights, the gradients [G], and
+// their per-step totals of one segment [k][G].
 struct Work {
-    float *ckpt, *seg_v, *seg_r, *seg_d, *seg_lam, *carry, *y, *ypart, *loss_tb, *gy, *tau_part,
-        *tau_steps, *wt, *dw_part, *dwo_part;
+    float *ckpt, *v, *chunk, *lam, *lamd, *carry[2], *seg_r, *seg_d, *seg_P, *y, *loss_tb, *gy,
+        *tau_part, *wt, *grad, *grad_part;
     long long floats;
+    bool aligned;            // on 16 bytes (every array then is)
 };
 
 Work carve(const Dims& D, void* base) {
@@ -840,131 +927,125 @@ Work carve(const Dims& D, void* base) {
         w.floats += n;
         return q;
     };
+    const long long weights = (long long)(D.L - 1) * D.K * D.N;
     w.ckpt = take((long long)D.nseg * D.S);
-    w.seg_v = take((long long)(D.k + 1) * D.S);
-    w.seg_r = take((long long)(D.k + 1) * D.S);
-    w.seg_d = take((long long)D.k * D.S);
-    w.seg_lam = take((long long)D.k * D.S);
-    w.carry = take(D.S);
+    w.v = take(D.S);
+    w.chunk = take(chunk_states(D) * D.S);
+    if (w.chunk) {
+        w.lam = w.chunk;
+        w.lamd = w.lam + D.S;
+        w.carry[0] = w.lamd + D.S;
+        w.carry[1] = w.carry[0] + D.S;
+        w.seg_r = w.chunk + carry_states(D) * D.S;
+        w.seg_d = w.seg_r + (long long)(D.k + 1) * D.S;
+        w.seg_P = w.seg_d + (long long)D.k * D.S;
+    }
     w.y = take((long long)D.T * D.B * D.O);
-    w.ypart = take((long long)D.T * D.B * D.nchunk * D.O);
     w.loss_tb = take((long long)D.T * D.B);
     w.gy = take((long long)D.T * D.B * D.O);
-    w.tau_part = take((long long)D.T * D.L * kTauBlocks);
-    w.tau_steps = take((long long)D.T * D.L);
-    w.wt = take((long long)std::max(D.L - 1, 0) * D.K * D.N);
-    const long long seg = std::min(D.k, D.T);
-    w.dw_part = take(seg * std::max(D.L - 1, 0) * D.N * D.K);
-    w.dwo_part = take(seg * D.O * D.N);
+    w.tau_part = take((long long)D.L * kTauBlocks);
+    w.wt = take(weights);
+    w.grad = take(D.G);
+    w.grad_part = take(D.k * D.G);
+    w.aligned = reinterpret_cast<uintptr_t>(base) % 16 == 0;
     return w;
 }
 
 unsigned grid_of(long long n) { return (unsigned)((n + 255) / 256); }
 
-void transpose_weights(const Dims& D, const float* w, const Work& W, cudaStream_t st) {
-    if (D.L < 2) return;
-    k_rate_transpose<<<grid_of((long long)(D.L - 1) * D.N * D.K), 256, 0, st>>>(D, w, W.wt);
-    SG_LAUNCH_CHECK();
-}
-
-dim3 tile_grid(const Dims& D) {
-    return dim3((unsigned)D.nchunk, (unsigned)D.L, (unsigned)((D.B + D.bg - 1) / D.bg));
-}
-
-#define SG_RATE_FIELD(F_RT, CALL)                                                 \
-    switch (F_RT) {                                                               \
-        case 1: { constexpr int F = 1; CALL; } break;                             \
-        case 3: { constexpr int F = 3; CALL; } break;                             \
-        case 5: { constexpr int F = 5; CALL; } break;                             \
-        case 7: { constexpr int F = 7; CALL; } break;                             \
-        default: { constexpr int F = 9; CALL; } break;                            \
-    }
-
-void step(const Dims& D, const float* x_t, const float* wo, const float* tau, const Work& W,
-          const float* v_prev, const float* r_prev, float* v_new, float* r_new, float* d_out,
-          float* ypart, cudaStream_t st) {
-    SG_RATE_FIELD(D.field, (k_rate_step<F><<<tile_grid(D), kBlock, 0, st>>>(
-                               D, x_t, W.wt, wo, tau, v_prev, r_prev, v_new, r_new, d_out, ypart)));
-    SG_LAUNCH_CHECK();
-}
-
-// One timestep of the adjoint, launched as a programmatic dependent of the
-// launch before it (the next step's adjoint, or any kernel, which then simply
-// completes first): each step's weight loads overlap the previous step's tail.
-void lambda_step(const Dims& D, const float* wo, const float* tau, const Work& W,
-                 const float* gy_t, const float* r_t, const float* lam_next, float* lam, float* dx_t,
-                 cudaStream_t st) {
+// Every launch of a pass is a programmatic dependent of the one before it.
+template <class... P, class... A>
+void launch(void (*kernel)(P...), dim3 grid, int threads, cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = tile_grid(D);
-    cfg.blockDim = dim3(kBlock);
-    cfg.dynamicSmemBytes = 0;
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const float* wt = W.wt;
-    SG_RATE_FIELD(D.field, SG_CUDA(cudaLaunchKernelEx(&cfg, k_rate_lambda<F>, D, wt, wo, tau, gy_t,
-                                                      r_t, lam_next, lam, dx_t)));
+    SG_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
 }
 
-// Shared memory of the multi-step kernel, or 0 where it does not fit (the
-// per-step kernels run instead, for the forward pass and the recompute alike).
-size_t fused_bytes(const Dims& D) {
-    static int optin = -1;
-    if (optin < 0) {
-        int dev = 0;
-        SG_CUDA(cudaGetDevice(&dev));
-        SG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+void transpose_weights(const Dims& D, const float* w, const Work& W, cudaStream_t st) {
+    if (D.L < 2) return;
+    launch(k_rate_transpose, dim3(grid_of((long long)(D.L - 1) * D.N * D.K)), 256, st, D, w, W.wt);
+}
+
+// Rows a thread takes: the full tile_py rows where that leaves a CTA for every
+// SM, one (most CTAs) in smaller problems, whose items wait on each other's
+// latency.
+unsigned tiles(const Dims& D, int py) {
+    const int ty = py * kTileWarps;
+    return (unsigned)(((D.rows + ty - 1) / ty) * ((D.cols + 31) / 32));
+}
+bool wide(const Dims& D, long long per_tile) { return tiles(D, tile_py(D.field)) * per_tile >= 152; }
+
+// Pieces of 4 floats need rows that start on 16 bytes.
+#define SG_RATE_TILE_V(D_, WIDE, VV, CALL)                                                 \
+    switch ((D_).field * 2 + ((WIDE) ? 1 : 0)) {                                           \
+        case 2: { constexpr int F = 1, PY = 1, V = VV; CALL; } break;                      \
+        case 3: { constexpr int F = 1, PY = tile_py(1), V = VV; CALL; } break;             \
+        case 6: { constexpr int F = 3, PY = 1, V = VV; CALL; } break;                      \
+        case 7: { constexpr int F = 3, PY = tile_py(3), V = VV; CALL; } break;             \
+        case 10: { constexpr int F = 5, PY = 1, V = VV; CALL; } break;                     \
+        case 11: { constexpr int F = 5, PY = tile_py(5), V = VV; CALL; } break;            \
+        case 14: { constexpr int F = 7, PY = 1, V = VV; CALL; } break;                     \
+        case 15: { constexpr int F = 7, PY = tile_py(7), V = VV; CALL; } break;            \
+        default: { constexpr int F = 9, PY = 1, V = VV; CALL; } break;                     \
     }
-    size_t floats = 0;
-    SG_RATE_FIELD(D.field, (floats = fused_smem_floats<F>(D.L)));
-    const size_t bytes = floats * sizeof(float);
-    return bytes <= (size_t)optin ? bytes : 0;
+#define SG_RATE_TILE(D_, W_, WIDE, CALL)                                                   \
+    if ((D_).cols % 4 == 0 && (W_).aligned) { SG_RATE_TILE_V(D_, WIDE, 4, CALL) }                          \
+    else { SG_RATE_TILE_V(D_, WIDE, 1, CALL) }
+
+// Batch elements a CTA takes one after the other: all of them share its weights,
+// but a CTA for each of the 5 or more that an SM can hold comes first (3 x 64x64,
+// batch 64: 1.85 ms with one element to a CTA, 2.11 with two).
+int batch_group(const Dims& D, unsigned ntiles) {
+    return (int)std::max<long long>(1, (long long)ntiles * D.B / (5 * 152));
 }
 
-void fused(const Dims& D, int mode, int c, int nt, const float* x, const float* wo,
-           const float* tau, const Work& W, const float* v0, float* ckpt, float* ypart,
-           float* seg_r, float* seg_d, cudaStream_t st) {
-    const size_t bytes = fused_bytes(D);
-    const dim3 grid((unsigned)D.nchunk, (unsigned)D.B);
-    SG_RATE_FIELD(D.field, ({
-        SG_CUDA(cudaFuncSetAttribute(k_rate_fused<F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)bytes));
-        k_rate_fused<F><<<grid, kBlock, bytes, st>>>(D, mode, c, nt, x, W.wt, wo, tau, v0, ckpt,
-                                                     ypart, seg_r, seg_d);
-    }));
-    SG_LAUNCH_CHECK();
+// Layer l through the steps c + 1 .. c + nt.
+void layer_steps(const Dims& D, int l, LayerArgs A, const float* x, const Work& W, const float* tau,
+                 cudaStream_t st) {
+    if (l == 0) {
+        launch(k_rate_input, dim3(grid_of(D.BN)), kBlock, st, D, A, x, tau);
+    } else {
+        SG_RATE_TILE(D, W, wide(D, D.B), ({
+            const unsigned nt = tiles(D, PY);
+            A.bg = batch_group(D, nt);
+            const dim3 grid(nt, (unsigned)((D.B + A.bg - 1) / A.bg));
+            launch(k_rate_layer<F, PY, V>, grid, kTileThreads, st, D, l, A, W.wt, tau);
+        }));
+    }
 }
 
 void forward(const Dims& D, const float* x, const float* w, const float* wo, const float* tau,
              const float* target, float* y_out, float* loss, void* ws, cudaStream_t st) {
     Work W = carve(D, ws);
     transpose_weights(D, w, W, st);
-    SG_CUDA(cudaMemsetAsync(W.ckpt, 0, D.S * sizeof(float), st));
-    if (fused_bytes(D)) {
-        fused(D, 0, 0, D.T, x, wo, tau, W, nullptr, W.ckpt, W.ypart, nullptr, nullptr, st);
-    } else {
-        float* v[2] = {W.seg_v, W.seg_v + D.S};
-        float* r[2] = {W.seg_r, W.seg_r + D.S};
-        SG_CUDA(cudaMemsetAsync(v[0], 0, D.S * sizeof(float), st));
-        k_rate_rates<<<grid_of(D.S), 256, 0, st>>>(D.S, v[0], r[0]);
-        SG_LAUNCH_CHECK();
-        for (int t = 1; t <= D.T; ++t) {
-            const int p = (t - 1) & 1, q = t & 1;
-            step(D, x + (long long)(t - 1) * D.B * D.N, wo, tau, W, v[p], r[p], v[q], r[q], nullptr,
-                 W.ypart + (long long)(t - 1) * D.B * D.nchunk * D.O, st);
-            if (t % D.k == 0 && t < D.T)
-                SG_CUDA(cudaMemcpyAsync(W.ckpt + (long long)(t / D.k) * D.S, v[q],
-                                        D.S * sizeof(float), cudaMemcpyDeviceToDevice, st));
+    float* buf[2] = {W.chunk, W.chunk + (D.chunk + 1) * D.BN};
+    for (int c = 0; c < D.T; c += D.chunk) {
+        const int nt = std::min(D.chunk, D.T - c);
+        for (int l = 0; l < D.L; ++l) {
+            LayerArgs A{};
+            A.src = buf[(l + 1) & 1];
+            A.r = buf[l & 1];
+            A.src_t = A.r_t = D.BN;
+            A.v0 = c > 0 ? W.v + l * D.BN : nullptr;
+            A.v1 = W.v + l * D.BN;
+            A.ckpt = W.ckpt + l * D.BN;
+            A.c = c;
+            A.nt = nt;
+            layer_steps(D, l, A, x, W, tau, st);
         }
-    }
-    k_rate_finish<<<grid_of((long long)D.T * D.B), 256, 0, st>>>(D, W.ypart, target, W.y,
-                                                                 W.loss_tb);
-    SG_LAUNCH_CHECK();
-    k_rate_loss<<<1, 256, 0, st>>>(D, W.loss_tb, loss);
-    SG_LAUNCH_CHECK();
+        const long long rows = (long long)nt * D.B;
+        launch(W.aligned && D.N % 4 == 0 ? k_rate_readout<4> : k_rate_readout<1>,
+               dim3((unsigned)((rows + kReadRows - 1) / kReadRows)), kBlock, st, D, c, nt,
+               buf[(D.L - 1) & 1], D.BN, wo, target, W.y, W.loss_tb);
+        }
+    launch(k_rate_loss, dim3(1), 256, st, D, W.loss_tb, loss);
     if (y_out)
         SG_CUDA(cudaMemcpyAsync(y_out, W.y, (size_t)D.T * D.B * D.O * sizeof(float),
                                 cudaMemcpyDeviceToDevice, st));
@@ -976,57 +1057,65 @@ void backward(const Dims& D, const float* x, const float* w, const float* wo, co
     Work W = carve(D, ws);
     transpose_weights(D, w, W, st);
     const float gscale = grad_loss * 2.0f / (float)((long long)D.T * D.B * D.O);
-    k_rate_gy<<<grid_of((long long)D.T * D.B * D.O), 256, 0, st>>>(D, gscale, W.y, target, W.gy);
-    SG_LAUNCH_CHECK();
-    if (D.L > 1)
-        SG_CUDA(cudaMemsetAsync(dw, 0, (size_t)(D.L - 1) * D.N * D.K * sizeof(float), st));
-    SG_CUDA(cudaMemsetAsync(dwo, 0, (size_t)D.O * D.N * sizeof(float), st));
-    SG_CUDA(cudaMemsetAsync(W.carry, 0, D.S * sizeof(float), st));
+    launch(k_rate_gy, dim3(grid_of((long long)D.T * D.B * D.O)), 256, st, D, gscale, W.y, target, W.gy);
+    const long long weights = (long long)(D.L - 1) * D.N * D.K;
+    // nothing follows the last step
+    if (D.L > 1) SG_CUDA(cudaMemsetAsync(W.carry[D.nseg & 1], 0, D.S * sizeof(float), st));
     for (int seg = D.nseg - 1; seg >= 0; --seg) {
         const int c = seg * D.k, nt = std::min(D.k, D.T - c);
-        if (fused_bytes(D)) {
-            fused(D, 1, c, nt, x, wo, tau, W, W.ckpt + (long long)seg * D.S, nullptr, nullptr,
-                  W.seg_r, W.seg_d, st);
-        } else {
-            SG_CUDA(cudaMemcpyAsync(W.seg_v, W.ckpt + (long long)seg * D.S, D.S * sizeof(float),
-                                    cudaMemcpyDeviceToDevice, st));
-            k_rate_rates<<<grid_of(D.S), 256, 0, st>>>(D.S, W.seg_v, W.seg_r);
-            SG_LAUNCH_CHECK();
-            for (int tt = 1; tt <= nt; ++tt)
-                step(D, x + (long long)(c + tt - 1) * D.B * D.N, wo, tau, W,
-                     W.seg_v + (tt - 1) * D.S, W.seg_r + (tt - 1) * D.S, W.seg_v + tt * D.S,
-                     W.seg_r + tt * D.S, W.seg_d + (tt - 1) * D.S, nullptr, st);
+        const bool first = seg == D.nseg - 1;
+        for (int l = 0; l < D.L; ++l) {
+            LayerArgs A{};
+            A.src = l > 0 ? W.seg_r + (l - 1) * D.BN : nullptr;
+            A.r = W.seg_r + l * D.BN;
+            A.src_t = A.r_t = D.S;
+            A.d = W.seg_d + l * D.BN;
+            A.v0 = seg > 0 ? W.ckpt + (long long)seg * D.S + l * D.BN : nullptr;
+            A.c = c;
+            A.nt = nt;
+            layer_steps(D, l, A, x, W, tau, st);
         }
-        for (int tt = nt; tt >= 1; --tt) {
-            const int t = c + tt;
-            const float* lam_next = tt == nt ? W.carry : W.seg_lam + (long long)tt * D.S;
-            lambda_step(D, wo, tau, W, W.gy + (long long)(t - 1) * D.B * D.O,
-                        W.seg_r + (long long)tt * D.S, lam_next,
-                        W.seg_lam + (long long)(tt - 1) * D.S,
-                        dx ? dx + (long long)(t - 1) * D.B * D.N : nullptr, st);
-        }
-        SG_CUDA(cudaMemcpyAsync(W.carry, W.seg_lam, D.S * sizeof(float),
-                                cudaMemcpyDeviceToDevice, st));
+        for (int l = D.L - 1; l >= 0; --l) {
+            AdjointArgs A{};
+            A.r = W.seg_r + l * D.BN;
+            A.d = W.seg_d + l * D.BN;
+            A.next = W.seg_P + (l + 1) * D.BN;
+            A.next_carry = W.carry[(seg + 1) & 1] + (l + 1) * D.BN;
+            // layer 0's P is dx, and nothing else reads it
+            A.P = l > 0 ? W.seg_P + l * D.BN : (dx ? dx + (long long)c * D.BN : nullptr);
+            A.P_t = l > 0 ? D.S : D.BN;
+            A.carry = l > 0 ? W.carry[seg & 1] + l * D.BN : nullptr;
+            A.first = first;
+            A.lam = W.lam + l * D.BN;
+            A.lamd = W.lamd + l * D.BN;
+            A.nt = nt;
+            if (l == D.L - 1) {
+                const dim3 grid((unsigned)((D.N + kBlock - 1) / kBlock), (unsigned)D.B);
+                launch(k_rate_adjoint_top, grid, kBlock, st, D, A, wo, W.gy + (long long)c * D.B * D.O, tau);
+            } else {
+                SG_RATE_TILE(D, W, wide(D, D.B), ({
+                    const unsigned n = tiles(D, PY);
+                    A.bg = batch_group(D, n);
+                    const dim3 grid(n, (unsigned)((D.B + A.bg - 1) / A.bg));
+                    launch(k_rate_adjoint<F, PY, V>, grid, kTileThreads, st, D, l, A, W.wt, tau);
+                }));
+            }
+                }
         if (D.L > 1) {
-            const dim3 grid((unsigned)D.nchunk, (unsigned)(D.L - 1), (unsigned)nt);
-            SG_RATE_FIELD(D.field, (k_rate_dw_staged<F><<<grid, kBlock, 0, st>>>(
-                                       D, W.seg_lam, W.seg_r, W.dw_part)));
-            SG_LAUNCH_CHECK();
-            k_rate_dw_acc<<<grid_of((long long)(D.L - 1) * D.N * D.K), 256, 0, st>>>(
-                D, nt, tau, W.dw_part, dw);
-            SG_LAUNCH_CHECK();
+            SG_RATE_TILE(D, W, wide(D, (long long)(D.L - 1) * nt), ({
+                const dim3 grid(tiles(D, PY), (unsigned)(D.L - 1), (unsigned)nt);
+                launch(k_rate_dw<F, PY, V>, grid, kTileThreads, st, D, W.seg_P, W.seg_r, W.grad_part);
+            }));
+                }
+        const int dwo_v = W.aligned && D.N % 4 == 0 ? 4 : 1, per = kReadoutThreads * dwo_v;
+        launch(dwo_v == 4 ? k_rate_dwo<4> : k_rate_dwo<1>,
+               dim3((unsigned)((D.N + per - 1) / per), (unsigned)nt), kReadoutThreads, st, D,
+               W.gy + (long long)c * D.B * D.O, W.seg_r, W.grad_part + weights);
+        launch(k_rate_acc, dim3(grid_of(D.G)), 256, st, D, nt, first, W.grad_part, W.grad);
         }
-        k_rate_dwo<<<dim3((unsigned)((D.N + 31) / 32), (unsigned)nt), kBlock, 0, st>>>(
-            D, c, W.gy, W.seg_r, W.dwo_part);
-        SG_LAUNCH_CHECK();
-        k_rate_dwo_acc<<<grid_of((long long)D.O * D.N), 256, 0, st>>>(D, nt, W.dwo_part, dwo);
-        SG_LAUNCH_CHECK();
-        k_rate_dtau_partial<<<dim3(kTauBlocks, D.L, nt), 256, 0, st>>>(D, c, W.seg_lam, W.seg_d,
-                                                                       W.tau_part);
-        SG_LAUNCH_CHECK();
-    }
-    k_rate_dtau_final<<<1, 256, 0, st>>>(D, tau, W.tau_part, W.tau_steps, dtau);
-    SG_LAUNCH_CHECK();
+    launch(k_rate_out, dim3(grid_of(D.G)), 256, st, D, W.grad, dw, dwo);
+    launch(k_rate_dtau_partial, dim3(kTauBlocks, D.L), 256, st, D, W.lamd, W.tau_part);
+    launch(k_rate_dtau_final, dim3((unsigned)((D.L + 255) / 256)), 256, st, D, tau, W.tau_part, dtau);
 }
 
 }  // namespace

@@ -164,3 +164,48 @@ def test_gol_whole_runs_on_ragged_boards(sg, rows, cols, diagonal, low, high):
     for steps in (1, 12, 37):
         assert_equal(run_both(sg, net, {("b", "output"): words}, steps,
                               [("b", "output"), ("b", "input")]))
+
+
+# tiles of 32 columns by 4 warps of 1, 2 or 8 rows, rows copied whole or by 4
+# floats, segments longer than the checkpoint, groups of the batch; the field
+# sizes that have their own tiles
+@pytest.mark.parametrize("cfg", [
+    dict(layers=2, rows=33, cols=36, field=1, outputs=1, batch=9, steps=5),
+    dict(layers=3, rows=65, cols=64, field=3, outputs=16, batch=40, steps=6),
+    dict(layers=2, rows=17, cols=31, field=5, outputs=9, batch=70, steps=34),
+    dict(layers=2, rows=9, cols=33, field=5, outputs=8, batch=33, steps=11),
+    dict(layers=3, rows=24, cols=68, field=7, outputs=3, batch=17, steps=7),
+    dict(layers=2, rows=7, cols=40, field=9, outputs=5, batch=6, steps=12)])
+def test_rate_tiles(cfg):
+    """Loss and gradients against the FP64 restatement, and bit for bit the
+    same whatever the checkpoint stride and the workspace's alignment."""
+    import ctypes
+    import torch
+    from oracle import rate_adjoint as ra
+    from synaptogenesis_gb300 import syngen
+    from tests.test_gpu_rate import close, gpu_grads, make
+    p = make(13, *(cfg[k] for k in ("layers", "rows", "cols", "field", "outputs", "batch", "steps")))
+    nets = [syngen.RateNetwork(checkpoint=k, **cfg) for k in (1, 3, cfg["steps"])]
+    results = [gpu_grads(torch, syngen, net, p) for net in nets]
+    for other in results[1:]:
+        for a, b in zip(other, results[0]):
+            assert np.array_equal(np.asarray(a), np.asarray(b))
+    want = ra.adjoint(dict(cfg, checkpoint=1, dt=1.0), p["x"], p["weights"], p["readout"], p["tau"],
+                      p["target"])
+    assert abs(results[0][0] - want[0]) <= 1e-5 * abs(want[0])
+    for got, w in zip(results[0][1:], want[1:]):
+        ok, norm = close(got, w)
+        assert ok, norm
+    # a workspace that starts 4 bytes off a 16-byte boundary
+    net, t = nets[1], {k: torch.tensor(v, device="cuda") for k, v in p.items()}
+    ws = torch.empty(net.workspace_bytes // 4 + 4, device="cuda")[1:]
+    loss = torch.empty((), device="cuda")
+    grads = [torch.empty_like(t[k]) for k in ("weights", "readout", "tau", "x")]
+    args = [t[k].data_ptr() for k in ("x", "weights", "readout", "tau", "target")]
+    stream = torch.cuda.current_stream().cuda_stream
+    assert syngen._syn.sg_rate_forward(ctypes.byref(net.shape), *args, None, loss.data_ptr(),
+                                       ws.data_ptr(), stream) == 0
+    assert syngen._syn.sg_rate_backward(ctypes.byref(net.shape), *args, 1.0, ws.data_ptr(),
+                                        *(g.data_ptr() for g in grads), stream) == 0
+    for a, b in zip([loss] + grads, results[0]):
+        np.testing.assert_allclose(a.cpu().numpy(), b, rtol=1e-4, atol=1e-4 * np.abs(b).max())
