@@ -137,12 +137,49 @@ SG_FF float div_int(float a) {
     return fma(r, y, q);
 }
 
+// (float)((double)p * c) for |p| below 2^-125 and |c| at most 1, whose result may
+// be subnormal: in units of 2^-149, p is an integer m of at most 24 bits and the
+// result the integer nearest m c.  The float-float product errs by less than
+// 2^-44 |m c| < 2^-20, so a fraction further than 2^-18 from a half decides (for
+// halves see product).  A decaying trace passes through this range, and stays at
+// its end, for as long as its neuron is silent.
+SG_FF bool tiny_product(float p, float c1, float c2, float& out, bool ties) {
+    // 2^149 in two exact steps
+    const float m = mul(mul(p, 1.2676506002282294e30f), 562949953421312.0f);
+    float h, l;
+    two_prod(m, c1, h, l);
+    l = add(l, mul(m, c2));
+#ifdef __CUDA_ARCH__
+    float n = rintf(h);
+#else
+    float n = std::rint(h);
+#endif
+    const float frac = add(sub(h, n), l);
+    const float a = absf(frac);
+    if (!(a < 0.5f - 3.814697265625e-6f || a > 0.5f + 3.814697265625e-6f)) {
+        if (!(ties && a < 1.0f)) return false;
+        if ((int)n & 1) n = add(n, frac > 0.0f ? 1.0f : -1.0f);
+    } else if (a > 0.5f) {
+        n = add(n, frac > 0.0f ? 1.0f : -1.0f);
+    }
+    if (n == 0.0f) n = mul(m, 0.0f);                       // the product's sign
+    out = mul(mul(n, 1.7763568394002505e-15f), 7.888609052210118e-31f);   // 2^-49, 2^-100
+    return true;
+}
+
 // (float)((double)p * c) for a double constant c ~ c1 + c2 (two floats, c2
-// the rounded remainder): Dekker's product plus the remainder's, error below
-// 2^-45 |p c| in all, bound 2^-40 |f|.  Operands below 2^-50 are scaled by
-// 2^64 first (exact, as are both roundings of a result in the normal float
-// range); results below 2^-126 return false.
-SG_FF bool product(float p, float c1, float c2, float& out) {
+// the rounded remainder), |c| at most 1: Dekker's product plus the remainder's,
+// error below 2^-45 |p c| in all, bound 2^-40 |f|.  Operands below 2^-50 are
+// scaled by 2^64 first (exact, as are both roundings of a result in the normal
+// float range); those whose result may be subnormal go to tiny_product.
+//
+// `ties`: c is a decimal of at most three digits d = n / 1000 and errs from it by
+// less than 2^-54 c (0.9, 0.95, 0.933 do).  p d then lies on a midpoint, which it
+// does for one p in 10, 20 or 1000, or at least 1/1000 of the float spacing from
+// it, so what the test rejects is a midpoint; p c is within half a double's spacing
+// of it, rounds to it in double, and from there to the even float.
+SG_FF bool product(float p, float c1, float c2, float& out, bool ties = false) {
+    if (absf(p) < 2.350988701644575e-38f) return tiny_product(p, c1, c2, out, ties);   // 2^-125
     const bool small = absf(p) < 8.881784197001252323e-16f;             // 2^-50
     const float ps = small ? mul(p, 18446744073709551616.0f) : p;       // 2^64
     float h, l;
@@ -150,7 +187,12 @@ SG_FF bool product(float p, float c1, float c2, float& out) {
     l = add(l, mul(ps, c2));
     float f, g;
     two_sum(h, l, f, g);
-    if (!rounds_to(f, g, mul(absf(f), kBound))) return false;
+    if (!rounds_to(f, g, mul(absf(f), kBound))) {
+        const uint32_t u = bits(f);
+        if (!ties || (u >> 23 & 0xFFu) - 26u > 227u) return false;
+        // the neighbour on g's side, if f is odd
+        if (u & 1u) f = from_bits((g > 0.0f) == (f > 0.0f) ? u + 1u : u - 1u);
+    }
     if (small) {
         if (absf(f) < 2.168404344971008868e-19f) return false;          // 2^-62: result below 2^-126
         f = mul(f, 5.421010862427522170e-20f);                          // 2^-64, exact for normal results
@@ -272,7 +314,8 @@ SG_FF bool short_term_w(float sw, bool spike, float& out) {
 // most u^2 (11 |P| + 10 S), P = 0.04 v v and S the largest partial sum, and
 // the reference's double roundings by less than 2^-53 (2 |P| + 5 S); the
 // bound used is 2^-43 (|P| + S), a factor of 2.9 above their sum.
-SG_FF bool iz_delta_v(float v, float recovery, float current, float& out) {
+// iz_delta_v_sum gives the value as f + g, f = RN(f + g), and the bound.
+SG_FF void iz_delta_v_sum(float v, float recovery, float current, float& f, float& g, float& B) {
     constexpr double C = 0.04;
     constexpr float C1 = (float)C;
     constexpr float C2 = (float)(C - (double)C1);
@@ -296,9 +339,14 @@ SG_FF bool iz_delta_v(float v, float recovery, float current, float& out) {
     two_sum(s, current, s, e);
     l2 = add(e, l2);
     smax = fmaxf(smax, absf(s));
-    float f, g;
     two_sum(s, l2, f, g);
-    if (!rounds_to(f, g, mul(add(absf(h2), smax), kBound5))) return false;
+    B = mul(add(absf(h2), smax), kBound5);
+}
+
+SG_FF bool iz_delta_v(float v, float recovery, float current, float& out) {
+    float f, g, B;
+    iz_delta_v_sum(v, recovery, current, f, g, B);
+    if (!rounds_to(f, g, B)) return false;
     out = f;
     return true;
 }
@@ -319,13 +367,16 @@ SG_FF void iz_denominator(float sum_c, float& d1, float& d2) {
     d2 = add(e, b2);
 }
 
-SG_FF bool iz_voltage(float v, float drive, float d1, float d2, float rd, float& out) {
+// `err` bounds how far the float drive may be from drive + tail (both zero where
+// the drive is known): the result then holds for every drive within it.
+SG_FF bool iz_voltage(float v, float drive, float d1, float d2, float rd, float& out,
+                      float tail = 0.0f, float err = 0.0f) {
     constexpr double T = 0.1;
     constexpr float T1 = (float)T;
     constexpr float T2 = (float)(T - (double)T1);
     float a1, a2;
     two_prod(drive, T1, a1, a2);
-    a2 = add(a2, mul(drive, T2));            // 0.1 drive ~ a1 + a2
+    a2 = add(a2, add(mul(drive, T2), mul(tail, T1)));    // 0.1 (drive + tail) ~ a1 + a2
     float n1, n2;
     two_sum(v, a1, n1, n2);
     n2 = add(n2, a2);                        // numerator ~ n1 + n2
@@ -338,9 +389,75 @@ SG_FF bool iz_voltage(float v, float drive, float d1, float d2, float rd, float&
     float f, g;
     two_sum(q1, q2, f, g);
     const float M = add(mul(add(absf(v), absf(a1)), rd), absf(f));
-    if (!rounds_to(f, g, mul(M, kBound4))) return false;
+    // (0.1 err / den, an eighth above it)
+    if (!rounds_to(f, g, add(mul(M, kBound4), mul(mul(err, 0.1125f), absf(rd))))) return false;
     out = f;
     return true;
+}
+
+// (float)((double)v + (double)d * 0.1), the spnet voltage step
+// (spnet_attributes.cpp:96-166): the product errs by at most 2^-47 of itself,
+// the sums by 2^-47 (|s| + |a1|) in all; the bound is 2^-43 (|s| + |a1|).  `err`
+// bounds how far the float d may be from d + tail, as in iz_voltage.
+SG_FF bool spnet_voltage(float v, float d, float& out, float tail = 0.0f, float err = 0.0f) {
+    constexpr double T = 0.1;
+    constexpr float T1 = (float)T;
+    constexpr float T2 = (float)(T - (double)T1);
+    float a1, a2;
+    two_prod(d, T1, a1, a2);
+    a2 = add(a2, add(mul(d, T2), mul(tail, T1)));        // 0.1 (d + tail) ~ a1 + a2
+    float s, e;
+    two_sum(v, a1, s, e);
+    float f, g;
+    two_sum(s, add(e, a2), f, g);
+    if (!rounds_to(f, g, add(mul(add(absf(s), absf(a1)), kBound5), mul(err, 0.1125f)))) return false;
+    out = f;
+    return true;
+}
+
+// (float)(0.9 * (double)x + p - q), the spnet weight derivative
+// (spnet_attributes.cpp:220-286), p and q floats: as above, with one more sum.
+SG_FF bool spnet_dw(float x, float p, float q, float& out) {
+    constexpr double N = 0.9;
+    constexpr float N1 = (float)N;
+    constexpr float N2 = (float)(N - (double)N1);
+    float h, l;
+    two_prod(x, N1, h, l);
+    l = add(l, mul(x, N2));                  // 0.9 x ~ h + l
+    float s, e, s2, e2;
+    two_sum(h, p, s, e);
+    l = add(e, l);
+    two_sum(s, -q, s2, e2);
+    l = add(e2, l);
+    float f, g;
+    two_sum(s2, l, f, g);
+    if (!rounds_to(f, g, mul(add(absf(h), add(absf(s), absf(s2))), kBound5))) return false;
+    out = f;
+    return true;
+}
+
+// The voltage where the derivative's rounding test failed, which is where it is
+// small (a neuron near rest: the terms cancel, and the float nearest the sum is not
+// known).  Its float is within B of f + g, give or take its own rounding, and that
+// decides the voltage unless the step ends next to a rounding boundary: those are
+// 2^-24 |v| apart, the uncertainty 2^-43 of the cancelled terms.  Only a step past
+// the threshold needs the derivative itself.
+constexpr float kHalfUlp = 5.9604701e-8f;                 // a little above 2^-24
+
+SG_FF bool spnet_voltage_near(float v, float f, float g, float B, float& out) {
+    return spnet_voltage(v, f, out, g, add(B, mul(absf(f), kHalfUlp))) && !(out > 30.0f);
+}
+
+// The same for iz_voltage: the Izhikevich drive is (delta_v + x) + y in float, x =
+// gabaa -70, y = gabab -90, three float roundings.  drive + tail is the sum without
+// them (tail: the derivative's g on entry), err what they and B can make of it.
+SG_FF void iz_drive_near(float f, float x, float y, float B, float& drive, float& tail, float& err) {
+    float s, e, e2;
+    two_sum(f, x, s, e);
+    two_sum(s, y, drive, e2);
+    tail = add(tail, add(e, e2));
+    // twice the roundings: the tail's own are far below
+    err = add(B, mul(add(absf(f), add(absf(s), absf(drive))), 2.0f * kHalfUlp));
 }
 
 // Recovery time constant of the substep that crosses the threshold

@@ -87,11 +87,12 @@ static __device__ __noinline__ float iz_tau_double(float voltage, float delta_v)
 
 // The same substeps with each double expression evaluated in float-float
 // arithmetic (ff_exact.cuh) and its float result taken where the rounding
-// test proves it equal to the double evaluation; elsewhere (about one
-// evaluation in a hundred: results within the error bound of a rounding
-// boundary, such as the first substep after a reset, where v = c is exact
-// and the terms cancel) the expression is evaluated in double.  The results
-// are iz_integrate's, bit for bit, at a fraction of its FP64 work.
+// test proves it equal to the double evaluation.  The derivative's test fails
+// where its terms cancel (near rest, and on the first substep after a reset); the
+// voltage is then decided from the unrounded derivative (iz_drive_near).  What is
+// left is evaluated in double.  A substep that changes neither voltage nor
+// recovery would be repeated by the rest, which are left out.  The results are
+// iz_integrate's, bit for bit, at a fraction of its FP64 work.
 __device__ __forceinline__ void iz_integrate_ff(float& voltage, float& recovery, float ampa_c,
                                                 float nmda_c, float gabaa_c, float gabab_c,
                                                 float mf, float base_current, float a, float b) {
@@ -109,18 +110,25 @@ __device__ __forceinline__ void iz_integrate_ff(float& voltage, float& recovery,
         current -= gabab_c * (voltage + 90);
         current *= 1 + mf;
         current += base_current;
-        float delta_v;
-        if (!ff::iz_delta_v(voltage, recovery, current, delta_v))
-            delta_v = iz_delta_v_double(voltage, recovery, current);
-        const float drive = delta_v + (gabaa_c * -70) + (gabab_c * -90);
-        float nv;
-        if (!ff::iz_voltage(voltage, drive, d1, d2, rd, nv))
-            nv = iz_voltage_double(voltage, drive, sum_c);
+        float delta_v, tail, bound, nv;
+        ff::iz_delta_v_sum(voltage, recovery, current, delta_v, tail, bound);
+        const float x = gabaa_c * -70, y = gabab_c * -90;
+        const bool known = ff::rounds_to(delta_v, tail, bound);
+        float drive = delta_v + x + y, err = 0.0f;
+        if (known) tail = 0.0f;
+        else ff::iz_drive_near(delta_v, x, y, bound, drive, tail, err);
+        if (!ff::iz_voltage(voltage, drive, d1, d2, rd, nv, tail, err) || !(known || nv <= 30.0f)) {
+            if (!known) delta_v = iz_delta_v_double(voltage, recovery, current);
+            nv = iz_voltage_double(voltage, delta_v + x + y, sum_c);
+        }
+        const float v0 = voltage, r0 = recovery;
         voltage = (nv != nv) ? 30.0f : nv;
         float adjusted_tau = (float)0.1;
         if (voltage > 30.0f && !ff::iz_adjusted_tau(voltage, delta_v, adjusted_tau))
             adjusted_tau = iz_tau_double(voltage, delta_v);
         recovery += a * adjusted_tau * ((b * voltage) - recovery);
+        // at rest: the remaining substeps would repeat this one
+        if (voltage == v0 && recovery == r0) break;
     }
 }
 #endif

@@ -123,7 +123,10 @@ __device__ __forceinline__ void iz_learn_apply(size_t wi, const LearnVals& v, in
         constexpr float C1 = (float)0.933;
         constexpr float C2 = (float)(0.933 - (double)C1);
         if (src_spike) src_trace = (float)0.004;
-        else if (!ff::product(v.presyn, C1, C2, src_trace)) src_trace = presyn_decay_exact(v.presyn);
+        else if (v.presyn == 0.0f || (__float_as_uint(v.presyn) & 0x7FFFFFFFu) == 7u)
+            src_trace = v.presyn;        // no spike yet, or where a silent trace ends: 0.933 leaves
+                                         // 7 units of 2^-149 as they are
+        else if (!ff::product(v.presyn, C1, C2, src_trace, true)) src_trace = presyn_decay_exact(v.presyn);
         presyn[wi] = src_trace;
         dest_trace = dest_exc_trace;
     } else {
@@ -528,6 +531,14 @@ __global__ void k_iz_delay_summary(int n_src, const int* __restrict__ counts,
     summary[f] = ne > kSummary ? 7ull : (sm | (unsigned long long)ne);
 }
 
+// trace * 0.95 in double, rounded to float.
+static __device__ __forceinline__ float decay_95(float trace) {
+    constexpr float D1 = (float)0.95, D2 = (float)(0.95 - (double)D1);
+    float out = trace;
+    if (trace != 0.0f && !ff::product(trace, D1, D2, out, true)) out = mul_fd_rn(trace, 0.95);
+    return out;
+}
+
 // Neuron update (izhikevich_attributes.cpp:102-213).  One launch updates the
 // Izhikevich layers of a step together (their neurons concatenated); each
 // layer's arrays are its own.  The substeps run in float-float arithmetic
@@ -549,6 +560,12 @@ struct IzUpdateGroup {
     IzLayerArgs L[kIzGroup];
 };
 
+// A neuron is a chain of dependent substeps, so few neurons are spread a warp to a
+// CTA (a warp to a scheduler) before warps share one.
+static int update_threads(int neurons) {
+    return neurons <= 152 * 4 * 32 ? 32 : 128;
+}
+
 __global__ void __launch_bounds__(256) k_iz_update(IzUpdateGroup G) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= G.start[G.n]) return;
@@ -565,7 +582,7 @@ __global__ void __launch_bounds__(256) k_iz_update(IzUpdateGroup G) {
     A.gabaa[nid] = 0.0f;
     A.gabab[nid] = 0.0f;
     A.mult[nid] = 0.0f;
-    A.dopamine[nid] = mul_fd_rn(A.dopamine[nid], 0.95);            // dopamine *= 0.95
+    A.dopamine[nid] = decay_95(A.dopamine[nid]);                     // dopamine *= 0.95
     const unsigned int spike = voltage >= 30.0f;                     // 30.0 is a float value
     // SHIFT_BIT_OUTPUTS (state/attributes.h:321-333)
     uint32_t* spikes = A.spikes;
@@ -578,7 +595,7 @@ __global__ void __launch_bounds__(256) k_iz_update(IzUpdateGroup G) {
     spikes[nid] = (curr >> 1) | (spike << 31);
     const bool prev_bit = curr >> 31;
     // post_trace = prev_bit ? 0.004 : post_trace * 0.95, stored as float
-    A.post_traces[nid] = prev_bit ? (float)0.004 : mul_fd_rn(A.post_traces[nid], 0.95);
+    A.post_traces[nid] = prev_bit ? (float)0.004 : decay_95(A.post_traces[nid]);
     int t = A.tss[nid] + 1;
     A.tss[nid] = prev_bit ? 0 : (t < 32 ? t : 32);
     A.voltages[nid] = spike ? __ldg(A.cs + nid) : voltage;
@@ -1035,7 +1052,8 @@ class IzhikevichModel : public Model {
             }
             G.start[G.n] = total;
             if (total == 0) continue;
-            k_iz_update<<<blocks_for(total, 256), 256, 0, ctx.stream>>>(G);
+            const int threads = update_threads(total);
+            k_iz_update<<<blocks_for(total, threads), threads, 0, ctx.stream>>>(G);
             SG_LAUNCH_CHECK();
             ctx.count();
         }
@@ -1174,33 +1192,72 @@ __global__ void __launch_bounds__(128) k_spnet_activate(DGeom g, const uint32_t*
     inputs[to] = aggregate(inputs[to], sum, opcode);
 }
 
-// spnet_attributes.cpp:96-166, the reference's expressions as written: the
-// double constants promote, and the float stores round.
-__global__ void __launch_bounds__(256) k_spnet_update(int size, int history, const float* __restrict__ in,
-                                                      uint32_t* spikes, float* vs, float* rs, float* post,
-                                                      int* tss, const float* __restrict__ as,
-                                                      const float* __restrict__ bs,
-                                                      const float* __restrict__ cs,
-                                                      const float* __restrict__ ds) {
-    const int nid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (nid >= size) return;
-    float voltage = vs[nid];
-    float recovery = rs[nid];
-    const float current = in[nid];
-    const float a = as[nid], b = bs[nid];
-    for (int i = 0; (i < 10) && (voltage < 30.0); ++i) {
-        const float delta_v = (0.04 * voltage * voltage) + (5 * voltage) + 140 - recovery + current;
-        voltage += delta_v * 0.1;
-        voltage = (voltage != voltage) ? 30.0f : voltage;
-        const float adjusted_tau = (voltage > 30.0) ? delta_v / (30.0 - voltage + delta_v) * 0.1 : 0.1;
+// The substep's double expressions in double, where a rounding test fails.
+static __device__ __noinline__ float spnet_delta_double(float voltage, float recovery, float current) {
+    return (0.04 * voltage * voltage) + (5 * voltage) + 140 - recovery + current;
+}
+static __device__ __noinline__ float spnet_voltage_double(float voltage, float delta_v) {
+    return voltage + delta_v * 0.1;
+}
+
+// Neuron update (spnet_attributes.cpp:96-166), the layers of a step in one
+// launch: the double expressions in float-float with rounding tests.  FP64 bounds
+// it otherwise: 65,536 and 16,384 neurons took 21.5 us a launch in double, in two
+// launches; 10.2 us together like this.
+struct SpnetLayerArgs {
+    int size, history;
+    const float* in;
+    uint32_t* spikes;
+    float *vs, *rs, *post;
+    int* tss;
+    const float *as, *bs, *cs, *ds;
+};
+struct SpnetUpdateGroup {
+    int n;
+    int start[kIzGroup + 1];
+    SpnetLayerArgs L[kIzGroup];
+};
+
+__global__ void __launch_bounds__(256) k_spnet_update(SpnetUpdateGroup G) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= G.start[G.n]) return;
+    int l = 0;
+    while (l + 1 < G.n && g >= G.start[l + 1]) ++l;
+    const SpnetLayerArgs& A = G.L[l];
+    const int nid = g - G.start[l];
+    float voltage = A.vs[nid];
+    float recovery = A.rs[nid];
+    const float current = A.in[nid];
+    const float a = A.as[nid], b = A.bs[nid];
+    for (int i = 0; (i < 10) && (voltage < 30.0f); ++i) {
+        float delta_v, tail, bound, nv;
+        ff::iz_delta_v_sum(voltage, recovery, current, delta_v, tail, bound);
+        const bool known = ff::rounds_to(delta_v, tail, bound);
+        const float err = known ? 0.0f : ff::add(bound, ff::mul(fabsf(delta_v), ff::kHalfUlp));
+        if (!ff::spnet_voltage(voltage, delta_v, nv, known ? 0.0f : tail, err) ||
+            !(known || nv <= 30.0f)) {
+            if (!known) delta_v = spnet_delta_double(voltage, recovery, current);
+            nv = spnet_voltage_double(voltage, delta_v);
+        }
+        const float v0 = voltage, r0 = recovery;
+        voltage = (nv != nv) ? 30.0f : nv;
+        float adjusted_tau = (float)0.1;
+        if (voltage > 30.0f && !ff::iz_adjusted_tau(voltage, delta_v, adjusted_tau))
+            adjusted_tau = iz_tau_double(voltage, delta_v);
         recovery += a * adjusted_tau * ((b * voltage) - recovery);
+        if (voltage == v0 && recovery == r0) break;          // at rest
     }
-    const uint32_t spike = voltage >= 30.0;
-    const uint32_t prev_bit = shift_bits(spikes, size, history, nid, spike);
-    post[nid] = prev_bit ? (float)(post[nid] + 0.1) : (float)(post[nid] * 0.95);
-    tss[nid] = prev_bit ? 0 : min(32, tss[nid] + 1);
-    vs[nid] = spike ? cs[nid] : voltage;
-    rs[nid] = recovery + (spike * ds[nid]);
+    const uint32_t spike = voltage >= 30.0f;
+    const uint32_t prev_bit = shift_bits(A.spikes, A.size, A.history, nid, spike);
+    const float post = A.post[nid];
+    float np;
+    constexpr float T1 = (float)0.1, T2 = (float)(0.1 - (double)T1);
+    if (!prev_bit) np = decay_95(post);
+    else if (!ff::add_const(post, T1, T2, np)) np = (float)(post + 0.1);
+    A.post[nid] = np;
+    A.tss[nid] = prev_bit ? 0 : min(32, A.tss[nid] + 1);
+    A.vs[nid] = spike ? A.cs[nid] : voltage;
+    A.rs[nid] = recovery + (spike * A.ds[nid]);
 }
 
 // spnet_attributes.cpp:220-286 ("add": presynaptic trace against the
@@ -1242,7 +1299,7 @@ __global__ void __launch_bounds__(128) k_spnet_learn(DGeom g, const uint32_t* __
     });
 }
 
-// The STDP kernel's rare double expressions, out of line (see f2d_hw).
+// The STDP kernel's rare double expressions, out of line (see f2d_exact).
 static __device__ __noinline__ float spnet_trace_step(float p) { return (float)(p + 0.1); }
 static __device__ __noinline__ float spnet_dw_full(float dw0, float f1, float f2) {
     return d2f_rn(__dadd_rn(__dadd_rn(mul_df_rn(dw0, 0.9), f2d_exact(f1)), -f2d_exact(f2)));
@@ -1250,11 +1307,14 @@ static __device__ __noinline__ float spnet_dw_full(float dw0, float f1, float f2
 
 // Sparse connections: one thread per compacted synapse (blockIdx.y is the
 // synapse's rank within its destination, x the destination), since each
-// synapse's update is independent.  The products with 0.9 / 0.95 and the
-// sums with 0.1 / 0.01 are float-float evaluations with a rounding test
-// (ff_exact.cuh), falling back to the integer helpers and double sums where
-// the test rejects; the full weight-derivative sum with spike terms stays
-// double.  Bit-identical to k_spnet_learn.
+// synapse's update is independent.  The double expressions are float-float
+// evaluations with a rounding test (ff_exact.cuh), falling back to integer helpers
+// and double sums where it rejects, which a warp pays for if one of its 32 synapses
+// does: products with 0.9 and 0.95 that land on a midpoint (one in 10 or 20), zero
+// and silent traces and derivatives, and sums with spike terms are therefore decided
+// on the fast path.  Issue bounds it (about 200 instructions a synapse): 7.3 M
+// synapses of a network that has run a while took 102 us with those on the slow
+// path, 78 us now.  Bit-identical to k_spnet_learn.
 template <int SR, bool SUB>
 __global__ void __launch_bounds__(256) k_spnet_learn_sparse(DGeom g, const uint32_t* __restrict__ dest_out,
                                                             const float* __restrict__ post,
@@ -1263,16 +1323,16 @@ __global__ void __launch_bounds__(256) k_spnet_learn_sparse(DGeom g, const uint3
                                                             float max_weight, float* __restrict__ w,
                                                             float* __restrict__ presyn,
                                                             float* __restrict__ dws, IzLut lut) {
-    const int d = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned d = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y;
-    if (d >= g.to_size) return;
+    if (d >= (unsigned)g.to_size) return;
     // every load that depends on nothing but the synapse's position first
     // (the [kmax][to] arrays are allocated for the padding too), then the
     // checks, then the source's time since spike
-    const int wi = i * g.to_size + d;
+    const unsigned wi = (unsigned)i * g.to_size + d;
     const int n = g.nz[d];
     float weight = w[wi];
-    const int from = g.sfrom[wi];
+    const unsigned from = (unsigned)g.sfrom[wi];
     const float p = SUB ? 0.0f : presyn[wi];
     const float dw0 = dws[wi];
     const uint32_t dword = dest_out[d];
@@ -1287,12 +1347,17 @@ __global__ void __launch_bounds__(256) k_spnet_learn_sparse(DGeom g, const uint3
         float np;
         constexpr float T1 = (float)0.1, T2 = (float)(0.1 - (double)T1);
         constexpr float D1 = (float)0.95, D2 = (float)(0.95 - (double)D1);
+        // 0.95 x 10 units of 2^-149 rounds back to them: where a silent trace ends
         if (src_spike) {
             if (!ff::add_const(p, T1, T2, np)) np = spnet_trace_step(p);
-        } else if (!ff::product(p, D1, D2, np)) {
-            np = mul_fd_rn(p, 0.95);
+            presyn[wi] = np;
+        } else if (p == 0.0f || (__float_as_uint(p) & 0x7FFFFFFFu) == 10u) {
+            np = p;
+        } else {
+            if (!ff::product(p, D1, D2, np, true)) np = mul_fd_rn(p, 0.95);
+            presyn[wi] = np;
         }
-        src_trace = presyn[wi] = np;
+        src_trace = np;
         dest_trace = dest_exc;
     } else {
         src_trace = (dest_spike > 0.0f && stss > 0 && stss < 32) ? lut.src[stss] : 0.0f;
@@ -1300,19 +1365,26 @@ __global__ void __launch_bounds__(256) k_spnet_learn_sparse(DGeom g, const uint3
     }
     const float f1 = dest_spike * src_trace;
     const float f2 = (src_spike ? 1.0f : 0.0f) * dest_trace;
-    // 0.9 dw + f1 - f2 in double: with f1, f2 zero and dw nonzero it is the
-    // rounded product alone
-    float dw;
+    // 0.9 dw + f1 - f2 in double: with dw zero the float difference (rounding the
+    // double one again changes nothing: 53 >= 2 * 24 + 2 bits), with f1, f2 zero
+    // the rounded product alone, which leaves 4 units of 2^-149 (a derivative's end)
+    // as they are
+    float dw = dw0;
     constexpr float N1 = (float)0.9, N2 = (float)(0.9 - (double)N1);
     constexpr float S1 = (float)0.01, S2 = (float)(0.01 - (double)S1);
-    if (f1 == 0.0f && f2 == 0.0f && dw0 != 0.0f) {
-        if (!ff::product(dw0, N1, N2, dw)) dw = mul_fd_rn(dw0, 0.9);
-    } else {
+    if (dw0 == 0.0f) {
+        dw = dw0 + f1 - f2;
+    } else if (f1 == 0.0f && f2 == 0.0f) {
+        if ((__float_as_uint(dw0) & 0x7FFFFFFFu) != 4u && !ff::product(dw0, N1, N2, dw, true))
+            dw = mul_fd_rn(dw0, 0.9);
+    } else if (!ff::spnet_dw(dw0, f1, f2, dw)) {
         dw = spnet_dw_full(dw0, f1, f2);
     }
-    dws[wi] = dw;
-    float weight_delta;
-    if (!ff::add_const(dw, S1, S2, weight_delta)) weight_delta = d2f_rn(__dadd_rn(f2d_exact(dw), 0.01));
+    if (__float_as_uint(dw) != __float_as_uint(dw0)) dws[wi] = dw;
+    // dw + 0.01 in double; what is below 2^-60 is gone in it
+    float weight_delta = S1;
+    if (fabsf(dw) > 8.673617379884035e-19f && !ff::add_const(dw, S1, S2, weight_delta))
+        weight_delta = d2f_rn(__dadd_rn(f2d_exact(dw), 0.01));
     weight += lr * weight_delta;
     const float capped = (max_weight < weight) ? max_weight : weight;
     w[wi] = (0.0001f > capped) ? 0.0001f : capped;
@@ -1377,14 +1449,36 @@ class SpnetModel : public Model {
         ctx.count(2);
     }
 
-    void update(State&, LayerState& ls, const StepCtx& ctx) const override {
-        const Layer& l = *ls.layer;
-        k_spnet_update<<<blocks_for(l.size, 256), 256, 0, ctx.stream>>>(
-            l.size, l.history(), ls.input->df(), ls.output->du(), ls.var("voltage")->df(),
-            ls.var("recovery")->df(), ls.var("post trace")->df(), ls.var("time since spike")->di(),
-            ls.var("a")->df(), ls.var("b")->df(), ls.var("c")->df(), ls.var("d")->df());
-        SG_LAUNCH_CHECK();
-        ctx.count();
+    void update(State& st, LayerState& ls, const StepCtx& ctx) const override {
+        std::vector<LayerState*> one{&ls};
+        update_group(st, one, ctx);
+    }
+
+    bool update_group(State&, const std::vector<LayerState*>& group,
+                      const StepCtx& ctx) const override {
+        for (size_t first = 0; first < group.size(); first += kIzGroup) {
+            SpnetUpdateGroup G{};
+            G.n = (int)std::min<size_t>(kIzGroup, group.size() - first);
+            int total = 0;
+            for (int i = 0; i < G.n; ++i) {
+                LayerState& ls = *group[first + i];
+                const Layer& l = *ls.layer;
+                G.start[i] = total;
+                G.L[i] = SpnetLayerArgs{l.size, l.history(), ls.input->df(), ls.output->du(),
+                                        ls.var("voltage")->df(), ls.var("recovery")->df(),
+                                        ls.var("post trace")->df(),
+                                        ls.var("time since spike")->di(), ls.var("a")->df(),
+                                        ls.var("b")->df(), ls.var("c")->df(), ls.var("d")->df()};
+                total += l.size;
+            }
+            G.start[G.n] = total;
+            if (total == 0) continue;
+            const int threads = update_threads(total);
+            k_spnet_update<<<blocks_for(total, threads), threads, 0, ctx.stream>>>(G);
+            SG_LAUNCH_CHECK();
+            ctx.count();
+        }
+        return true;
     }
 
     bool learns(const Connection& c) const override { return true; }

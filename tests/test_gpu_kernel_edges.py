@@ -209,3 +209,100 @@ def test_rate_tiles(cfg):
                                         *(g.data_ptr() for g in grads), stream) == 0
     for a, b in zip([loss] + grads, results[0]):
         np.testing.assert_allclose(a.cpu().numpy(), b, rtol=1e-4, atol=1e-4 * np.abs(b).max())
+
+
+@pytest.mark.parametrize("opcode", ["add", "sub"])
+@pytest.mark.parametrize("rows,cols", [(1, 7), (10, 33)])
+def test_spnet_neurons_and_sparse_learning(sg, opcode, rows, cols):
+    """Zero and nonzero traces and derivatives, spikes on either side, voltages
+    on both sides of the threshold; two layers of different sizes in one launch."""
+    from tests.golden.cases import Case
+    from tests.harness import compare, run_library, run_oracle
+    n, m = rows * cols, (rows + 2) * cols
+    net = network([layer("a", "spnet", rows, cols, params="regular"),
+                   layer("b", "spnet", rows + 2, cols, params="fast")],
+                  [connection("c", "a", "b", "fully connected", opcode=opcode, plastic=True,
+                              sparse=True)])
+
+    def inject(rng, sizes):
+        size, dense = sizes["conn:c"], sizes["dense:c"]
+        draw = lambda lo, hi, k: rng.uniform(lo, hi, k).astype(np.float32)    # noqa: E731
+        some = lambda v: np.where(rng.random(v.size) < 0.4, 0, v).astype(np.float32)  # noqa: E731
+        words = rng.integers(0, 2**32, n, dtype=np.uint64).astype(np.uint32)
+        kept = np.arange(dense) % 5 < 3                      # as many for every destination
+        size = int(kept.sum()) if size == dense else size
+        got = {("matrix", "c", "init weights"): np.where(kept, draw(0.1, 5, dense), 0).astype(np.float32),
+               ("neuron", "s", "a", "output"): words, ("neuron", "s", "a", "voltage"): draw(-90, 45, n),
+               ("neuron", "s", "b", "voltage"): draw(-90, 45, m),
+               ("neuron", "s", "a", "recovery"): draw(-20, 20, n),
+               ("neuron", "s", "b", "post trace"): some(draw(0, 1, m)),
+               ("neuron", "s", "b", "time since spike"): rng.integers(0, 33, m).astype(np.int32)}
+        if n % 5 == 0:
+            got[("matrix", "c", "presyn trace")] = some(draw(0, 1, size))
+            got[("matrix", "c", "weight derivative")] = some(draw(-0.1, 0.1, size))
+        return got
+
+    final = [("neuron", "s", "a", k) for k in ("voltage", "recovery", "output")]
+    final += [("neuron", "s", "b", k) for k in ("voltage", "recovery", "post trace", "output", "input")]
+    final += [("matrix", "c", k) for k in ("weights", "presyn trace", "weight derivative",
+                                           "time since spike")]
+    case = Case("spnet_edges", net, 40, rows * cols, inject=inject, final=final,
+                inputs={"a": lambda rng, t, k: (rng.random(k) < 0.2) * 20.0,
+                        "b": lambda rng, t, k: (rng.random(k) < 0.2) * 20.0})
+    problems = compare(run_library(case, sg), run_oracle(case))
+    assert not problems, problems[:3]
+
+
+def test_state_moves_only_what_was_handed_out(sg, tmp_path):
+    """A caller that reads and changes a few arrays, late and between runs, over a
+    save and a load, sees what one that holds every array sees."""
+    from tests.golden.configs import c0_inject, c0_net
+    from tests.harness import case_sizes
+    from tests.golden.cases import Case
+    case = Case("state", c0_net(8), 1, 5, inject=lambda rng, sizes: c0_inject(rng, sizes, 8))
+    inject = case.injections(case_sizes(case))
+    net_dict = case.net
+    for c in net_dict["connections"]:
+        c["myelinated"] = True
+    keys = [("iz", k) for k in ("voltage", "recovery", "output", "input", "nmda", "time since spike")]
+    keys += [("in", "output"), ("in", "input")]
+    keys += [("matrix", c, k) for c in ("c_in", "c_rec") for k in ("weights", "long trace", "delays")]
+
+    def run(hold_all):
+        net = sg.Network(net_dict)
+        net.build_state()
+
+        def get(key):
+            if key[0] == "matrix":
+                return net.get_weight_matrix(key[1], key[2]).to_np_array()
+            return net.get_neuron_data("s", key[0], key[1]).to_np_array()
+
+        def step(n):
+            if hold_all:
+                [get(k) for k in keys]
+            net.run({"modules": []}, {"iterations": n, "learning flag": False, "graphs": False})
+
+        for key, values in inject.items():
+            dst = get(key[1:] if key[0] == "matrix" and False else
+                      (key if key[0] == "matrix" else key[2:]))
+            dst.view(values.dtype)[:] = values
+        step(3)
+        get(("iz", "voltage"))[:] -= 1.0
+        step(2)
+        kept = get(("matrix", "c_in", "long trace"))          # first handed out after runs
+        kept *= 2.0
+        step(4)
+        get(("iz", "recovery"))
+        kept *= 0.5                                           # refreshed by any getter
+        step(2)
+        path = str(tmp_path / ("state%d" % hold_all))
+        get(("iz", "voltage"))[:] += 0.5
+        net.save_state(path)
+        step(3)
+        net.load_state(path)
+        step(5)
+        return {k: get(k).copy().view(np.uint32) for k in keys}
+
+    few, every = run(False), run(True)
+    for k in keys:
+        assert np.array_equal(few[k], every[k]), k
