@@ -194,8 +194,9 @@ ARRAY get_neuron_data(STATE st, char* structure, char* layer, char* key) {
     SG_TRY(null_array())
     auto* h = (StateHandle*)st;
     Layer* l = h->net->layer(structure, layer);
-    if (!h->state->on_host()) h->state->to_host(engine_stream());
-    return array_of(h->state->layer_state(l)->var(key));
+    Array* a = h->state->layer_state(l)->var(key);
+    h->state->expose(a);
+    return array_of(a);
     SG_CATCH(null_array())
 }
 
@@ -206,8 +207,9 @@ ARRAY get_weight_matrix(STATE st, char* conn, char* key) {
     SG_TRY(null_array())
     auto* h = (StateHandle*)st;
     Connection* c = h->net->connection(conn);
-    if (!h->state->on_host()) h->state->to_host(engine_stream());
-    return array_of(h->state->conn_state(c)->var(key ? key : "weights"));
+    Array* a = h->state->conn_state(c)->var(key ? key : "weights");
+    h->state->expose(a);
+    return array_of(a);
     SG_CATCH(null_array())
 }
 

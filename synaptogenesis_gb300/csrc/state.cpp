@@ -8,6 +8,7 @@
 #include <functional>
 
 #include "cuda_check.h"
+#include "engine.h"
 #include "models.h"
 #include "weight_init.h"
 
@@ -263,7 +264,8 @@ void State::to_device(cudaStream_t stream) {
     // buffer and a conversion kernel; the stream orders each conversion
     // before the next copy into the buffer.
     for (auto& a : arrays_) {
-        if (a->dev_count == 0 || a->scratch) continue;
+        if (a->dev_count == 0 || a->scratch || (a->on_device && !a->exposed)) continue;
+        a->on_device = true;
         const uint32_t* src = a->host.data();
         if (a->layout == LAYOUT_BANDED) {
             SG_CUDA(cudaMemcpyAsync(stage_, src, a->count * 4, cudaMemcpyHostToDevice, stream));
@@ -282,29 +284,48 @@ void State::to_device(cudaStream_t stream) {
     on_host_ = false;
 }
 
-void State::to_host(cudaStream_t stream) {
-    if (on_host_) return;
-    SG_CUDA(cudaStreamSynchronize(stream));
-    check_iz_cols_errors();
-    check_debug_errors();
-    for (auto& a : arrays_) {
-        if (a->dev_count == 0 || a->scratch) continue;
-        const size_t n = std::min(a->dev_count, a->count);
-        if (a->layout == LAYOUT_BANDED) {
-            launch_from_bands(a->du(), stage_, a->rows, a->cols, a->dev_count, stream);
-            SG_CUDA(cudaMemcpyAsync(a->host.data(), stage_, a->count * 4, cudaMemcpyDeviceToHost,
-                                    stream));
-        } else if (needs_transpose(*a)) {
-            // device [cols][rows] -> host [rows][cols]
-            launch_transpose(a->du(), stage_, a->cols, a->rows, stream);
-            SG_CUDA(cudaMemcpyAsync(a->host.data(), stage_, a->count * 4, cudaMemcpyDeviceToHost,
-                                    stream));
-        } else {
-            SG_CUDA(cudaMemcpyAsync(a->host.data(), a->dev, n * 4, cudaMemcpyDeviceToHost, stream));
-        }
+void State::download(Array& a, cudaStream_t stream) {
+    if (a.layout == LAYOUT_BANDED) {
+        launch_from_bands(a.du(), stage_, a.rows, a.cols, a.dev_count, stream);
+        SG_CUDA(cudaMemcpyAsync(a.host.data(), stage_, a.count * 4, cudaMemcpyDeviceToHost, stream));
+    } else if (needs_transpose(a)) {
+        // device [cols][rows] -> host [rows][cols]
+        launch_transpose(a.du(), stage_, a.cols, a.rows, stream);
+        SG_CUDA(cudaMemcpyAsync(a.host.data(), stage_, a.count * 4, cudaMemcpyDeviceToHost, stream));
+    } else {
+        SG_CUDA(cudaMemcpyAsync(a.host.data(), a.dev, std::min(a.dev_count, a.count) * 4,
+                                cudaMemcpyDeviceToHost, stream));
     }
-    SG_CUDA(cudaStreamSynchronize(stream));
+}
+
+void State::to_host(cudaStream_t stream, bool all) {
+    const bool newer = !on_host_;
+    if (!newer && !all) return;
+    if (newer) {
+        SG_CUDA(cudaStreamSynchronize(stream));
+        check_iz_cols_errors();
+        check_debug_errors();
+    }
+    bool any = false;
+    for (auto& a : arrays_) {
+        if (!a->on_device || (a->exposed ? !newer : !all)) continue;
+        download(*a, stream);
+        any = true;
+    }
+    if (any) SG_CUDA(cudaStreamSynchronize(stream));
     on_host_ = true;
+}
+
+void State::expose(Array* a) {
+    const bool late = !a->exposed && on_host_ && a->on_device;
+    a->exposed = true;
+    if (!late && on_host_) return;
+    const cudaStream_t stream = engine_stream();
+    if (late) {
+        download(*a, stream);
+        SG_CUDA(cudaStreamSynchronize(stream));
+    }
+    to_host(stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -342,7 +363,7 @@ static std::vector<Rec> records(State& st) {
 }
 
 void State::save(const std::string& path) {
-    to_host(0);
+    to_host(0, true);
     std::ofstream f(path, std::ios::binary);
     if (!f) throw SgError("Error writing state to file!");
     for (auto& r : records(*this)) {
@@ -357,7 +378,8 @@ void State::save(const std::string& path) {
 void State::load(const std::string& path) {
     std::ifstream f(path, std::ios::binary);
     if (!f) throw SgError("Could not open file: " + path);
-    to_host(0);
+    to_host(0, true);
+    for (auto& a : arrays_) a->on_device = false;
     auto recs = records(*this);
     for (;;) {
         size_t key[3];

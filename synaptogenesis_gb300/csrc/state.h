@@ -5,7 +5,10 @@
 // GPU layout (per-synapse arrays transposed so consecutive destinations are
 // contiguous, src/core/state/weight_matrix.cpp:192-228).  Device copies live in
 // one arena allocation.  Like the reference (state.cpp:259-323), handing out
-// host pointers moves the state to the host, and the next run moves it back.
+// host pointers moves the state to the host, and the next run moves it back --
+// but only the arrays of which a host pointer was ever handed out: no caller can
+// read or change the others.  Once handed out an array always moves, since the
+// caller may keep the pointer.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -38,6 +41,8 @@ struct Array {
     void* dev = nullptr;
     size_t dev_offset = 0;
     bool scratch = false;    // device-only working buffer: never uploaded or downloaded
+    bool on_device = false;  // uploaded, and no load() has replaced it since
+    bool exposed = false;    // a getter has handed out its host copy
 
     float* hf() { return reinterpret_cast<float*>(host.data()); }
     int32_t* hi() { return reinterpret_cast<int32_t*>(host.data()); }
@@ -134,8 +139,11 @@ class State {
 
     // Host <-> device movement.
     void to_device(cudaStream_t stream);     // uploads if the host copy is newer
-    void to_host(cudaStream_t stream);       // downloads if the device copy is newer
-    bool on_host() const { return on_host_; }
+    // downloads the exposed arrays if the device copy is newer; with `all`, every
+    // other array too (a snapshot)
+    void to_host(cudaStream_t stream, bool all = false);
+    // marks an array exposed, its host copy up to date with the others'
+    void expose(Array* a);
     void mark_device_newer() { on_host_ = false; }
 
     // Output word `word` of a layer on the device.
@@ -153,6 +161,7 @@ class State {
   private:
     void build();
     void allocate_device();
+    void download(Array& a, cudaStream_t stream);
     std::vector<std::unique_ptr<Array>> arrays_;
     void* arena_ = nullptr;
     size_t arena_bytes_ = 0;
