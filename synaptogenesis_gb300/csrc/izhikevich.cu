@@ -433,31 +433,40 @@ __global__ void k_iz_gap(DGeom g, const float* __restrict__ voltage, const float
 // Every visit with the same delay reads the same spike bit, so a source's
 // last (at most 32) visits are summarised after each upload
 // (k_iz_delay_summary) as, per distinct delay, the position of its last
-// visit: the latest position whose delay shows a spike decides.  A source
-// with more than kSummary distinct delays among those visits scans them.
+// visit, latest first: the first whose delay shows a spike decides.  A source
+// with more than kSummary distinct delays among those visits scans them, a
+// dependent gather per visit: with room for 6, the 15 x 15 fields of spnet's
+// distance delays (7 or 8 of them) took 13.3 us for 65,536 sources, 32 loads deep;
+// with 12 they take 3.8 us.
 //
-// Summary word: bits 0-2 the number of entries (7: scan), entry i in bits
-// 3 + 10 i: delay (5 bits), then position (5 bits).
-constexpr int kSummary = 6;
+// Summary: two words.  Bits 0-3 of the first hold the number of entries (15: scan),
+// entries 0-5 follow in bits 4 + 10 i, entries 6-11 are bits 10 (i - 6) of the
+// second; an entry is delay (5 bits), then position (5 bits).
+constexpr int kSummary = 12;
+constexpr int kSummaryScan = 15;
 
 __device__ __forceinline__ void tss_update(int f, const int* __restrict__ counts,
                                            const int* __restrict__ last,
                                            const int* __restrict__ delays,
-                                           const unsigned long long* __restrict__ summary,
+                                           const ulonglong2* __restrict__ summary,
                                            const uint32_t* __restrict__ src, int src_type,
                                            int* __restrict__ tss) {
-    int n = counts[f];
+    const int n = counts[f];
+    const uint32_t word = src[f];
+    const ulonglong2 sm = summary[f];
     if (n == 0) return;
-    uint32_t word = src[f];
     const int m = n < 32 ? n : 32;
-    const unsigned long long sm = summary[f];
-    const int ne = (int)(sm & 7);
-    if (ne != 7) {
+    const int ne = (int)(sm.x & 15);
+    if (ne != kSummaryScan) {
+        unsigned long long part = sm.x >> 4;
         int best = -1;
-        for (int i = 0; i < ne; ++i) {
-            const int e = (int)(sm >> (3 + 10 * i)) & 1023;
-            const int pos = e >> 5;
-            if (pos > best && extract_rt(word, e & 31, src_type) > 0.0f) best = pos;
+        for (int i = 0; i < ne; ++i, part >>= 10) {
+            if (i == 6) part = sm.y;
+            const int e = (int)part & 1023;
+            if (extract_rt(word, e & 31, src_type) > 0.0f) {
+                best = e >> 5;
+                break;
+            }
         }
         if (best >= 0) {
             tss[f] = m - 1 - best;
@@ -478,7 +487,7 @@ __device__ __forceinline__ void tss_update(int f, const int* __restrict__ counts
 
 __global__ void k_iz_time_since_spike(int n_src, const int* __restrict__ counts,
                                       const int* __restrict__ last, const int* __restrict__ delays,
-                                      const unsigned long long* __restrict__ summary,
+                                      const ulonglong2* __restrict__ summary,
                                       const uint32_t* __restrict__ src, int src_type,
                                       int* __restrict__ tss) {
     int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -491,7 +500,7 @@ __global__ void k_iz_time_since_spike(int n_src, const int* __restrict__ counts,
 struct TssArgs {
     int n_src, src_type;
     const int *counts, *last, *delays;
-    const unsigned long long* summary;
+    const ulonglong2* summary;
     const uint32_t* src;
     int* tss;
 };
@@ -512,12 +521,12 @@ __global__ void k_iz_time_since_spike_group(TssGroup G) {
 }
 __global__ void k_iz_delay_summary(int n_src, const int* __restrict__ counts,
                                    const int* __restrict__ last, const int* __restrict__ delays,
-                                   unsigned long long* __restrict__ summary) {
+                                   ulonglong2* __restrict__ summary) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= n_src) return;
     const int m = min(counts[f], 32);
     const int* L = last + (size_t)f * 32;
-    unsigned long long sm = 0;
+    unsigned long long part[2] = {0, 0};
     unsigned seen = 0;
     int ne = 0;
     for (int j = m - 1; j >= 0 && ne <= kSummary; --j) {
@@ -525,10 +534,12 @@ __global__ void k_iz_delay_summary(int n_src, const int* __restrict__ counts,
         if (d < 0 || d > 31) { ne = kSummary + 1; break; }
         if (seen & (1u << d)) continue;
         seen |= 1u << d;
-        if (ne < kSummary) sm |= (unsigned long long)(d | (j << 5)) << (3 + 10 * ne);
+        if (ne < kSummary)
+            part[ne / 6] |= (unsigned long long)(d | (j << 5)) << (ne < 6 ? 4 + 10 * ne : 10 * (ne - 6));
         ++ne;
     }
-    summary[f] = ne > kSummary ? 7ull : (sm | (unsigned long long)ne);
+    part[0] |= (unsigned long long)(ne > kSummary ? kSummaryScan : ne);
+    summary[f] = make_ulonglong2(part[0], part[1]);
 }
 
 // trace * 0.95 in double, rounded to float.
@@ -751,7 +762,7 @@ static void iz_delays_and_visits(State& st, ConnState& cs) {
     int nsrc = c.from->size;
     cs.visit_counts = st.add_array("visit counts", 'i', nsrc);
     cs.last_visits = st.add_array("last visits", 'i', (size_t)nsrc * 32);
-    cs.delay_summary = st.add_array("delay summary", 'i', 0, LAYOUT_PLAIN, 1, 1, (size_t)nsrc * 2);
+    cs.delay_summary = st.add_array("delay summary", 'i', 0, LAYOUT_PLAIN, 1, 1, (size_t)nsrc * 4);
     cs.delay_summary->scratch = true;
     int32_t* cnt = cs.visit_counts->hi();
     int32_t* last = cs.last_visits->hi();
@@ -776,6 +787,34 @@ __global__ void k_iz_delay_bytes_plain(size_t n, const int* __restrict__ delays,
                                        uint8_t* __restrict__ d8) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) d8[i] = (uint8_t)delays[i];
+}
+
+// The time-since-spike updates of several connections, in launches of up to
+// kTssGroup; false (and none made) for fewer than two.
+static bool tss_group(State& st, const std::vector<ConnState*>& todo, const StepCtx& ctx) {
+    if (todo.size() < 2) return false;
+    for (size_t first = 0; first < todo.size(); first += kTssGroup) {
+        TssGroup G{};
+        G.n = (int)std::min<size_t>(kTssGroup, todo.size() - first);
+        int total = 0;
+        for (int i = 0; i < G.n; ++i) {
+            ConnState& cs = *todo[first + i];
+            const Connection& c = *cs.conn;
+            G.start[i] = total;
+            G.C[i] = TssArgs{c.from->size, (int)c.from->output_type, cs.visit_counts->di(),
+                             cs.last_visits->di(), cs.delays->di(),
+                             reinterpret_cast<const ulonglong2*>(cs.delay_summary->di()),
+                             st.dev_output(c.from, word_index(c.delay, c.from->output_type)),
+                             cs.var("time since spike")->di()};
+            total += c.from->size;
+            cs.prologue_done = true;
+        }
+        G.start[G.n] = total;
+        k_iz_time_since_spike_group<<<blocks_for(total, 256), 256, 0, ctx.stream>>>(G);
+        SG_LAUNCH_CHECK();
+        ctx.count();
+    }
+    return true;
 }
 
 class IzhikevichModel : public Model {
@@ -803,7 +842,7 @@ class IzhikevichModel : public Model {
         const int n = cs.conn->from->size;
         k_iz_delay_summary<<<blocks_for(n, 256), 256, 0, s>>>(
             n, cs.visit_counts->di(), cs.last_visits->di(), cs.delays->di(),
-            reinterpret_cast<unsigned long long*>(cs.delay_summary->di()));
+            reinterpret_cast<ulonglong2*>(cs.delay_summary->di()));
         SG_LAUNCH_CHECK();
     }
 
@@ -892,29 +931,7 @@ class IzhikevichModel : public Model {
         std::vector<ConnState*> todo;
         for (ConnState* cs : conns)
             if (trace_connection(*cs->conn) && cs->delay_summary) todo.push_back(cs);
-        if (todo.size() < 2) return false;
-        for (size_t first = 0; first < todo.size(); first += kTssGroup) {
-            TssGroup G{};
-            G.n = (int)std::min<size_t>(kTssGroup, todo.size() - first);
-            int total = 0;
-            for (int i = 0; i < G.n; ++i) {
-                ConnState& cs = *todo[first + i];
-                const Connection& c = *cs.conn;
-                G.start[i] = total;
-                G.C[i] = TssArgs{c.from->size, (int)c.from->output_type, cs.visit_counts->di(),
-                                 cs.last_visits->di(), cs.delays->di(),
-                                 reinterpret_cast<const unsigned long long*>(cs.delay_summary->di()),
-                                 st.dev_output(c.from, word_index(c.delay, c.from->output_type)),
-                                 cs.var("time since spike")->di()};
-                total += c.from->size;
-                cs.prologue_done = true;
-            }
-            G.start[G.n] = total;
-            k_iz_time_since_spike_group<<<blocks_for(total, 256), 256, 0, ctx.stream>>>(G);
-            SG_LAUNCH_CHECK();
-            ctx.count();
-        }
-        return true;
+        return tss_group(st, todo, ctx);
     }
 
     void activate(State& st, ConnState& cs, const StepCtx& ctx) const override {
@@ -958,7 +975,7 @@ class IzhikevichModel : public Model {
         } else {
             k_iz_time_since_spike<<<blocks_for(c.from->size, 256), 256, 0, ctx.stream>>>(
                 c.from->size, cs.visit_counts->di(), cs.last_visits->di(), cs.delays->di(),
-                reinterpret_cast<const unsigned long long*>(cs.delay_summary->di()), src,
+                reinterpret_cast<const ulonglong2*>(cs.delay_summary->di()), src,
                 (int)c.from->output_type, cs.var("time since spike")->di());
             SG_LAUNCH_CHECK();
             ctx.count();
@@ -1192,6 +1209,142 @@ __global__ void __launch_bounds__(128) k_spnet_activate(DGeom g, const uint32_t*
     inputs[to] = aggregate(inputs[to], sum, opcode);
 }
 
+// Sparse connections whose destinations, in blocks of kWindowDests, draw on few
+// sources: a block's outputs are staged in shared memory (`window` of them from
+// first[block] on, around the layer's end), and a synapse is one word, its source's
+// place in the window | its delay << 27 (k_spnet_pack).  A warp's 32 sources lie on
+// some 20 lines of the output array, which the cache looks up one a cycle: 7.3 M
+// synapses of 65,536 destinations took 27 us through it, with 12 bytes read a
+// synapse.  With the outputs from shared memory and 8 bytes for each of kSpnetAhead
+// to 2 kSpnetAhead synapses in flight a thread they take 20 us; bound by the 24
+// instructions a synapse in the 13 warps of an SM, not by bytes.
+constexpr int kSpnetAhead = 16;
+constexpr int kWindowDests = 128;
+
+__global__ void k_spnet_pack(DGeom g, size_t n, const int* __restrict__ delays,
+                             const int* __restrict__ first, int n_src, uint32_t* __restrict__ packed) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int d = (int)(i % (size_t)g.to_size), k = (int)(i / (size_t)g.to_size);
+    if (k >= g.nz[d]) return;
+    int at = g.sfrom[i] - first[d / kWindowDests];
+    if (at < 0) at += n_src;
+    packed[i] = (uint32_t)at * 4 | (uint32_t)delays[i] << 27;
+}
+
+template <int SR>
+__global__ void __launch_bounds__(kWindowDests) k_spnet_activate_window(
+    DGeom g, const uint32_t* __restrict__ src, int n_src, const int* __restrict__ first, int window,
+    const uint32_t* __restrict__ packed, const float* __restrict__ w, float gc, int opcode,
+    float* __restrict__ inputs) {
+    extern __shared__ uint32_t staged[];
+    const unsigned d = blockIdx.x * kWindowDests + threadIdx.x;
+    const int n = d < (unsigned)g.n_dest ? g.nz[d] : 0;
+    const unsigned stride = (unsigned)g.to_size;
+    const int lo = first[blockIdx.x];
+    auto stage = [&] {
+        for (int i = threadIdx.x; i < window; i += kWindowDests) {
+            const int from = lo + i;
+            staged[i] = src[from < n_src ? from : from - n_src];
+        }
+        __syncthreads();
+    };
+    float sum = 0.0f;
+    const int nmin = __reduce_min_sync(0xFFFFFFFFu, n), nmax = __reduce_max_sync(0xFFFFFFFFu, n);
+    const unsigned at0 = min(d, stride - 1);
+    uint32_t x[2][kSpnetAhead] = {};
+    float v[2][kSpnetAhead] = {};
+    auto load = [&](int b, int i) {
+        unsigned at = at0 + (unsigned)i * stride;
+        if (i + kSpnetAhead <= nmax) {
+#pragma unroll
+            for (int u = 0; u < kSpnetAhead; ++u, at += stride) {
+                x[b][u] = __ldg(packed + at);
+                v[b][u] = __ldg(w + at);
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < kSpnetAhead; ++u, at += stride)
+                if (i + u < nmax) {
+                    x[b][u] = __ldg(packed + at);
+                    v[b][u] = __ldg(w + at);
+                }
+        }
+    };
+    auto term = [&](uint32_t xu, float vu) {
+        const uint32_t word = *reinterpret_cast<const uint32_t*>(
+            reinterpret_cast<const char*>(staged) + (xu & 0xFFFFu));
+        // extract, a bit's 1 without a conversion
+        const float spike = SR == S_BIT
+            ? __int_as_float(((int)(word << (xu >> 27)) >> 31) & 0x3F800000)
+            : extract<SR>(word, 0);
+        return spike * vu * gc;
+    };
+    auto add = [&](int b, int i) {
+        if (i + kSpnetAhead <= nmin) {
+#pragma unroll
+            for (int u = 0; u < kSpnetAhead; ++u) sum += term(x[b][u], v[b][u]);
+        } else {
+#pragma unroll
+            for (int u = 0; u < kSpnetAhead; ++u) {
+                // what lies past n is a zero word or an earlier one: a place in the window
+                const float t = term(x[b][u], v[b][u]);
+                sum = i + u < n ? sum + t : sum;
+            }
+        }
+    };
+    load(0, 0);
+    load(1, kSpnetAhead);
+    stage();
+    for (int i = 0; i < nmax; i += 2 * kSpnetAhead) {
+        add(0, i);
+        load(0, i + 2 * kSpnetAhead);
+        add(1, i + kSpnetAhead);
+        load(1, i + 3 * kSpnetAhead);
+    }
+    if (d < (unsigned)g.n_dest) inputs[d] = aggregate(inputs[d], sum, opcode);
+}
+
+// The windows of a sparse connection: per block of destinations the shortest run of
+// sources, around the layer's end, that holds all of theirs, in groups of 32.
+// Staged where the longest is at most kWindowWords (48 KB) and the blocks stage less
+// than half of what they gather.
+constexpr int kWindowWords = 12288;
+
+static void spnet_windows(State& st, ConnState& cs) {
+    if (!cs.sparse_from) return;
+    const Connection& c = *cs.conn;
+    const int n_src = c.from->size, n_dest = c.to->size, K = c.matrix_cols;
+    const int groups = (n_src + 31) / 32, blocks = (n_dest + kWindowDests - 1) / kWindowDests;
+    const int32_t* nz = cs.sparse_nonzero->hi();
+    const int32_t* from = cs.sparse_from->hi();
+    std::vector<int32_t> first(blocks, 0);
+    std::vector<uint8_t> used(groups);
+    long window = 0, gathers = 0;
+    for (int b = 0; b < blocks; ++b) {
+        std::fill(used.begin(), used.end(), 0);
+        for (int d = b * kWindowDests; d < std::min(n_dest, (b + 1) * kWindowDests); ++d) {
+            for (int k = 0; k < nz[d]; ++k) used[from[(size_t)d * K + k] / 32] = 1;
+            gathers += nz[d];
+        }
+        // the longest circular run of unused groups ends where the window starts
+        int gap = 0, start = 0, run = 0;
+        for (int i = 0; i < 2 * groups && run < groups; ++i) {
+            run = used[i % groups] ? 0 : run + 1;
+            if (run > gap) { gap = run; start = (i + 1) % groups; }
+        }
+        first[b] = start * 32;
+        window = std::max(window, (long)std::min(n_src, (groups - gap) * 32));
+    }
+    if (window > kWindowWords || window * blocks * 2 > gathers) return;
+    cs.window = (int)window;
+    cs.window_first = st.add_array("source windows", 'i', blocks);
+    std::memcpy(cs.window_first->hi(), first.data(), (size_t)blocks * 4);
+    cs.sparse_packed = st.add_array("packed sources", 'u', 0, LAYOUT_PLAIN, 1, 1,
+                                    cs.sparse_from->dev_count);
+    cs.sparse_packed->scratch = true;
+}
+
 // The substep's double expressions in double, where a rounding test fails.
 static __device__ __noinline__ float spnet_delta_double(float voltage, float recovery, float current) {
     return (0.04 * voltage * voltage) + (5 * voltage) + 140 - recovery + current;
@@ -1305,18 +1458,22 @@ static __device__ __noinline__ float spnet_dw_full(float dw0, float f1, float f2
     return d2f_rn(__dadd_rn(__dadd_rn(mul_df_rn(dw0, 0.9), f2d_exact(f1)), -f2d_exact(f2)));
 }
 
-// Sparse connections: one thread per compacted synapse (blockIdx.y is the
-// synapse's rank within its destination, x the destination), since each
+// Sparse connections: a thread takes kSpnetRanks compacted synapses of one
+// destination (blockIdx.y is their ranks' group, x the destination), since each
 // synapse's update is independent.  The double expressions are float-float
 // evaluations with a rounding test (ff_exact.cuh), falling back to integer helpers
 // and double sums where it rejects, which a warp pays for if one of its 32 synapses
 // does: products with 0.9 and 0.95 that land on a midpoint (one in 10 or 20), zero
 // and silent traces and derivatives, and sums with spike terms are therefore decided
-// on the fast path.  Issue bounds it (about 200 instructions a synapse): 7.3 M
-// synapses of a network that has run a while took 102 us with those on the slow
-// path, 78 us now.  Bit-identical to k_spnet_learn.
+// on the fast path.  Memory latency bounds it, two loads deep: 28 bytes a synapse and
+// its source's spike.  7.3 M synapses of a network that has run a while: 70 us (102
+// with those expressions on the slow path, 78 with a synapse a thread).
+// Bit-identical to k_spnet_learn.
+constexpr int kSpnetRanks = 4;
+constexpr int kSpnetLearnThreads = 128;
+
 template <int SR, bool SUB>
-__global__ void __launch_bounds__(256) k_spnet_learn_sparse(DGeom g, const uint32_t* __restrict__ dest_out,
+__global__ void __launch_bounds__(kSpnetLearnThreads) k_spnet_learn_sparse(DGeom g, const uint32_t* __restrict__ dest_out,
                                                             const float* __restrict__ post,
                                                             const int* __restrict__ to_tss,
                                                             const int* __restrict__ from_tss, float lr,
@@ -1324,70 +1481,88 @@ __global__ void __launch_bounds__(256) k_spnet_learn_sparse(DGeom g, const uint3
                                                             float* __restrict__ presyn,
                                                             float* __restrict__ dws, IzLut lut) {
     const unsigned d = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y;
+    const int i0 = blockIdx.y * kSpnetRanks;
     if (d >= (unsigned)g.to_size) return;
     // every load that depends on nothing but the synapse's position first
-    // (the [kmax][to] arrays are allocated for the padding too), then the
-    // checks, then the source's time since spike
-    const unsigned wi = (unsigned)i * g.to_size + d;
-    const int n = g.nz[d];
-    float weight = w[wi];
-    const unsigned from = (unsigned)g.sfrom[wi];
-    const float p = SUB ? 0.0f : presyn[wi];
-    const float dw0 = dws[wi];
+    // (the [kmax][to] arrays are allocated for the padding too), then the sources'
+    // times since spike, then the updates
+    const unsigned stride = (unsigned)g.to_size;
+    const unsigned at = (unsigned)i0 * stride + d;
+    const int n = g.nz[d] - i0;
+    const int ranks = min(kSpnetRanks, g.kmax - i0);
+    float ws[kSpnetRanks], ps[kSpnetRanks], dw0s[kSpnetRanks];
+    int stsss[kSpnetRanks];
+#pragma unroll
+    for (int r = 0; r < kSpnetRanks; ++r)
+        if (r < ranks) {
+            const unsigned wi = at + r * stride;
+            stsss[r] = g.sfrom[wi];
+            ws[r] = w[wi];
+            ps[r] = SUB ? 0.0f : presyn[wi];
+            dw0s[r] = dws[wi];
+        }
     const uint32_t dword = dest_out[d];
     const float dest_exc = SUB ? 0.0f : post[d];
     const int dtss = SUB ? to_tss[d] : 0;
-    if (i >= n || !(weight >= 0.0001f)) return;
-    const int stss = from_tss[from];
-    const bool src_spike = stss == 0;
+#pragma unroll
+    for (int r = 0; r < kSpnetRanks; ++r)
+        if (r < n) stsss[r] = from_tss[stsss[r]];
     const float dest_spike = extract<SR>(dword, 0);          // the source's extractor
-    float src_trace, dest_trace;
-    if (!SUB) {
-        float np;
-        constexpr float T1 = (float)0.1, T2 = (float)(0.1 - (double)T1);
-        constexpr float D1 = (float)0.95, D2 = (float)(0.95 - (double)D1);
-        // 0.95 x 10 units of 2^-149 rounds back to them: where a silent trace ends
-        if (src_spike) {
-            if (!ff::add_const(p, T1, T2, np)) np = spnet_trace_step(p);
-            presyn[wi] = np;
-        } else if (p == 0.0f || (__float_as_uint(p) & 0x7FFFFFFFu) == 10u) {
-            np = p;
+#pragma unroll
+    for (int r = 0; r < kSpnetRanks; ++r) {
+        if (r >= n || !(ws[r] >= 0.0001f)) continue;
+        const unsigned wi = at + r * stride;
+        float weight = ws[r];
+        const float p = ps[r], dw0 = dw0s[r];
+        const int stss = stsss[r];
+        const bool src_spike = stss == 0;
+        float src_trace, dest_trace;
+        if (!SUB) {
+            float np;
+            constexpr float T1 = (float)0.1, T2 = (float)(0.1 - (double)T1);
+            constexpr float D1 = (float)0.95, D2 = (float)(0.95 - (double)D1);
+            // 0.95 x 10 units of 2^-149 rounds back to them: where a silent trace ends
+            if (src_spike) {
+                if (!ff::add_const(p, T1, T2, np)) np = spnet_trace_step(p);
+                presyn[wi] = np;
+            } else if (p == 0.0f || (__float_as_uint(p) & 0x7FFFFFFFu) == 10u) {
+                np = p;
+            } else {
+                if (!ff::product(p, D1, D2, np, true)) np = mul_fd_rn(p, 0.95);
+                presyn[wi] = np;
+            }
+            src_trace = np;
+            dest_trace = dest_exc;
         } else {
-            if (!ff::product(p, D1, D2, np, true)) np = mul_fd_rn(p, 0.95);
-            presyn[wi] = np;
+            src_trace = (dest_spike > 0.0f && stss > 0 && stss < 32) ? lut.src[stss] : 0.0f;
+            dest_trace = (src_spike && dtss > 0 && dtss < 32) ? lut.dst[dtss] : 0.0f;
         }
-        src_trace = np;
-        dest_trace = dest_exc;
-    } else {
-        src_trace = (dest_spike > 0.0f && stss > 0 && stss < 32) ? lut.src[stss] : 0.0f;
-        dest_trace = (src_spike && dtss > 0 && dtss < 32) ? lut.dst[dtss] : 0.0f;
+        const float f1 = dest_spike * src_trace;
+        const float f2 = (src_spike ? 1.0f : 0.0f) * dest_trace;
+        // 0.9 dw + f1 - f2 in double: with dw zero the float difference (rounding the
+        // double one again changes nothing: 53 >= 2 * 24 + 2 bits), with f1, f2 zero
+        // the rounded product alone, which leaves 4 units of 2^-149 (a derivative's end)
+        // as they are
+        float dw = dw0;
+        constexpr float N1 = (float)0.9, N2 = (float)(0.9 - (double)N1);
+        constexpr float S1 = (float)0.01, S2 = (float)(0.01 - (double)S1);
+        if (dw0 == 0.0f) {
+            dw = dw0 + f1 - f2;
+        } else if (f1 == 0.0f && f2 == 0.0f) {
+            if ((__float_as_uint(dw0) & 0x7FFFFFFFu) != 4u && !ff::product(dw0, N1, N2, dw, true))
+                dw = mul_fd_rn(dw0, 0.9);
+        } else if (!ff::spnet_dw(dw0, f1, f2, dw)) {
+            dw = spnet_dw_full(dw0, f1, f2);
+        }
+        if (__float_as_uint(dw) != __float_as_uint(dw0)) dws[wi] = dw;
+        // dw + 0.01 in double; what is below 2^-60 is gone in it
+        float weight_delta = S1;
+        if (fabsf(dw) > 8.673617379884035e-19f && !ff::add_const(dw, S1, S2, weight_delta))
+            weight_delta = d2f_rn(__dadd_rn(f2d_exact(dw), 0.01));
+        weight += lr * weight_delta;
+        const float capped = (max_weight < weight) ? max_weight : weight;
+        w[wi] = (0.0001f > capped) ? 0.0001f : capped;
     }
-    const float f1 = dest_spike * src_trace;
-    const float f2 = (src_spike ? 1.0f : 0.0f) * dest_trace;
-    // 0.9 dw + f1 - f2 in double: with dw zero the float difference (rounding the
-    // double one again changes nothing: 53 >= 2 * 24 + 2 bits), with f1, f2 zero
-    // the rounded product alone, which leaves 4 units of 2^-149 (a derivative's end)
-    // as they are
-    float dw = dw0;
-    constexpr float N1 = (float)0.9, N2 = (float)(0.9 - (double)N1);
-    constexpr float S1 = (float)0.01, S2 = (float)(0.01 - (double)S1);
-    if (dw0 == 0.0f) {
-        dw = dw0 + f1 - f2;
-    } else if (f1 == 0.0f && f2 == 0.0f) {
-        if ((__float_as_uint(dw0) & 0x7FFFFFFFu) != 4u && !ff::product(dw0, N1, N2, dw, true))
-            dw = mul_fd_rn(dw0, 0.9);
-    } else if (!ff::spnet_dw(dw0, f1, f2, dw)) {
-        dw = spnet_dw_full(dw0, f1, f2);
-    }
-    if (__float_as_uint(dw) != __float_as_uint(dw0)) dws[wi] = dw;
-    // dw + 0.01 in double; what is below 2^-60 is gone in it
-    float weight_delta = S1;
-    if (fabsf(dw) > 8.673617379884035e-19f && !ff::add_const(dw, S1, S2, weight_delta))
-        weight_delta = d2f_rn(__dadd_rn(f2d_exact(dw), 0.01));
-    weight += lr * weight_delta;
-    const float capped = (max_weight < weight) ? max_weight : weight;
-    w[wi] = (0.0001f > capped) ? 0.0001f : capped;
 }
 
 class SpnetModel : public Model {
@@ -1396,11 +1571,18 @@ class SpnetModel : public Model {
     OutputType output_type() const override { return OUT_BIT; }
 
     void prepare_device(State&, ConnState& cs, cudaStream_t s) const override {
+        if (cs.sparse_packed) {
+            const size_t n = cs.sparse_packed->dev_count;
+            k_spnet_pack<<<blocks_for((long)n, 256), 256, 0, s>>>(
+                cs.geom, n, cs.delays->di(), cs.window_first->di(), cs.conn->from->size,
+                cs.sparse_packed->du());
+            SG_LAUNCH_CHECK();
+        }
         if (!cs.delay_summary) return;
         const int n = cs.conn->from->size;
         k_iz_delay_summary<<<blocks_for(n, 256), 256, 0, s>>>(
             n, cs.visit_counts->di(), cs.last_visits->di(), cs.delays->di(),
-            reinterpret_cast<unsigned long long*>(cs.delay_summary->di()));
+            reinterpret_cast<ulonglong2*>(cs.delay_summary->di()));
         SG_LAUNCH_CHECK();
     }
 
@@ -1430,23 +1612,50 @@ class SpnetModel : public Model {
         int32_t* tss = cs.vars["time since spike"]->hi();
         for (size_t i = 0; i < tss_n; ++i) tss[i] = 32;
         iz_delays_and_visits(st, cs);
+        spnet_windows(st, cs);
+    }
+
+    bool activate_prologue(State& st, const std::vector<ConnState*>& conns,
+                           const StepCtx& ctx) const override {
+        return tss_group(st, conns, ctx);
     }
 
     void activate(State& st, ConnState& cs, const StepCtx& ctx) const override {
         const Connection& c = *cs.conn;
         const uint32_t* src = st.dev_output(c.from, word_index(c.delay, c.from->output_type));
-        k_iz_time_since_spike<<<blocks_for(c.from->size, 256), 256, 0, ctx.stream>>>(
-            c.from->size, cs.visit_counts->di(), cs.last_visits->di(), cs.delays->di(),
-            reinterpret_cast<const unsigned long long*>(cs.delay_summary->di()), src, (int)c.from->output_type, cs.var("time since spike")->di());
-        SG_LAUNCH_CHECK();
+        if (cs.prologue_done) {
+            cs.prologue_done = false;
+        } else {
+            k_iz_time_since_spike<<<blocks_for(c.from->size, 256), 256, 0, ctx.stream>>>(
+                c.from->size, cs.visit_counts->di(), cs.last_visits->di(), cs.delays->di(),
+                reinterpret_cast<const ulonglong2*>(cs.delay_summary->di()), src,
+                (int)c.from->output_type, cs.var("time since spike")->di());
+            SG_LAUNCH_CHECK();
+            ctx.count();
+        }
         const unsigned blocks = blocks_for(cs.geom.n_dest, 128);
         float* inputs = input_register(st, cs);
-        SG_DISPATCH_TYPE_SRC((int)c.type, (int)c.from->output_type,
-            (k_spnet_activate<TY, SR><<<blocks, 128, 0, ctx.stream>>>(
-                cs.geom, src, cs.weights->df(), cs.delays->di(), cs.params.at("conductance"),
-                (int)c.opcode, inputs)));
+        if (cs.sparse_packed) {
+            const size_t smem = (size_t)cs.window * 4;
+            const int op = (int)c.opcode;
+#define SG_SPNET_WINDOW(SRV)                                                               \
+    k_spnet_activate_window<SRV><<<blocks, kWindowDests, smem, ctx.stream>>>(              \
+        cs.geom, src, c.from->size, cs.window_first->di(), cs.window, cs.sparse_packed->du(), \
+        cs.weights->df(), cs.params.at("conductance"), op, inputs)
+            switch ((int)c.from->output_type) {
+                case 0: SG_SPNET_WINDOW(0); break;
+                case 1: SG_SPNET_WINDOW(1); break;
+                default: SG_SPNET_WINDOW(2); break;
+            }
+#undef SG_SPNET_WINDOW
+        } else {
+            SG_DISPATCH_TYPE_SRC((int)c.type, (int)c.from->output_type,
+                (k_spnet_activate<TY, SR><<<blocks, 128, 0, ctx.stream>>>(
+                    cs.geom, src, cs.weights->df(), cs.delays->di(), cs.params.at("conductance"),
+                    (int)c.opcode, inputs)));
+        }
         SG_LAUNCH_CHECK();
-        ctx.count(2);
+        ctx.count();
     }
 
     void update(State& st, LayerState& ls, const StepCtx& ctx) const override {
@@ -1492,9 +1701,10 @@ class SpnetModel : public Model {
             return t;
         }();
         if (c.type == SPARSE) {
-            const dim3 grid(blocks_for(c.to->size, 256), std::max(1, cs.geom.kmax));
+            const int kmax = std::max(1, cs.geom.kmax);
+            const dim3 grid(blocks_for(c.to->size, kSpnetLearnThreads), (kmax + kSpnetRanks - 1) / kSpnetRanks);
 #define SG_SPNET_SPARSE(SRV, SUBV)                                                              \
-    k_spnet_learn_sparse<SRV, SUBV><<<grid, 256, 0, ctx.stream>>>(                              \
+    k_spnet_learn_sparse<SRV, SUBV><<<grid, kSpnetLearnThreads, 0, ctx.stream>>>(                              \
         cs.geom, st.dev_output(c.to, 0), to.var("post trace")->df(),                           \
         to.var("time since spike")->di(), cs.var("time since spike")->di(),                    \
         cs.params.at("learning rate"), c.max_weight, cs.weights->df(),                         \

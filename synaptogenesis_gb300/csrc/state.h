@@ -116,6 +116,12 @@ struct ConnState {
     // synapse's source (same layout as the weights).
     Array* sparse_nonzero = nullptr;
     Array* sparse_from = nullptr;
+    // ... and, where blocks of destinations draw on few sources, each block's first
+    // source, their number, and per synapse its place among them | delay << 27
+    // (device only, refilled after every upload).
+    Array* window_first = nullptr;
+    Array* sparse_packed = nullptr;
+    int window = 0;
     Array* var(const std::string& k) const;
 };
 

@@ -306,3 +306,79 @@ def test_state_moves_only_what_was_handed_out(sg, tmp_path):
     few, every = run(False), run(True)
     for k in keys:
         assert np.array_equal(few[k], every[k]), k
+
+
+# summaries of up to 12 distinct delays among a source's last 32 visits, six to a
+# word, and the scan beyond; 16 compacted synapses in flight
+@pytest.mark.parametrize("model", ["izhikevich", "spnet"])
+@pytest.mark.parametrize("delays,dests", [(1, 1), (6, 15), (7, 17), (12, 33), (13, 40), (31, 64)])
+def test_time_since_spike_summaries(sg, model, delays, dests):
+    from tests.golden.cases import Case
+    from tests.harness import compare, run_library, run_oracle
+    layers = [layer("a", model, 3, 13, params="regular"), layer("b", model, 1, dests, params="fast")]
+    conns = [connection("c", "a", "b", "fully connected"), connection("r", "b", "a", "fully connected")]
+    for c in conns:
+        del c["myelinated"]
+        c["sparse"] = model == "spnet"
+
+    def inject(rng, sizes):
+        got = {("neuron", "s", "a", "output"): rng.integers(0, 2**32, 39, dtype=np.uint64).astype(np.uint32)
+               & rng.integers(0, 2**32, 39, dtype=np.uint64).astype(np.uint32)}
+        for c in ("c", "r"):
+            n = sizes["dense:" + c]
+            got[("matrix", c, "init weights")] = rng.uniform(0.1, 1, n).astype(np.float32)
+            got[("matrix", c, "delays")] = rng.integers(0, delays, n).astype(np.int32)
+        return got
+
+    final = [("matrix", c, "time since spike") for c in ("c", "r")]
+    final += [("neuron", "s", l, k) for l in ("a", "b") for k in ("voltage", "input", "output")]
+    case = Case("summaries", network(layers, conns), 6, delays + dests, inject=inject, final=final,
+                inputs={"a": lambda rng, t, k: (rng.random(k) < 0.3) * 30.0})
+    problems = compare(run_library(case, sg), run_oracle(case))
+    assert not problems, problems[:3]
+
+
+# blocks of 128 destinations and the sources they draw on, staged in shared memory
+# (places past the layer's end, groups of 32 sources, ragged rows of 16 synapses) or
+# too many to stage; spikes, numbers and whole numbers as outputs
+@pytest.mark.parametrize("source", ["spnet", "relay", "game_of_life"])
+@pytest.mark.parametrize("rows,cols,field,wrap", [
+    (1, 127, 5, False), (16, 8, 9, True), (3, 43, 3, False), (20, 33, 7, True), (40, 40, 17, True),
+    (120, 120, 3, True), (150, 160, 1, False)])
+def test_spnet_source_windows(sg, source, rows, cols, field, wrap):
+    from tests.golden.cases import Case
+    from tests.harness import compare, run_library, run_oracle
+    half = -(field // 2)                    # the field around its destination
+    net = network([layer("a", source, rows, cols, **({"params": "regular"} if source == "spnet" else {})),
+                   layer("b", "spnet", rows, cols, params="fast")],
+                  [connection("c", "a", "b", "convergent", opcode="sub", sparse=True, plastic=False,
+                              **{"arborized config": {"field size": field, "stride": 1, "wrap": wrap,
+                                                      "offset": half}})])
+
+    n, positions = rows * cols, field * field
+    rng = np.random.default_rng(n + field)
+    bits = rng.integers(0, 2**32, n, dtype=np.uint64).astype(np.uint32)
+    output = {"spnet": bits, "relay": rng.normal(0, 3, n).astype(np.float32).view(np.uint32),
+              "game_of_life": bits % 7}[source]
+    weights = (rng.uniform(0.1, 5, (n, positions)) * (rng.random((n, positions)) < 0.7)).astype(np.float32)
+    delays = rng.integers(0, 32, (n, positions)).astype(np.int32)
+    # the delays of a destination's compacted synapses: nonzero weights inside the layer
+    r, c = np.divmod(np.arange(n)[:, None], cols)
+    dr, dc = np.divmod(np.arange(positions), field)
+    inside = wrap | ((r + dr + half >= 0) & (r + dr + half < rows) & (c + dc + half >= 0) & (c + dc + half < cols))
+    kept = inside & (weights != 0)
+    compact = np.zeros((n, kept.sum(1).max()), np.int32)
+    for d in range(n):
+        compact[d, :kept[d].sum()] = delays[d, kept[d]]
+
+    final = [("neuron", "s", l, k) for l in ("a", "b") for k in ("output", "input")]
+    final += [("matrix", "c", "time since spike"), ("neuron", "s", "b", "voltage")]
+
+    def case(delays):
+        given = {("neuron", "s", "a", "output"): output, ("matrix", "c", "init weights"): weights.ravel(),
+                 ("matrix", "c", "delays"): delays.ravel()}
+        return Case("windows", net, 3, 1, inject=lambda rng, sizes: given, final=final,
+                    inputs={"a": lambda rng, t, k: (rng.random(k) < 0.2) * 20.0})
+
+    problems = compare(run_library(case(delays), sg), run_oracle(case(compact)))
+    assert not problems, problems[:3]
