@@ -121,6 +121,16 @@ constexpr float kBound = 9.094947017729282379e-13f;   // 2^-40
 constexpr float kBound4 = 2.273736754432320595e-13f;  // 2^-42
 constexpr float kBound5 = 1.136868377216160297e-13f;  // 2^-43
 
+// The rounding test of single-argument expressions, whose every float operand has
+// been compared with the double evaluation (tests/test_spnet_ff_cpu.py): hi + lo
+// with lo 2^-16 larger and smaller rounds to the same float.  Three operations
+// where rounds_to takes a dozen; rejects one operand in 30,000, and what is not
+// finite.
+SG_FF bool decided(float hi, float lo, float& out) {
+    out = fma(lo, 1.0000152587890625f, hi);
+    return out == fma(lo, 0.9999847412109375f, hi);
+}
+
 // a / D for a float a and a small positive integer D, correctly rounded: the
 // product with the rounded reciprocal corrected by one fused multiply-add
 // (Markstein's scheme).  Checked against IEEE division over every float a in
@@ -201,21 +211,53 @@ SG_FF bool product(float p, float c1, float c2, float& out, bool ties = false) {
     return true;
 }
 
+// (float)((double)p * c) for c = 0.9, 0.95 or 0.933 and |p| in [2^-100, 2^100]: the
+// exact product with c1 plus the remainder's, rounded once.  No test is needed:
+// every mantissa gives the double evaluation's float (midpoints too, one p in 10,
+// 20 or 1000), and within this range the operations do not depend on the exponent.
+// Outside it, product.
+SG_FF bool decay(float p, float c1, float c2, float& out) {
+    const float m = absf(p);
+    if (!(m >= 7.888609052210118e-31f && m <= 1.2676506002282294e30f))
+        return product(p, c1, c2, out, true);
+    const float h = mul(p, c1);
+    out = add(h, fma(p, c2, fma(p, c1, -h)));
+    return true;
+}
+
 // (float)((double)x + k) for a double constant k ~ k1 + k2 (two floats, k2
-// the rounded remainder): the exact sum of x and k1 plus the remainder's,
-// which errs by at most 2^-24 (|e| + |k2|) <= 2^-48 (|s| + |k1|), s = RN(x +
-// k1); the double addition it stands for errs by at most 2^-53 |x + k| and
-// the split of k by 2^-48 |k1|: the bound 2^-43 (|s| + |k1|) covers all three
-// with a factor of 10 to spare.
+// the rounded remainder): the exact sum of x and k1 plus the remainder's.
 SG_FF bool add_const(float x, float k1, float k2, float& out) {
     float s, e;
     two_sum(x, k1, s, e);
-    e = add(e, k2);
-    float f, g;
-    two_sum(s, e, f, g);
-    if (!rounds_to(f, g, mul(add(absf(s), absf(k1)), kBound5))) return false;
-    out = f;
-    return true;
+    return decided(s, add(e, k2), out);
+}
+
+// The weight derivative below without spike terms.
+SG_FF bool weight_decay(float x, float& out) {
+    constexpr double A = 0.000001, T = 0.0001;
+    constexpr float A1 = (float)A, A2 = (float)(A - (double)A1);
+    constexpr float T1 = (float)T, T2 = (float)(T - (double)T1);
+    float s, e, r, re;
+    two_sum(x, -A1, s, e);                               // x - A ~ s + (e - A2)
+    const float c = mul(s, T1);                          // (x - A) T ~ c + lo
+    const float lo = add(fma(s, T1, -c), fma(s, T2, mul(sub(e, A2), T1)));
+    two_sum(x, -c, r, re);
+    return decided(r, sub(re, lo), out);
+}
+
+// short_term_w below without a spike.
+template <bool SUB>
+SG_FF bool short_term_w_rest(float sw, float& out) {
+    constexpr double U = SUB ? 0.2 : 0.5;
+    constexpr int F = SUB ? 20 : 1000;
+    constexpr float U1 = (float)U, U2 = (float)(U - (double)U1), RF = (float)(1.0 / F);
+    float d, e, r, re;
+    two_sum(U1, -sw, d, e);                              // U - sw ~ d + (e + U2)
+    const float q = mul(d, RF);                          // (U - sw) / F ~ q + q2
+    const float q2 = mul(add(fma(-q, (float)F, d), add(e, U2)), RF);
+    two_sum(sw, q, r, re);
+    return decided(r, add(re, q2), out);
 }
 
 // Weight derivative of the STDP updater: (float)(x - c) with

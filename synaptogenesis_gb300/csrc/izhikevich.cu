@@ -126,7 +126,7 @@ __device__ __forceinline__ void iz_learn_apply(size_t wi, const LearnVals& v, in
         else if (v.presyn == 0.0f || (__float_as_uint(v.presyn) & 0x7FFFFFFFu) == 7u)
             src_trace = v.presyn;        // no spike yet, or where a silent trace ends: 0.933 leaves
                                          // 7 units of 2^-149 as they are
-        else if (!ff::product(v.presyn, C1, C2, src_trace, true)) src_trace = presyn_decay_exact(v.presyn);
+        else if (!ff::decay(v.presyn, C1, C2, src_trace)) src_trace = presyn_decay_exact(v.presyn);
         presyn[wi] = src_trace;
         dest_trace = dest_exc_trace;
     } else {
@@ -137,7 +137,8 @@ __device__ __forceinline__ void iz_learn_apply(size_t wi, const LearnVals& v, in
     const float p = dest_spike * src_trace;
     const bool has_p = dest_spike != 0.0f;
     float weight_delta;
-    if (!ff::weight_derivative(v.wd, p, has_p, dest_trace, src_spike, weight_delta))
+    if (has_p || src_spike ? !ff::weight_derivative(v.wd, p, has_p, dest_trace, src_spike, weight_delta)
+                           : !ff::weight_decay(v.wd, weight_delta))
         weight_delta = wd_double(v.wd, p, has_p, dest_trace, src_spike);
     wd[wi] = weight_delta;
     weight += lr * weight_delta;
@@ -152,7 +153,9 @@ __device__ __forceinline__ void iz_learn_apply(size_t wi, const LearnVals& v, in
         if (src_spike || !(U == (double)(float)U && sw == (float)U)) {
             // stp_w += (U - sw) / F + U * (1 - sw) * src_spike
             float nsw;
-            if (!ff::short_term_w<SUB>(sw, src_spike, nsw)) nsw = sw_double<SUB>(sw, src_spike);
+            if (src_spike ? !ff::short_term_w<SUB>(sw, true, nsw)
+                          : !ff::short_term_w_rest<SUB>(sw, nsw))
+                nsw = sw_double<SUB>(sw, src_spike);
             stp_w[wi] = nsw;
         }
     }
@@ -546,7 +549,7 @@ __global__ void k_iz_delay_summary(int n_src, const int* __restrict__ counts,
 static __device__ __forceinline__ float decay_95(float trace) {
     constexpr float D1 = (float)0.95, D2 = (float)(0.95 - (double)D1);
     float out = trace;
-    if (trace != 0.0f && !ff::product(trace, D1, D2, out, true)) out = mul_fd_rn(trace, 0.95);
+    if (trace != 0.0f && !ff::decay(trace, D1, D2, out)) out = mul_fd_rn(trace, 0.95);
     return out;
 }
 
@@ -1461,13 +1464,14 @@ static __device__ __noinline__ float spnet_dw_full(float dw0, float f1, float f2
 // Sparse connections: a thread takes kSpnetRanks compacted synapses of one
 // destination (blockIdx.y is their ranks' group, x the destination), since each
 // synapse's update is independent.  The double expressions are float-float
-// evaluations with a rounding test (ff_exact.cuh), falling back to integer helpers
-// and double sums where it rejects, which a warp pays for if one of its 32 synapses
-// does: products with 0.9 and 0.95 that land on a midpoint (one in 10 or 20), zero
-// and silent traces and derivatives, and sums with spike terms are therefore decided
-// on the fast path.  Memory latency bounds it, two loads deep: 28 bytes a synapse and
-// its source's spike.  7.3 M synapses of a network that has run a while: 70 us (102
-// with those expressions on the slow path, 78 with a synapse a thread).
+// evaluations (ff_exact.cuh), falling back to integer helpers and double sums where
+// a rounding test rejects, which a warp pays for if one of its 32 synapses does:
+// products with 0.9 and 0.95, zero and silent traces and derivatives, and sums with
+// spike terms are therefore decided on the fast path, the products and the sum with
+// 0.01 without the general test.  Memory bounds it, two loads deep: 28 bytes a
+// synapse and its source's spike, 4.8 TB/s with the GPU to itself.  7.3 M synapses of
+// a network that has run a while, next to an activation: 50 us (102 with those
+// expressions on the slow path, 78 with a synapse a thread, 70 with the general test).
 // Bit-identical to k_spnet_learn.
 constexpr int kSpnetRanks = 4;
 constexpr int kSpnetLearnThreads = 128;
@@ -1528,7 +1532,7 @@ __global__ void __launch_bounds__(kSpnetLearnThreads) k_spnet_learn_sparse(DGeom
             } else if (p == 0.0f || (__float_as_uint(p) & 0x7FFFFFFFu) == 10u) {
                 np = p;
             } else {
-                if (!ff::product(p, D1, D2, np, true)) np = mul_fd_rn(p, 0.95);
+                if (!ff::decay(p, D1, D2, np)) np = mul_fd_rn(p, 0.95);
                 presyn[wi] = np;
             }
             src_trace = np;
@@ -1549,7 +1553,7 @@ __global__ void __launch_bounds__(kSpnetLearnThreads) k_spnet_learn_sparse(DGeom
         if (dw0 == 0.0f) {
             dw = dw0 + f1 - f2;
         } else if (f1 == 0.0f && f2 == 0.0f) {
-            if ((__float_as_uint(dw0) & 0x7FFFFFFFu) != 4u && !ff::product(dw0, N1, N2, dw, true))
+            if ((__float_as_uint(dw0) & 0x7FFFFFFFu) != 4u && !ff::decay(dw0, N1, N2, dw))
                 dw = mul_fd_rn(dw0, 0.9);
         } else if (!ff::spnet_dw(dw0, f1, f2, dw)) {
             dw = spnet_dw_full(dw0, f1, f2);

@@ -91,6 +91,46 @@ extern "C" unsigned long long check_decimal(double c, unsigned begin, unsigned e
     return bad;
 }
 
+// Single-argument expressions over every `step`-th float: 0-2 decays by 0.9, 0.95
+// and 0.933, 3-4 sums with 0.01 and 0.1, 5 the weight derivative without spikes, 6-7
+// the short-term "w" of "add" and "sub" without one.
+extern "C" unsigned long long check_single(int which, unsigned long long begin, unsigned long long step,
+                                           unsigned long long* accepted) {
+    unsigned long long bad = 0, ok = 0;
+#pragma omp parallel for reduction(+ : bad, ok)
+    for (long long i = (long long)begin; i < (1ll << 32); i += (long long)step) {
+        const uint32_t u = (uint32_t)i;
+        float x, got = 0.0f, want;
+        std::memcpy(&x, &u, 4);
+        const double d = x;
+        bool took;
+        if (which < 3) {
+            const double c = which == 0 ? 0.9 : (which == 1 ? 0.95 : 0.933);
+            const float c1 = (float)c;
+            took = sg::ff::decay(x, c1, (float)(c - (double)c1), got);
+            want = (float)(d * c);
+        } else if (which < 5) {
+            const double k = which == 3 ? 0.01 : 0.1;
+            const float k1 = (float)k;
+            took = sg::ff::add_const(x, k1, (float)(k - (double)k1), got);
+            want = (float)(d + k);
+        } else if (which == 5) {
+            took = sg::ff::weight_decay(x, got);
+            want = (float)(d - ((d - 0.000001) * 0.0001));
+        } else if (which == 6) {
+            took = sg::ff::short_term_w_rest<false>(x, got);
+            want = (float)(d + (0.5 - d) / 1000);
+        } else {
+            took = sg::ff::short_term_w_rest<true>(x, got);
+            want = (float)(d + (0.2 - d) / 20);
+        }
+        ok += took;
+        bad += took && bits(got) != bits(want);
+    }
+    *accepted = ok;
+    return bad;
+}
+
 // Mismatches; *accepted counts the draws the rounding test took.
 extern "C" unsigned long long check_spnet(int which, int lo, int hi, unsigned long long seed,
                                           unsigned long long n, unsigned long long* accepted) {

@@ -13,12 +13,12 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 @pytest.fixture(scope="module")
 def lib(tmp_path_factory):
     out = str(tmp_path_factory.mktemp("spnetff") / "libspnetff.so")
-    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-shared", "-fPIC", "-I",
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-fopenmp", "-shared", "-fPIC", "-I",
                     os.path.join(ROOT, "synaptogenesis_gb300", "csrc"),
                     os.path.join(ROOT, "tests", "cpu_checks", "spnet_ff_check.cpp"), "-o", out],
                    check=True)
     lib = ctypes.CDLL(out)
-    for f in (lib.check_spnet, lib.check_near, lib.check_decimal):
+    for f in (lib.check_spnet, lib.check_near, lib.check_decimal, lib.check_single):
         f.restype = ctypes.c_ulonglong
     return lib
 
@@ -73,3 +73,15 @@ def test_derivative_of_subnormal_size_is_gone_in_the_sum():
     import numpy as np
     for dw in (2.0**-60, -2.0**-60, 2.0**-149):
         assert np.float32(np.float64(np.float32(dw)) + 0.01) == np.float32(0.01)
+
+
+# every 61st float here (a minute and more on a few cores for every one, which is
+# what the expressions rest on: SG_EVERY_FLOAT=1)
+@pytest.mark.parametrize("which", range(8))
+def test_single_argument_expressions(lib, which):
+    step = 1 if os.environ.get("SG_EVERY_FLOAT") else 61
+    accepted = ctypes.c_ulonglong()
+    assert lib.check_single(which, ctypes.c_ulonglong(which if step > 1 else 0),
+                            ctypes.c_ulonglong(step), ctypes.byref(accepted)) == 0
+    # what is rejected: non-finite and huge operands
+    assert accepted.value > 0.7 * (1 << 32) / step
