@@ -386,74 +386,122 @@ struct IzColsPlan {
 };
 
 // Source rows up to which a band's pre-decay traces fit in shared memory
-// (2 x rows x 8 floats) and the one-pass kernel beats the TMA pipeline.
+// (2 x 8 columns) and the one-pass kernel beats the TMA pipeline.
 constexpr int kSmallRows = 1536;
 
 // One-pass activator for matrices of at most kSmallRows source rows: one CTA
-// per band of 8 destinations reads the band's synapses with plain coalesced
-// loads (every synapse of the band in flight across the CTA), writes the
-// decayed traces back and the pre-decay traces to shared memory, then 8 (16
-// for two traces) threads add each destination's terms in source order.  The
-// float operations are the pipelined kernel's, in the same order.
+// per band of 8 destinations.  16 warps read the band's synapses with plain
+// coalesced loads, two chunks of 256 rows in flight, write the decayed traces back
+// and the pre-decay traces to shared memory; a 17th adds each destination's terms
+// (8 lanes a trace) in source order, a chunk behind them, a named barrier a chunk.
+// What bounds it is that chain, 4 cycles a row, after the first chunk's latency: with
+// the sum after all rows and a load from shared memory a term, 1024 x 1024 synapses
+// with two traces took 9.7 us; columns of 16-byte words with the next 16 rows' loads
+// in flight beside the chunks to come 6.7 us.  The float operations are the
+// pipelined kernel's, in the same order.
+constexpr int kSmallProducers = 512, kSmallChunk = 256, kSmallPer = kSmallChunk * kBand / kSmallProducers;
+static_assert((kSmallRows + kSmallChunk - 1) / kSmallChunk < 16, "a named barrier for each chunk");
+
+// Pitch of a destination's column: 16-byte words of 8 columns on different banks,
+// and of a warp's 4 rows x 8 columns.
+static SG_HOST_DEVICE int small_pitch(int nrows) { return (nrows + 31) / 32 * 32 + 4; }
+
 template <int SR, bool LONG, bool SUBSET, bool EFF>
-__global__ void __launch_bounds__(512) k_iz_cols_small(const ColsParams p, const float* __restrict__ w,
-                                                       const float* __restrict__ stp_r,
-                                                       const float* __restrict__ stp_w,
-                                                       const uint8_t* __restrict__ d8, size_t pitch) {
-    extern __shared__ float pre[];                         // [2][nrows * 8]
-    constexpr int U = 8;                                   // synapses a thread has in flight
-    const int band = blockIdx.x, n = p.nrows * kBand;
-    const size_t base = (size_t)band * n;
-    for (int e0 = threadIdx.x; e0 < n; e0 += U * blockDim.x) {
-        uint32_t word[U];
-        int delay[U];
-        float weight[U], st[U], lt[U];
+__global__ void __launch_bounds__(kSmallProducers + 32) k_iz_cols_small(
+    const ColsParams p, const float* __restrict__ w, const float* __restrict__ stp_r,
+    const float* __restrict__ stp_w, const uint8_t* __restrict__ d8, size_t pitch) {
+    extern __shared__ __align__(16) float pre[];           // [trace][8][small_pitch]
+    const int band = blockIdx.x, tid = threadIdx.x, nrows = p.nrows;
+    const int cpitch = small_pitch(nrows), nchunks = (nrows + kSmallChunk - 1) / kSmallChunk;
+    if (tid < kSmallProducers) {
+        const int r_in = tid / kBand;                      // + 64 u: the rows of a chunk
+        const size_t base = (size_t)band * nrows * kBand;
+        float* to = pre + (tid % kBand) * cpitch;
+        struct Regs {
+            uint32_t word[kSmallPer];
+            int delay[kSmallPer];
+            float weight[kSmallPer], st[kSmallPer], lt[kSmallPer];
+        } v[2];
+        auto load = [&](int ch, Regs& x) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int e = min(e0 + u * (int)blockDim.x, n - 1);
-            const size_t i = base + e;
-            word[u] = __ldg(p.src + source_of_row<SUBSET>(p.g, e >> 3));
-            delay[u] = SR == S_BIT ? (int)__ldg(d8 + (size_t)band * pitch + e) : 0;
-            weight[u] = EFF ? __ldg(w + i) : __ldg(w + i) * (__ldg(stp_r + i) * __ldg(stp_w + i));
-            st[u] = __ldcs(p.short_tr + i);
-            lt[u] = LONG ? __ldcs(p.long_tr + i) : 0.0f;
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int e = e0 + u * (int)blockDim.x;
-            if (e >= n) break;
-            const size_t i = base + e;
-            const float add = (extract<SR>(word[u], delay[u]) * weight[u]) * p.gcond;
-            const float sv = st[u] + add;
-            pre[e] = sv;
-            __stcs(p.short_tr + i, sv * p.short_tau);
-            if (LONG) {
-                const float lv = lt[u] + add;
-                pre[n + e] = lv;
-                __stcs(p.long_tr + i, lv * p.long_tau);
+            for (int u = 0; u < kSmallPer; ++u) {
+                const int row = ch * kSmallChunk + r_in + u * (kSmallProducers / kBand);
+                if (row >= nrows) continue;
+                const int e = row * kBand + tid % kBand;
+                const size_t i = base + e;
+                x.word[u] = __ldg(p.src + source_of_row<SUBSET>(p.g, row));
+                x.delay[u] = SR == S_BIT ? (int)__ldg(d8 + (size_t)band * pitch + e) : 0;
+                x.weight[u] = EFF ? __ldg(w + i) : __ldg(w + i) * (__ldg(stp_r + i) * __ldg(stp_w + i));
+                x.st[u] = __ldcs(p.short_tr + i);
+                x.lt[u] = LONG ? __ldcs(p.long_tr + i) : 0.0f;
             }
+        };
+        auto store = [&](int ch, const Regs& x) {
+#pragma unroll
+            for (int u = 0; u < kSmallPer; ++u) {
+                const int row = ch * kSmallChunk + r_in + u * (kSmallProducers / kBand);
+                if (row >= nrows) {                        // up to the summed groups of 16 rows
+                    if (row < cpitch) {
+                        to[row] = 0.0f;
+                        if (LONG) to[kBand * cpitch + row] = 0.0f;
+                    }
+                    continue;
+                }
+                const size_t i = base + row * kBand + tid % kBand;
+                const float add = (extract<SR>(x.word[u], x.delay[u]) * x.weight[u]) * p.gcond;
+                const float sv = x.st[u] + add;
+                to[row] = sv;
+                __stcs(p.short_tr + i, sv * p.short_tau);
+                if (LONG) {
+                    const float lv = x.lt[u] + add;
+                    to[kBand * cpitch + row] = lv;
+                    __stcs(p.long_tr + i, lv * p.long_tau);
+                }
+            }
+            asm volatile("bar.arrive %0, %1;" ::"r"(1 + ch), "n"(kSmallProducers + 32) : "memory");
+        };
+        load(0, v[0]);
+        load(1, v[1]);
+        for (int ch = 0; ch < nchunks; ch += 2) {
+            store(ch, v[0]);
+            if (ch + 1 >= nchunks) break;
+            load(ch + 2, v[0]);
+            store(ch + 1, v[1]);
+            load(ch + 3, v[1]);
+        }
+        return;
+    }
+    const int kind = (tid >> 3) & 1, lane = tid & 7;       // 16 lanes have a column, the others read one
+    const int c = band * kBand + lane;
+    const bool mine = tid < kSmallProducers + (LONG ? 16 : 8) && c < p.ncols;
+    float* cond = kind == 0 ? p.short_cond : p.long_cond;
+    const int to = mine ? dest_of<SUBSET ? T_SUBSET : T_FC>(p.g, c) : 0;
+    const float before = mine ? cond[to] : 0.0f;
+    const float* col = pre + (LONG ? kind * kBand + lane : lane) * cpitch;
+    float acc = 0.0f;
+    for (int ch = 0; ch < nchunks; ++ch) {
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + ch), "n"(kSmallProducers + 32) : "memory");
+        const float4* t = reinterpret_cast<const float4*>(col + ch * kSmallChunk);
+        const int groups = (min(kSmallChunk, nrows - ch * kSmallChunk) + 15) / 16;
+        float4 a[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) a[q] = t[q];
+        for (int i = 1; i <= groups; ++i) {
+            float4 b[4];                                   // the next 16 while these are added
+#pragma unroll
+            for (int q = 0; q < 4; ++q) b[q] = t[(i < groups ? 4 * i : 0) + q];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                acc += a[q].x;
+                acc += a[q].y;
+                acc += a[q].z;
+                acc += a[q].w;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) a[q] = b[q];
         }
     }
-    __syncthreads();
-    const int kind = threadIdx.x >> 3, lane = threadIdx.x & 7;
-    if (threadIdx.x >= 16 || (kind == 1 && !LONG)) return;
-    const float* col = pre + kind * n + lane;
-    float acc = 0.0f;
-    int r = 0;
-    for (; r + 8 <= p.nrows; r += 8) {
-        float v[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = col[(r + j) * kBand];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc += v[j];
-    }
-    for (; r < p.nrows; ++r) acc += col[r * kBand];
-    const int c = band * kBand + lane;
-    if (c < p.ncols) {
-        const int to = dest_of<SUBSET ? T_SUBSET : T_FC>(p.g, c);
-        if (kind == 0) p.short_cond[to] += acc;
-        else p.long_cond[to] += acc;
-    }
+    if (mine) cond[to] = before + acc;
 }
 
 // w * (R * w_stp), the activator's weight of a synapse, over the whole banded
@@ -570,7 +618,7 @@ std::shared_ptr<IzColsPlan> make_iz_cols_plan(int nrows, int ncols, const float*
 template <int SR, bool LONG, bool SUBSET, bool EFF>
 static void launch_t(const IzColsPlan& plan, const ColsParams& p, cudaStream_t s) {
     if (plan.small) {
-        const size_t bytes = (size_t)2 * p.nrows * kBand * sizeof(float);
+        const size_t bytes = (size_t)(LONG ? 2 : 1) * kBand * small_pitch(p.nrows) * sizeof(float);
         static size_t small_configured = 0;
         if (bytes > 48 * 1024 && small_configured < bytes) {
             SG_CUDA(cudaFuncSetAttribute(k_iz_cols_small<SR, LONG, SUBSET, EFF>,
@@ -578,7 +626,7 @@ static void launch_t(const IzColsPlan& plan, const ColsParams& p, cudaStream_t s
             small_configured = bytes;
         }
         const int bands = (p.ncols + kBand - 1) / kBand;
-        k_iz_cols_small<SR, LONG, SUBSET, EFF><<<bands, 512, bytes, s>>>(
+        k_iz_cols_small<SR, LONG, SUBSET, EFF><<<bands, kSmallProducers + 32, bytes, s>>>(
             p, plan.w, plan.stp_r, plan.stp_w, plan.delays, iz_delay_bytes_pitch(p.nrows));
         SG_LAUNCH_CHECK();
         return;

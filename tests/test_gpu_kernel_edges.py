@@ -382,3 +382,27 @@ def test_spnet_source_windows(sg, source, rows, cols, field, wrap):
 
     problems = compare(run_library(case(delays), sg), run_oracle(case(compact)))
     assert not problems, problems[:3]
+
+
+# chunks of 256 source rows, sums of 16, columns padded to 32; the last width of the
+# kernel; every output type (its fused weight with learning off)
+@pytest.mark.parametrize("sources,dests", [(1, 1), (15, 9), (255, 8), (256, 7), (257, 17), (512, 3),
+                                           (800, 8), (1536, 9)])
+@pytest.mark.parametrize("model,opcode,learning", [("izhikevich", "add", True), ("izhikevich", "sub", False),
+                                                   ("relay", "add", False), ("game_of_life", "mult", False)])
+def test_one_pass_trace_activator(sg, sources, dests, model, opcode, learning):
+    rng = np.random.default_rng(sources + dests)
+    n = sources * dests
+    net = network([layer("a", model, 1, sources, **({"params": "regular"} if model == "izhikevich" else {})),
+                   layer("b", "izhikevich", 1, dests, params="fast")],
+                  [connection("c", "a", "b", "fully connected", opcode=opcode, plastic=learning,
+                              **({"learning rate": 0.1} if learning else {}))])
+    draw = lambda lo, hi, m: rng.uniform(lo, hi, m).astype(np.float32)    # noqa: E731
+    bits = rng.integers(0, 2**32, sources, dtype=np.uint64).astype(np.uint32)
+    output = {"izhikevich": bits, "relay": draw(-2, 2, sources).view(np.uint32), "game_of_life": bits % 5}[model]
+    inject = {("a", "output"): output, ("matrix", "c", "weights"): draw(0, 0.5, n),
+              ("matrix", "c", "delays"): rng.integers(0, 32, n).astype(np.int32),
+              ("matrix", "c", "short term R"): draw(0.5, 1, n),
+              ("matrix", "c", "short term w"): draw(0.2, 0.8, n)}
+    keys = [("matrix", "c", "short trace"), ("b", "voltage"), ("b", "input")]
+    assert_equal(run_both(sg, net, inject, 4, keys, learning=learning))
