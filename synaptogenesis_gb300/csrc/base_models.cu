@@ -6,6 +6,7 @@
 #include "gol_step.cuh"
 #include "cuda_check.h"
 #include "history.cuh"
+#include "launch.cuh"
 #include "models.h"
 #include "state.h"
 
@@ -46,6 +47,7 @@ __global__ void __launch_bounds__(256) k_activate_base(DGeom g, const uint32_t* 
                                                        int delay, int opcode,
                                                        const float* __restrict__ w,
                                                        float* __restrict__ inputs) {
+    wait_for_previous();
     int d = blockIdx.x * blockDim.x + threadIdx.x;
     if (d >= g.n_dest) return;
     float sum = 0.0f;
@@ -89,6 +91,7 @@ template <int SR, bool SUBSET>
 __global__ void __launch_bounds__(kColsProducers + 32) k_activate_cols(
     DGeom g, int nrows, const uint32_t* __restrict__ src, int delay, int opcode,
     const float* __restrict__ w, float* __restrict__ inputs) {
+    wait_for_previous();
     __shared__ __align__(16) float prod[2][kBand * kColsPitch];
     const int tid = threadIdx.x, band = blockIdx.x;
     const int nchunks = (nrows + kColsRows - 1) / kColsRows;
@@ -181,10 +184,10 @@ void launch_base_activator(State& st, ConnState& cs, float* inputs, cudaStream_t
         const unsigned bands = blocks_for(cs.geom.n_dest, kBand);
 #define SG_COLS(SRV)                                                                        \
     if (subset)                                                                              \
-        k_activate_cols<SRV, true><<<bands, kColsProducers + 32, 0, s>>>(cs.geom, nrows, src,   \
+        launch_dependent(k_activate_cols<SRV, true>, bands, kColsProducers + 32, 0, s, cs.geom, nrows, src,   \
                                                                          c.delay, op, w, inputs); \
     else                                                                                     \
-        k_activate_cols<SRV, false><<<bands, kColsProducers + 32, 0, s>>>(cs.geom, nrows, src,  \
+        launch_dependent(k_activate_cols<SRV, false>, bands, kColsProducers + 32, 0, s, cs.geom, nrows, src,  \
                                                                           c.delay, op, w, inputs)
         switch ((int)c.from->output_type) {
             case S_FLOAT: SG_COLS(S_FLOAT); break;
@@ -196,7 +199,7 @@ void launch_base_activator(State& st, ConnState& cs, float* inputs, cudaStream_t
         return;
     }
     SG_DISPATCH_TYPE_SRC((int)c.type, (int)c.from->output_type,
-        (k_activate_base<TY, SR><<<blocks, threads, 0, s>>>(cs.geom, src, c.delay, (int)c.opcode,
+        (launch_dependent(k_activate_base<TY, SR>, blocks, threads, 0, s, cs.geom, src, c.delay, (int)c.opcode,
                                                            w, inputs)));
     SG_LAUNCH_CHECK();
 }
@@ -283,6 +286,7 @@ void launch_dendrite_fold(int n, float* src, float* dst, int opcode, float trail
 
 // relay_attributes.cpp:10-18 (the ramp is std::fmax on doubles, i.e. fmax)
 __global__ void k_relay(int size, int history, const float* __restrict__ in, float* out, int ramp) {
+    wait_for_previous();
     int nid = blockIdx.x * blockDim.x + threadIdx.x;
     if (nid >= size) return;
     float input = in[nid];
@@ -291,6 +295,7 @@ __global__ void k_relay(int size, int history, const float* __restrict__ in, flo
 
 // rate_encoding_attributes.cpp:122-131 (tanh of a float is tanhf)
 __global__ void k_rate(int size, int history, const float* __restrict__ in, float* out) {
+    wait_for_previous();
     int nid = blockIdx.x * blockDim.x + threadIdx.x;
     if (nid >= size) return;
     float input = in[nid];
@@ -1075,7 +1080,7 @@ class RelayModel : public Model {
     }
     void update(State&, LayerState& ls, const StepCtx& ctx) const override {
         const Layer& l = *ls.layer;
-        k_relay<<<blocks_for(l.size, 256), 256, 0, ctx.stream>>>(
+        launch_dependent(k_relay, blocks_for(l.size, 256), 256, 0, ctx.stream,
             l.size, l.history(), ls.input->df(), ls.output->df(), (int)ls.params.at("ramp"));
         SG_LAUNCH_CHECK();
         ctx.count();
@@ -1089,7 +1094,7 @@ class RateEncodingModel : public Model {
     OutputType output_type() const override { return OUT_FLOAT; }
     void update(State&, LayerState& ls, const StepCtx& ctx) const override {
         const Layer& l = *ls.layer;
-        k_rate<<<blocks_for(l.size, 256), 256, 0, ctx.stream>>>(l.size, l.history(), ls.input->df(),
+        launch_dependent(k_rate, blocks_for(l.size, 256), 256, 0, ctx.stream, l.size, l.history(), ls.input->df(),
                                                                 ls.output->df());
         SG_LAUNCH_CHECK();
         ctx.count();

@@ -6,6 +6,7 @@
 #include <cstring>
 
 #include "cuda_check.h"
+#include "launch.cuh"
 #include "models.h"
 #include "weight_init.h"
 
@@ -75,6 +76,7 @@ struct InputGroup {
 // it, so one launch per step keeps graphs valid.  The count is taken while the noise is
 // drawn: 3.0 -> 2.1 us for 784 neurons (with a fence and the count at the end).
 __global__ void __launch_bounds__(256) k_init_inputs(InputGroup G) {
+    wait_for_previous();
     __shared__ unsigned long long step;
     int c = 0;
     while (c + 1 < G.n && (int)blockIdx.x >= G.start[c + 1]) ++c;
@@ -328,7 +330,7 @@ void Engine::enqueue_step(bool last) {
     auto flush = [&] {
         if (group.n == 0) return;
         timed("init", 1, [&] {
-            k_init_inputs<<<group.start[group.n], 256, 0, stream_>>>(group);
+            launch_dependent(k_init_inputs, group.start[group.n], 256, 0, stream_, group);
             SG_LAUNCH_CHECK();
         });
         ++launches_;

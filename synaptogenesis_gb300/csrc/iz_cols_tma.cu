@@ -40,6 +40,7 @@
 
 #include "cuda_check.h"
 #include "iz_cols_tma.cuh"
+#include "launch.cuh"
 
 namespace sg {
 
@@ -138,6 +139,7 @@ __device__ __forceinline__ int source_of_row(const DGeom& g, int row) {
 template <int SR, bool LONG, bool SUBSET, bool EFF>
 __global__ void __launch_bounds__(kThreads, 1)
     k_iz_cols_bulk(const __grid_constant__ ColsMaps maps, const ColsParams p) {
+    wait_for_previous();
     constexpr int HAS_D = SR == S_BIT ? 1 : 0;
     constexpr int NW = EFF ? 1 : 3;                        // weight arrays
     constexpr int NA = NW + 1 + HAS_D + (LONG ? 1 : 0);
@@ -410,6 +412,7 @@ template <int SR, bool LONG, bool SUBSET, bool EFF>
 __global__ void __launch_bounds__(kSmallProducers + 32) k_iz_cols_small(
     const ColsParams p, const float* __restrict__ w, const float* __restrict__ stp_r,
     const float* __restrict__ stp_w, const uint8_t* __restrict__ d8, size_t pitch) {
+    wait_for_previous();
     extern __shared__ __align__(16) float pre[];           // [trace][8][small_pitch]
     const int band = blockIdx.x, tid = threadIdx.x, nrows = p.nrows;
     const int cpitch = small_pitch(nrows), nchunks = (nrows + kSmallChunk - 1) / kSmallChunk;
@@ -626,7 +629,7 @@ static void launch_t(const IzColsPlan& plan, const ColsParams& p, cudaStream_t s
             small_configured = bytes;
         }
         const int bands = (p.ncols + kBand - 1) / kBand;
-        k_iz_cols_small<SR, LONG, SUBSET, EFF><<<bands, kSmallProducers + 32, bytes, s>>>(
+        launch_dependent(k_iz_cols_small<SR, LONG, SUBSET, EFF>, bands, kSmallProducers + 32, bytes, s,
             p, plan.w, plan.stp_r, plan.stp_w, plan.delays, iz_delay_bytes_pitch(p.nrows));
         SG_LAUNCH_CHECK();
         return;
@@ -637,7 +640,7 @@ static void launch_t(const IzColsPlan& plan, const ColsParams& p, cudaStream_t s
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
         configured = (int)plan.smem;
     }
-    k_iz_cols_bulk<SR, LONG, SUBSET, EFF><<<plan.n_cta, kThreads, plan.smem, s>>>(plan.maps, p);
+    launch_dependent(k_iz_cols_bulk<SR, LONG, SUBSET, EFF>, plan.n_cta, kThreads, plan.smem, s, plan.maps, p);
     SG_LAUNCH_CHECK();
 }
 

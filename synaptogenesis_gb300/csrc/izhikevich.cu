@@ -17,6 +17,7 @@
 #include "history.cuh"
 #include "iz_cols_tma.cuh"
 #include "iz_neuron.cuh"
+#include "launch.cuh"
 #include "models.h"
 #include "state.h"
 #include "weight_init.h"
@@ -188,6 +189,7 @@ __global__ void __launch_bounds__(128) k_iz_activate(
     const float* __restrict__ stp_r, const float* __restrict__ stp_w, const int* __restrict__ delays,
     float* __restrict__ short_tr, float* __restrict__ long_tr, float gcond, float short_tau,
     float long_tau, float* short_cond, float* long_cond) {
+    wait_for_previous();
     int d0 = blockIdx.x * blockDim.x + threadIdx.x;
     int d1 = d0 + 1;
     if (serial) { if (d0 != 0) return; d1 = g.n_dest; }
@@ -274,6 +276,7 @@ __global__ void __launch_bounds__(256, 4) k_iz_activate_conv_tile(
     const float* __restrict__ stp_r, const float* __restrict__ stp_w, const uint8_t* __restrict__ delays,
     float* __restrict__ short_tr, float* __restrict__ long_tr, float gcond, float short_tau,
     float long_tau, float* __restrict__ short_cond, float* __restrict__ long_cond) {
+    wait_for_previous();
     __shared__ float s_st[kConvMaxK][32];
     __shared__ float s_lt[LONG ? kConvMaxK : 1][32];
     __shared__ int2 koff[kConvMaxK];
@@ -355,6 +358,7 @@ __global__ void __launch_bounds__(256, 4) k_iz_learn_conv_tile(
     const int* __restrict__ to_tss, const int* __restrict__ from_tss, float lr, int stp_flag,
     float max_weight, float* __restrict__ w, float* __restrict__ presyn, float* __restrict__ wd,
     float* __restrict__ stp_r, float* __restrict__ stp_w, IzLut lut) {
+    wait_for_previous();
     __shared__ int2 koff[kConvMaxK];
     conv_offsets(g, K, koff);
     __syncthreads();
@@ -493,6 +497,7 @@ __global__ void k_iz_time_since_spike(int n_src, const int* __restrict__ counts,
                                       const ulonglong2* __restrict__ summary,
                                       const uint32_t* __restrict__ src, int src_type,
                                       int* __restrict__ tss) {
+    wait_for_previous();
     int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= n_src) return;
     tss_update(f, counts, last, delays, summary, src, src_type, tss);
@@ -515,6 +520,7 @@ struct TssGroup {
 };
 
 __global__ void k_iz_time_since_spike_group(TssGroup G) {
+    wait_for_previous();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= G.start[G.n]) return;
     int c = 0;
@@ -581,6 +587,7 @@ static int update_threads(int neurons) {
 }
 
 __global__ void __launch_bounds__(256) k_iz_update(IzUpdateGroup G) {
+    wait_for_previous();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= G.start[G.n]) return;
     int l = 0;
@@ -653,6 +660,7 @@ __global__ void __launch_bounds__(256, 4) k_iz_learn_2d(
     const int* __restrict__ from_tss, float lr, int stp_flag, float max_weight,
     float* __restrict__ w, float* __restrict__ presyn, float* __restrict__ wd,
     float* __restrict__ stp_r, float* __restrict__ stp_w, IzLut lut) {
+    wait_for_previous();
     const int col = blockIdx.x * kBand + threadIdx.x % kBand;
     if (col >= ncols) return;
     const int row0 = blockIdx.y * (32 * kLearnBatch) + threadIdx.x / kBand;
@@ -813,7 +821,7 @@ static bool tss_group(State& st, const std::vector<ConnState*>& todo, const Step
             cs.prologue_done = true;
         }
         G.start[G.n] = total;
-        k_iz_time_since_spike_group<<<blocks_for(total, 256), 256, 0, ctx.stream>>>(G);
+        launch_dependent(k_iz_time_since_spike_group, blocks_for(total, 256), 256, 0, ctx.stream, G);
         SG_LAUNCH_CHECK();
         ctx.count();
     }
@@ -976,7 +984,7 @@ class IzhikevichModel : public Model {
         if (cs.prologue_done) {
             cs.prologue_done = false;
         } else {
-            k_iz_time_since_spike<<<blocks_for(c.from->size, 256), 256, 0, ctx.stream>>>(
+            launch_dependent(k_iz_time_since_spike, blocks_for(c.from->size, 256), 256, 0, ctx.stream,
                 c.from->size, cs.visit_counts->di(), cs.last_visits->di(), cs.delays->di(),
                 reinterpret_cast<const ulonglong2*>(cs.delay_summary->di()), src,
                 (int)c.from->output_type, cs.var("time since spike")->di());
@@ -993,7 +1001,7 @@ class IzhikevichModel : public Model {
             unsigned nb = blocks_for(c.to->size, 32);
             int sr = (int)c.from->output_type;
 #define SG_CONV_TILE(SRV, LV)                                                                     \
-    k_iz_activate_conv_tile<SRV, LV><<<nb, 256, 0, ctx.stream>>>(                                 \
+    launch_dependent(k_iz_activate_conv_tile<SRV, LV>, nb, 256, 0, ctx.stream,                                  \
         cs.geom, K, src, cs.weights->df(), cs.var("short term R")->df(),                        \
         cs.var("short term w")->df(), reinterpret_cast<const uint8_t*>(cs.delays8->du()),        \
         cs.var("short trace")->df(),                                                            \
@@ -1034,7 +1042,7 @@ class IzhikevichModel : public Model {
         }
 #define SG_IZ_ACT(LONG)                                                                        \
     SG_DISPATCH_TYPE_SRC((int)c.type, (int)c.from->output_type,                                \
-        (k_iz_activate<TY, SR, LONG><<<blocks, threads, 0, ctx.stream>>>(                      \
+        (launch_dependent(k_iz_activate<TY, SR, LONG>, blocks, threads, 0, ctx.stream,                       \
             cs.geom, serial, src, cs.weights->df(), cs.var("short term R")->df(),              \
             cs.var("short term w")->df(), cs.delays->di(), cs.var("short trace")->df(),        \
             cs.var("long trace")->df(), g, stau, ltau, sc, lc)))
@@ -1073,7 +1081,7 @@ class IzhikevichModel : public Model {
             G.start[G.n] = total;
             if (total == 0) continue;
             const int threads = update_threads(total);
-            k_iz_update<<<blocks_for(total, threads), threads, 0, ctx.stream>>>(G);
+            launch_dependent(k_iz_update, blocks_for(total, threads), threads, 0, ctx.stream, G);
             SG_LAUNCH_CHECK();
             ctx.count();
         }
@@ -1103,7 +1111,7 @@ class IzhikevichModel : public Model {
 #define SG_CONV_LEARN(SRV, SUBV)                                                                  \
     do {                                                                                         \
         prefer_max_shared((const void*)k_iz_learn_conv_tile<SRV, SUBV>);                        \
-        k_iz_learn_conv_tile<SRV, SUBV><<<grid, 256, 0, ctx.stream>>>(                            \
+        launch_dependent(k_iz_learn_conv_tile<SRV, SUBV>, grid, 256, 0, ctx.stream,                             \
             cs.geom, K, st.dev_output(c.to, 0), to.var("post trace")->df(),                     \
             to.var("time since spike")->di(), cs.var("time since spike")->di(),                 \
             cs.params.at("learning rate"), (int)cs.params.at("stp"), c.max_weight,              \
@@ -1129,7 +1137,7 @@ class IzhikevichModel : public Model {
             dim3 grid(blocks_for(ncols, kBand), blocks_for(nrows, 32 * kLearnBatch));
             bool subset = c.type == SUBSET;
 #define SG_IZ_LEARN2D(SRV, SUBV, SSV)                                                           \
-    k_iz_learn_2d<SRV, SUBV, SSV><<<grid, 256, 0, ctx.stream>>>(                                \
+    launch_dependent(k_iz_learn_2d<SRV, SUBV, SSV>, grid, 256, 0, ctx.stream,                                 \
         cs.geom, nrows, ncols, st.dev_output(c.to, 0), to.var("post trace")->df(),             \
         to.var("time since spike")->di(), cs.var("time since spike")->di(),                    \
         cs.params.at("learning rate"), (int)cs.params.at("stp"), c.max_weight,                 \
@@ -1177,6 +1185,7 @@ __global__ void __launch_bounds__(128) k_spnet_activate(DGeom g, const uint32_t*
                                                         const float* __restrict__ w,
                                                         const int* __restrict__ delays, float gc,
                                                         int opcode, float* __restrict__ inputs) {
+    wait_for_previous();
     const int d = blockIdx.x * blockDim.x + threadIdx.x;
     if (d >= g.n_dest) return;
     float sum = 0.0f;
@@ -1240,6 +1249,7 @@ __global__ void __launch_bounds__(kWindowDests) k_spnet_activate_window(
     DGeom g, const uint32_t* __restrict__ src, int n_src, const int* __restrict__ first, int window,
     const uint32_t* __restrict__ packed, const float* __restrict__ w, float gc, int opcode,
     float* __restrict__ inputs) {
+    wait_for_previous();
     extern __shared__ uint32_t staged[];
     const unsigned d = blockIdx.x * kWindowDests + threadIdx.x;
     const int n = d < (unsigned)g.n_dest ? g.nz[d] : 0;
@@ -1375,6 +1385,7 @@ struct SpnetUpdateGroup {
 };
 
 __global__ void __launch_bounds__(256) k_spnet_update(SpnetUpdateGroup G) {
+    wait_for_previous();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= G.start[G.n]) return;
     int l = 0;
@@ -1484,6 +1495,7 @@ __global__ void __launch_bounds__(kSpnetLearnThreads) k_spnet_learn_sparse(DGeom
                                                             float max_weight, float* __restrict__ w,
                                                             float* __restrict__ presyn,
                                                             float* __restrict__ dws, IzLut lut) {
+    wait_for_previous();
     const unsigned d = blockIdx.x * blockDim.x + threadIdx.x;
     const int i0 = blockIdx.y * kSpnetRanks;
     if (d >= (unsigned)g.to_size) return;
@@ -1630,7 +1642,7 @@ class SpnetModel : public Model {
         if (cs.prologue_done) {
             cs.prologue_done = false;
         } else {
-            k_iz_time_since_spike<<<blocks_for(c.from->size, 256), 256, 0, ctx.stream>>>(
+            launch_dependent(k_iz_time_since_spike, blocks_for(c.from->size, 256), 256, 0, ctx.stream,
                 c.from->size, cs.visit_counts->di(), cs.last_visits->di(), cs.delays->di(),
                 reinterpret_cast<const ulonglong2*>(cs.delay_summary->di()), src,
                 (int)c.from->output_type, cs.var("time since spike")->di());
@@ -1643,7 +1655,7 @@ class SpnetModel : public Model {
             const size_t smem = (size_t)cs.window * 4;
             const int op = (int)c.opcode;
 #define SG_SPNET_WINDOW(SRV)                                                               \
-    k_spnet_activate_window<SRV><<<blocks, kWindowDests, smem, ctx.stream>>>(              \
+    launch_dependent(k_spnet_activate_window<SRV>, blocks, kWindowDests, smem, ctx.stream,               \
         cs.geom, src, c.from->size, cs.window_first->di(), cs.window, cs.sparse_packed->du(), \
         cs.weights->df(), cs.params.at("conductance"), op, inputs)
             switch ((int)c.from->output_type) {
@@ -1654,7 +1666,7 @@ class SpnetModel : public Model {
 #undef SG_SPNET_WINDOW
         } else {
             SG_DISPATCH_TYPE_SRC((int)c.type, (int)c.from->output_type,
-                (k_spnet_activate<TY, SR><<<blocks, 128, 0, ctx.stream>>>(
+                (launch_dependent(k_spnet_activate<TY, SR>, blocks, 128, 0, ctx.stream,
                     cs.geom, src, cs.weights->df(), cs.delays->di(), cs.params.at("conductance"),
                     (int)c.opcode, inputs)));
         }
@@ -1687,7 +1699,7 @@ class SpnetModel : public Model {
             G.start[G.n] = total;
             if (total == 0) continue;
             const int threads = update_threads(total);
-            k_spnet_update<<<blocks_for(total, threads), threads, 0, ctx.stream>>>(G);
+            launch_dependent(k_spnet_update, blocks_for(total, threads), threads, 0, ctx.stream, G);
             SG_LAUNCH_CHECK();
             ctx.count();
         }
@@ -1708,7 +1720,7 @@ class SpnetModel : public Model {
             const int kmax = std::max(1, cs.geom.kmax);
             const dim3 grid(blocks_for(c.to->size, kSpnetLearnThreads), (kmax + kSpnetRanks - 1) / kSpnetRanks);
 #define SG_SPNET_SPARSE(SRV, SUBV)                                                              \
-    k_spnet_learn_sparse<SRV, SUBV><<<grid, kSpnetLearnThreads, 0, ctx.stream>>>(                              \
+    launch_dependent(k_spnet_learn_sparse<SRV, SUBV>, grid, kSpnetLearnThreads, 0, ctx.stream,                               \
         cs.geom, st.dev_output(c.to, 0), to.var("post trace")->df(),                           \
         to.var("time since spike")->di(), cs.var("time since spike")->di(),                    \
         cs.params.at("learning rate"), c.max_weight, cs.weights->df(),                         \

@@ -56,6 +56,7 @@
 
 #include "../../include/syngen.h"
 #include "cuda_check.h"
+#include "launch.cuh"
 
 namespace sg {
 void set_last_error(const char* what);
@@ -88,14 +89,6 @@ __device__ __forceinline__ float sigmoid(float v) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
     // (an infinite d, v below -88, has a zero reciprocal and no correction)
     return d > 1.0e38f ? y : __fmaf_rn(y, __fmaf_rn(-d, y, 1.0f), y);
-}
-
-// Launches follow one another closely (programmatic dependents): a kernel waits
-// here for the one before it, which has waited for its own predecessor, so what
-// was written two launches ago or earlier may be read before the wait.
-__device__ __forceinline__ void wait_for_previous() {
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
 // wt[l][k][i] = w[l][i][k]
@@ -956,16 +949,7 @@ unsigned grid_of(long long n) { return (unsigned)((n + 255) / 256); }
 // Every launch of a pass is a programmatic dependent of the one before it.
 template <class... P, class... A>
 void launch(void (*kernel)(P...), dim3 grid, int threads, cudaStream_t st, A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    SG_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    launch_dependent(kernel, grid, dim3((unsigned)threads), 0, st, args...);
 }
 
 void transpose_weights(const Dims& D, const float* w, const Work& W, cudaStream_t st) {
