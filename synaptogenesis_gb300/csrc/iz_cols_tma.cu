@@ -412,7 +412,6 @@ template <int SR, bool LONG, bool SUBSET, bool EFF>
 __global__ void __launch_bounds__(kSmallProducers + 32) k_iz_cols_small(
     const ColsParams p, const float* __restrict__ w, const float* __restrict__ stp_r,
     const float* __restrict__ stp_w, const uint8_t* __restrict__ d8, size_t pitch) {
-    wait_for_previous();
     extern __shared__ __align__(16) float pre[];           // [trace][8][small_pitch]
     const int band = blockIdx.x, tid = threadIdx.x, nrows = p.nrows;
     const int cpitch = small_pitch(nrows), nchunks = (nrows + kSmallChunk - 1) / kSmallChunk;
@@ -421,7 +420,6 @@ __global__ void __launch_bounds__(kSmallProducers + 32) k_iz_cols_small(
         const size_t base = (size_t)band * nrows * kBand;
         float* to = pre + (tid % kBand) * cpitch;
         struct Regs {
-            uint32_t word[kSmallPer];
             int delay[kSmallPer];
             float weight[kSmallPer], st[kSmallPer], lt[kSmallPer];
         } v[2];
@@ -432,14 +430,20 @@ __global__ void __launch_bounds__(kSmallProducers + 32) k_iz_cols_small(
                 if (row >= nrows) continue;
                 const int e = row * kBand + tid % kBand;
                 const size_t i = base + e;
-                x.word[u] = __ldg(p.src + source_of_row<SUBSET>(p.g, row));
                 x.delay[u] = SR == S_BIT ? (int)__ldg(d8 + (size_t)band * pitch + e) : 0;
                 x.weight[u] = EFF ? __ldg(w + i) : __ldg(w + i) * (__ldg(stp_r + i) * __ldg(stp_w + i));
                 x.st[u] = __ldcs(p.short_tr + i);
                 x.lt[u] = LONG ? __ldcs(p.long_tr + i) : 0.0f;
             }
         };
+        const uint32_t* src = nullptr;
         auto store = [&](int ch, const Regs& x) {
+            uint32_t word[kSmallPer];
+#pragma unroll
+            for (int u = 0; u < kSmallPer; ++u) {
+                const int row = ch * kSmallChunk + r_in + u * (kSmallProducers / kBand);
+                if (row < nrows) word[u] = __ldg(src + source_of_row<SUBSET>(p.g, row));
+            }
 #pragma unroll
             for (int u = 0; u < kSmallPer; ++u) {
                 const int row = ch * kSmallChunk + r_in + u * (kSmallProducers / kBand);
@@ -451,7 +455,7 @@ __global__ void __launch_bounds__(kSmallProducers + 32) k_iz_cols_small(
                     continue;
                 }
                 const size_t i = base + row * kBand + tid % kBand;
-                const float add = (extract<SR>(x.word[u], x.delay[u]) * x.weight[u]) * p.gcond;
+                const float add = (extract<SR>(word[u], x.delay[u]) * x.weight[u]) * p.gcond;
                 const float sv = x.st[u] + add;
                 to[row] = sv;
                 __stcs(p.short_tr + i, sv * p.short_tau);
@@ -463,8 +467,12 @@ __global__ void __launch_bounds__(kSmallProducers + 32) k_iz_cols_small(
             }
             asm volatile("bar.arrive %0, %1;" ::"r"(1 + ch), "n"(kSmallProducers + 32) : "memory");
         };
+        // the synapses' variables are this kernel's and the learning one's, which the
+        // setting of the registers at least has followed: before the wait
         load(0, v[0]);
         load(1, v[1]);
+        wait_for_previous();
+        src = after_wait(p.src);
         for (int ch = 0; ch < nchunks; ch += 2) {
             store(ch, v[0]);
             if (ch + 1 >= nchunks) break;
@@ -474,6 +482,7 @@ __global__ void __launch_bounds__(kSmallProducers + 32) k_iz_cols_small(
         }
         return;
     }
+    wait_for_previous();
     const int kind = (tid >> 3) & 1, lane = tid & 7;       // 16 lanes have a column, the others read one
     const int c = band * kBand + lane;
     const bool mine = tid < kSmallProducers + (LONG ? 16 : 8) && c < p.ncols;

@@ -276,7 +276,6 @@ __global__ void __launch_bounds__(256, 4) k_iz_activate_conv_tile(
     const float* __restrict__ stp_r, const float* __restrict__ stp_w, const uint8_t* __restrict__ delays,
     float* __restrict__ short_tr, float* __restrict__ long_tr, float gcond, float short_tau,
     float long_tau, float* __restrict__ short_cond, float* __restrict__ long_cond) {
-    wait_for_previous();
     __shared__ float s_st[kConvMaxK][32];
     __shared__ float s_lt[LONG ? kConvMaxK : 1][32];
     __shared__ int2 koff[kConvMaxK];
@@ -287,19 +286,15 @@ __global__ void __launch_bounds__(256, 4) k_iz_activate_conv_tile(
     __syncthreads();
     const int2 base = conv_base(g, ok ? d : 0);
     constexpr int B = 4;                 // kernel positions whose loads are in flight together
-    for (int k0 = warp; k0 < K; k0 += 8 * B) {
-        uint32_t word[B];
-        int dl[B];
-        float wv[B], rv[B], sv[B], st0[B], lt0[B];
-        bool on[B];
+    int from[B], dl[B];
+    float wv[B], rv[B], sv[B], st0[B], lt0[B];
+    auto load = [&](int k0) {            // the synapses' own variables
 #pragma unroll
         for (int b = 0; b < B; ++b) {
             const int k = k0 + 8 * b;
-            const int from = (ok && k < K) ? conv_source_at(g, base, koff[k]) : -1;
-            on[b] = from >= 0;
-            if (on[b]) {
+            from[b] = (ok && k < K) ? conv_source_at(g, base, koff[k]) : -1;
+            if (from[b] >= 0) {
                 const size_t wi = (size_t)k * g.to_size + d;
-                word[b] = __ldg(src + from);
                 dl[b] = SR == S_BIT ? (int)__ldg(delays + wi) : 0;
                 wv[b] = __ldg(w + wi);
                 rv[b] = __ldg(stp_r + wi);
@@ -308,12 +303,22 @@ __global__ void __launch_bounds__(256, 4) k_iz_activate_conv_tile(
                 lt0[b] = LONG ? long_tr[wi] : 0.0f;
             }
         }
+    };
+    // the synapses' variables are this kernel's and the learning one's, which the
+    // setting of the registers at least has followed: before the wait
+    load(warp);
+    wait_for_previous();
+    const uint32_t* words = after_wait(src);
+    for (int k0 = warp; k0 < K;) {
+        uint32_t word[B];
+#pragma unroll
+        for (int b = 0; b < B; ++b) word[b] = from[b] >= 0 ? __ldg(words + from[b]) : 0u;
 #pragma unroll
         for (int b = 0; b < B; ++b) {
             const int k = k0 + 8 * b;
             if (k >= K) break;
             float st_pre = 0.0f, lt_pre = 0.0f;
-            if (on[b]) {
+            if (from[b] >= 0) {
                 const size_t wi = (size_t)k * g.to_size + d;
                 const float spike = extract<SR>(word[b], dl[b]);
                 const float weight = wv[b] * (rv[b] * sv[b]);
@@ -327,6 +332,8 @@ __global__ void __launch_bounds__(256, 4) k_iz_activate_conv_tile(
             s_st[k][lane] = st_pre;
             if (LONG) s_lt[k][lane] = lt_pre;
         }
+        k0 += 8 * B;
+        if (k0 < K) load(k0);
     }
     __syncthreads();
     if (!ok) return;
@@ -358,38 +365,47 @@ __global__ void __launch_bounds__(256, 4) k_iz_learn_conv_tile(
     const int* __restrict__ to_tss, const int* __restrict__ from_tss, float lr, int stp_flag,
     float max_weight, float* __restrict__ w, float* __restrict__ presyn, float* __restrict__ wd,
     float* __restrict__ stp_r, float* __restrict__ stp_w, IzLut lut) {
-    wait_for_previous();
     __shared__ int2 koff[kConvMaxK];
     conv_offsets(g, K, koff);
     __syncthreads();
     const int d = blockIdx.x * 32 + (threadIdx.x & 31);
-    if (d >= g.to_size) return;
-    const float dest_exc_trace = __ldg(to_exc + d);
-    const int dest_tss = __ldg(to_tss + d);
-    const float dest_spike = extract<SR>(__ldg(dest_out + d), 0);
-    const int2 base = conv_base(g, d);
+    const bool mine = d < g.to_size;
+    const int2 base = conv_base(g, mine ? d : 0);
     const int kstep = 8 * gridDim.y;
-    for (int k0 = (threadIdx.x >> 5) + 8 * blockIdx.y; k0 < K; k0 += kstep * kLearnBatch) {
-        LearnVals v[kLearnBatch];
-        int src_tss[kLearnBatch];
-        bool ok[kLearnBatch];
+    LearnVals v[kLearnBatch];
+    int src_tss[kLearnBatch];
+    bool ok[kLearnBatch];
+    auto load = [&](int k0) {
 #pragma unroll
         for (int b = 0; b < kLearnBatch; ++b) {
             const int k = k0 + kstep * b;
-            const int from = k < K ? conv_source_at(g, base, koff[k]) : -1;
+            const int from = mine && k < K ? conv_source_at(g, base, koff[k]) : -1;
             ok[b] = from >= 0;
             if (ok[b]) {
                 v[b] = iz_learn_load<SUB>((size_t)k * g.to_size + d, stp_flag, w, presyn, wd,
                                           stp_r, stp_w);
-                src_tss[b] = __ldg(from_tss + from);
+                src_tss[b] = from_tss[from];
             }
         }
+    };
+    // before the wait: all but the destinations' spikes, traces and times, which the
+    // neuron update just before sets
+    int k0 = (threadIdx.x >> 5) + 8 * blockIdx.y;
+    load(k0);
+    wait_for_previous();
+    if (!mine) return;
+    const float dest_exc_trace = after_wait(to_exc)[d];
+    const int dest_tss = after_wait(to_tss)[d];
+    const float dest_spike = extract<SR>(after_wait(dest_out)[d], 0);
+    while (k0 < K) {
 #pragma unroll
         for (int b = 0; b < kLearnBatch; ++b)
             if (ok[b])
                 iz_learn_apply<SUB>((size_t)(k0 + kstep * b) * g.to_size + d, v[b], src_tss[b],
                                     dest_spike, dest_exc_trace, dest_tss, lr, stp_flag, max_weight,
                                     w, presyn, wd, stp_r, stp_w, lut);
+        k0 += kstep * kLearnBatch;
+        if (k0 < K) load(k0);
     }
 }
 
@@ -587,27 +603,34 @@ static int update_threads(int neurons) {
 }
 
 __global__ void __launch_bounds__(256) k_iz_update(IzUpdateGroup G) {
-    wait_for_previous();
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= G.start[G.n]) return;
+    const int g = min(blockIdx.x * blockDim.x + threadIdx.x, G.start[G.n] - 1);
     int l = 0;
     while (l + 1 < G.n && g >= G.start[l + 1]) ++l;
     const IzLayerArgs& A = G.L[l];
     const int nid = g - G.start[l], size = A.size, history = A.history;
+    uint32_t* spikes = A.spikes;
+    // what only this kernel writes, once a step: before the wait (the registers were
+    // set since)
     float voltage = A.voltages[nid];
     float recovery = A.recoveries[nid];
+    const float a = __ldg(A.as + nid), b = __ldg(A.bs + nid);
+    const float c = __ldg(A.cs + nid), d = __ldg(A.ds + nid);
+    const float post = A.post_traces[nid];
+    const int tss = A.tss[nid];
+    uint32_t curr = spikes[(size_t)size * (history - 1) + nid];
+    wait_for_previous();
+    if (blockIdx.x * blockDim.x + threadIdx.x >= G.start[G.n]) return;
+    const float dopamine = A.dopamine[nid];
     iz_integrate_ff(voltage, recovery, A.ampa[nid], A.nmda[nid], A.gabaa[nid], A.gabab[nid],
-                    A.mult[nid], A.inputs[nid], __ldg(A.as + nid), __ldg(A.bs + nid));
+                    A.mult[nid], A.inputs[nid], a, b);
     A.ampa[nid] = 0.0f;
     A.nmda[nid] = 0.0f;
     A.gabaa[nid] = 0.0f;
     A.gabab[nid] = 0.0f;
     A.mult[nid] = 0.0f;
-    A.dopamine[nid] = decay_95(A.dopamine[nid]);                     // dopamine *= 0.95
+    A.dopamine[nid] = decay_95(dopamine);                            // dopamine *= 0.95
     const unsigned int spike = voltage >= 30.0f;                     // 30.0 is a float value
     // SHIFT_BIT_OUTPUTS (state/attributes.h:321-333)
-    uint32_t* spikes = A.spikes;
-    uint32_t curr = spikes[(size_t)size * (history - 1) + nid];
     for (int idx = history - 1; idx > 0; --idx) {
         uint32_t prev = spikes[(size_t)size * (idx - 1) + nid];
         spikes[(size_t)size * idx + nid] = (curr >> 1) | (prev << 31);
@@ -616,11 +639,11 @@ __global__ void __launch_bounds__(256) k_iz_update(IzUpdateGroup G) {
     spikes[nid] = (curr >> 1) | (spike << 31);
     const bool prev_bit = curr >> 31;
     // post_trace = prev_bit ? 0.004 : post_trace * 0.95, stored as float
-    A.post_traces[nid] = prev_bit ? (float)0.004 : decay_95(A.post_traces[nid]);
-    int t = A.tss[nid] + 1;
+    A.post_traces[nid] = prev_bit ? (float)0.004 : decay_95(post);
+    const int t = tss + 1;
     A.tss[nid] = prev_bit ? 0 : (t < 32 ? t : 32);
-    A.voltages[nid] = spike ? __ldg(A.cs + nid) : voltage;
-    A.recoveries[nid] = recovery + (spike * __ldg(A.ds + nid));
+    A.voltages[nid] = spike ? c : voltage;
+    A.recoveries[nid] = recovery + (spike * d);
 }
 
 
@@ -660,25 +683,26 @@ __global__ void __launch_bounds__(256, 4) k_iz_learn_2d(
     const int* __restrict__ from_tss, float lr, int stp_flag, float max_weight,
     float* __restrict__ w, float* __restrict__ presyn, float* __restrict__ wd,
     float* __restrict__ stp_r, float* __restrict__ stp_w, IzLut lut) {
-    wait_for_previous();
     const int col = blockIdx.x * kBand + threadIdx.x % kBand;
-    if (col >= ncols) return;
+    const bool mine = col < ncols;
     const int row0 = blockIdx.y * (32 * kLearnBatch) + threadIdx.x / kBand;
     LearnVals v[kLearnBatch];
     int src_tss[kLearnBatch];
 #pragma unroll
     for (int b = 0; b < kLearnBatch; ++b) {
         const int row = row0 + 32 * b;
-        if (row < nrows) {
+        if (mine && row < nrows) {
             v[b] = iz_learn_load<SUB>((size_t)banded_index(col, row, nrows), stp_flag, w, presyn, wd,
                                       stp_r, stp_w);
-            src_tss[b] = __ldg(from_tss + row_source<SUBSET>(g, row));
+            src_tss[b] = from_tss[row_source<SUBSET>(g, row)];
         }
     }
+    wait_for_previous();                 // (as k_iz_learn_conv_tile)
+    if (!mine) return;
     const int to = dest_of<SUBSET ? T_SUBSET : T_FC>(g, col);
-    const float dest_exc_trace = __ldg(to_exc + to);
-    const int dest_tss = __ldg(to_tss + to);
-    const float dest_spike = extract<SR>(__ldg(dest_out + to), 0);
+    const float dest_exc_trace = after_wait(to_exc)[to];
+    const int dest_tss = after_wait(to_tss)[to];
+    const float dest_spike = extract<SR>(after_wait(dest_out)[to], 0);
 #pragma unroll
     for (int b = 0; b < kLearnBatch; ++b) {
         const int row = row0 + 32 * b;
@@ -1385,17 +1409,20 @@ struct SpnetUpdateGroup {
 };
 
 __global__ void __launch_bounds__(256) k_spnet_update(SpnetUpdateGroup G) {
-    wait_for_previous();
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= G.start[G.n]) return;
+    const int g = min(blockIdx.x * blockDim.x + threadIdx.x, G.start[G.n] - 1);
     int l = 0;
     while (l + 1 < G.n && g >= G.start[l + 1]) ++l;
     const SpnetLayerArgs& A = G.L[l];
     const int nid = g - G.start[l];
+    // what only this kernel writes, once a step: before the wait (as k_iz_update)
     float voltage = A.vs[nid];
     float recovery = A.rs[nid];
+    const float a = A.as[nid], b = A.bs[nid], c = A.cs[nid], reset = A.ds[nid];
+    const float post = A.post[nid];
+    const int tss = A.tss[nid];
+    wait_for_previous();
+    if (blockIdx.x * blockDim.x + threadIdx.x >= G.start[G.n]) return;
     const float current = A.in[nid];
-    const float a = A.as[nid], b = A.bs[nid];
     for (int i = 0; (i < 10) && (voltage < 30.0f); ++i) {
         float delta_v, tail, bound, nv;
         ff::iz_delta_v_sum(voltage, recovery, current, delta_v, tail, bound);
@@ -1416,15 +1443,14 @@ __global__ void __launch_bounds__(256) k_spnet_update(SpnetUpdateGroup G) {
     }
     const uint32_t spike = voltage >= 30.0f;
     const uint32_t prev_bit = shift_bits(A.spikes, A.size, A.history, nid, spike);
-    const float post = A.post[nid];
     float np;
     constexpr float T1 = (float)0.1, T2 = (float)(0.1 - (double)T1);
     if (!prev_bit) np = decay_95(post);
     else if (!ff::add_const(post, T1, T2, np)) np = (float)(post + 0.1);
     A.post[nid] = np;
-    A.tss[nid] = prev_bit ? 0 : min(32, A.tss[nid] + 1);
-    A.vs[nid] = spike ? A.cs[nid] : voltage;
-    A.rs[nid] = recovery + (spike * A.ds[nid]);
+    A.tss[nid] = prev_bit ? 0 : min(32, tss + 1);
+    A.vs[nid] = spike ? c : voltage;
+    A.rs[nid] = recovery + (spike * reset);
 }
 
 // spnet_attributes.cpp:220-286 ("add": presynaptic trace against the

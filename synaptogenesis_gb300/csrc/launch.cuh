@@ -20,6 +20,17 @@ __device__ __forceinline__ void wait_for_previous() {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
+// p for loads after the wait that the compiler is not to move before it (read-only
+// ones, which no memory clobber holds), in kernels that load anything before it.
+// What may be loaded before it is what the kernel before does not write: the one
+// before that has completed, since the kernel before waited for it before it let
+// this one be launched.
+template <class T>
+__device__ __forceinline__ T* after_wait(T* p) {
+    asm volatile("" : "+l"(p));
+    return p;
+}
+
 template <class... P, class... A>
 void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                       A&&... args) {
