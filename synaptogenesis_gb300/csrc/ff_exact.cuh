@@ -101,20 +101,15 @@ SG_FF void two_prod(float a, float b, float& p, float& e) {
     e = fma(a, b, -p);
 }
 
-// True when every real within B of f + g rounds to f, where f = RN(f + g)
-// (so |g| is at most half an ulp of f).  f must be a normal float of
-// magnitude at least 2^-101; the nearest rounding boundaries are half an ulp
-// away from f, a quarter of f's ulp below a power of two.  The comparison
-// leaves a relative margin of 2^-20 for the rounding of |g| + B.
+// True when every real within B of f + g rounds to f, where f = RN(f + g) (so |g| is
+// at most half an ulp of f), f a float of magnitude at least 2^-101: the two ends of
+// the interval round to f, and so does what lies between.  The float sums g + B and
+// g - B err by less than 2^-48 |f|, a 32nd of the smallest B used (2^-43 of terms at
+// least as large as f), which the bounds have room for.  What is not finite fails: g
+// is NaN beside an infinite f.  Six operations; reading the half ulp from f's
+// exponent took thirteen.
 SG_FF bool rounds_to(float f, float g, float B) {
-    const uint32_t u = bits(f) & 0x7FFFFFFFu;
-    const uint32_t E = u >> 23;
-    if (E - 26u > 227u) return false;                  // E outside [26, 253]
-    // a power of two: the boundary below is a quarter of its ulp away (taken
-    // on both sides)
-    const uint32_t hE = (u & 0x7FFFFFu) == 0u ? E - 25u : E - 24u;
-    const float lim = mul(from_bits(hE << 23), 0.99999904632568359375f);   // 1 - 2^-20
-    return add(absf(g), B) <= lim;
+    return absf(f) >= 3.944304526105059e-31f && add(f, add(g, B)) == f && add(f, sub(g, B)) == f;
 }
 
 constexpr float kBound = 9.094947017729282379e-13f;   // 2^-40
