@@ -50,6 +50,7 @@
 #include "counter_rng.h"
 #include "cuda_check.h"
 #include "iz_neuron.cuh"
+#include "launch.cuh"
 #include "props.h"
 
 namespace sg {
@@ -110,20 +111,60 @@ __device__ __forceinline__ float relay_value(const InstDev& I, long long t, int 
                                                                                     : 0.0f;
 }
 
-// kFcUnroll slots of a lane are loaded while as many are summed, OCC CTAs to an
-// SM.  HBM bounds a batch that fills the GPU, so what counts is bytes in flight:
-// 64 instances of 16..128 a side take 2.74 ms a step with 8 slots and 2 CTAs
-// (6.0 TB/s without padding), 2.97 with 16 and 1, 3.43 with 4 and 3, and took
-// 3.41 with 4 slots whose trace stores held back the next loads.  With no more
-// units than SMs a second CTA has nothing to do and the loads' latency is the
-// bound: 12 instances of 16..48 take 41 us a step with 16 slots, 48 with 8, and
-// took 66.
-template <int kFcUnroll, int OCC>
-__global__ void __launch_bounds__(kMaxThreads, OCC) k_batch_step(StepArgs A) {
+// A unit's source words and the relay values around its rows, by all threads.
+__device__ __forceinline__ void stage_unit(const InstDev& I, int row0, int tile_rows, long long t,
+                                           const uint32_t* __restrict__ words_in, uint32_t* sm,
+                                           float* relay) {
+    const int relay_rows = tile_rows + I.field - 1;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < I.n; i += blockDim.x) sm[i] = words_in[I.neuron_off + i];
+    for (int e = threadIdx.x; e < relay_rows * I.cols; e += blockDim.x) {
+        int rr = e / I.cols, cc = e - rr * I.cols;
+        int fr = wrap1(row0 - I.field / 2 + rr, I.rows);
+        relay[e] = t > 0 ? relay_value(I, t - 1, fr * I.cols + cc) : 0.0f;
+    }
+}
+
+// Neuron update; conductances were cleared by the previous update, so each is 0 +
+// this step's sum; the layer's input current is 0.
+__device__ __forceinline__ void batch_neuron(const StepArgs& A, const InstDev& I, int local,
+                                             float s_sum, float l_sum, float f_sum, float fl_sum,
+                                             const uint32_t* sm, uint32_t* words_out) {
+    const long long nid = I.neuron_off + local;
+    float voltage = A.v[nid], recovery = A.u[nid];
+    iz_integrate_ff(voltage, recovery, 0.0f + s_sum, 0.0f + l_sum, 0.0f + f_sum, 0.0f + fl_sum,
+                    0.0f, 0.0f, I.a, I.b);
+    unsigned int spike = voltage >= 30.0;
+    words_out[nid] = (sm[local] >> 1) | (spike << 31);
+    A.v[nid] = spike ? I.c : voltage;
+    A.u[nid] = recovery + (spike * I.d);
+}
+
+// The last CTA to finish sets the unit counter and the step for the next launch.
+__device__ __forceinline__ void batch_step_done(const StepArgs& A, long long t) {
+    __threadfence();
+    if (atomicAdd(A.done, 1) == (int)gridDim.x - 1) {
+        *A.ctr = 0;
+        *A.done = 0;
+        *A.step = t + 1;
+        __threadfence();
+    }
+}
+
+// kFcUnroll slots of a lane are loaded while as many are summed, two CTAs to an SM.
+// HBM bounds a batch that fills the GPU, so what counts is bytes in flight: 64
+// instances of 16..128 a side take 2.74 ms a step with 8 slots and 2 CTAs (6.0 TB/s
+// without padding), 2.97 with 16 and 1, 3.43 with 4 and 3, and took 3.41 with 4 slots
+// whose trace stores held back the next loads.  (With no more units than SMs:
+// k_batch_step_split.)
+constexpr int kFcUnroll = 8;
+
+__global__ void __launch_bounds__(kMaxThreads, 2) k_batch_step(StepArgs A) {
     extern __shared__ uint32_t sm[];
     __shared__ int s_unit;
     __shared__ long long s_t;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    wait_for_previous();
     if (tid == 0) s_t = *A.step;
     __syncthreads();
     const long long t = s_t;
@@ -140,14 +181,7 @@ __global__ void __launch_bounds__(kMaxThreads, OCC) k_batch_step(StepArgs A) {
         const InstDev I = A.inst[U.inst];
         const int h = I.field / 2;
         const int tile_rows = min(A.tile_rows, I.rows - U.row0);
-        const int relay_rows = tile_rows + I.field - 1;
-
-        for (int i = tid; i < I.n; i += blockDim.x) sm[i] = words_in[I.neuron_off + i];
-        for (int e = tid; e < relay_rows * I.cols; e += blockDim.x) {
-            int rr = e / I.cols, cc = e - rr * I.cols;
-            int fr = wrap1(U.row0 - h + rr, I.rows);
-            relay[e] = t > 0 ? relay_value(I, t - 1, fr * I.cols + cc) : 0.0f;
-        }
+        stage_unit(I, U.row0, tile_rows, t, words_in, sm, relay);
         __syncthreads();
 
         const int tr = warp / A.tile_cblocks, tcb = warp - tr * A.tile_cblocks;
@@ -232,30 +266,160 @@ __global__ void __launch_bounds__(kMaxThreads, OCC) k_batch_step(StepArgs A) {
                 }
             }
 
-            // neuron update; conductances were cleared by the previous update,
-            // so each is 0 + this step's sum; the layer's input current is 0
-            const int local = gr * I.cols + col;
-            const long long nid = I.neuron_off + local;
-            float voltage = A.v[nid], recovery = A.u[nid];
-            iz_integrate_ff(voltage, recovery, 0.0f + s_sum, 0.0f + l_sum, 0.0f + f_sum,
-                            0.0f + fl_sum, 0.0f, 0.0f, I.a, I.b);
-            unsigned int spike = voltage >= 30.0;
-            words_out[nid] = (sm[local] >> 1) | (spike << 31);
-            A.v[nid] = spike ? I.c : voltage;
-            A.u[nid] = recovery + (spike * I.d);
+            batch_neuron(A, I, gr * I.cols + col, s_sum, l_sum, f_sum, fl_sum, sm, words_out);
         }
         __syncthreads();
     }
 
-    if (tid == 0) {
-        __threadfence();
-        if (atomicAdd(A.done, 1) == (int)gridDim.x - 1) {
-            *A.ctr = 0;
-            *A.done = 0;
-            *A.step = t + 1;
-            __threadfence();
+    if (tid == 0) batch_step_done(A, t);
+}
+
+// The same step with a CTA of kParts + 1 warps to a group of 32 destinations: kParts
+// take the slots in turn, kPartSlots each a round, store their traces and put them in
+// shared memory; the last adds the round's in slot order, a round behind, and updates
+// the neurons.  For batches too small to fill the GPU, where a group's own chain
+// bounds the step (500 slots of 18 instructions in one warp, 6 cycles each) and then
+// its neurons' substeps.  12 instances of 16..48 take 29 us a step with 7 + 1 warps,
+// 32 with two groups of 3 + 1 in a CTA, 40 with 15 + 1, and took 41 with a warp a
+// group and 8 groups a CTA.
+constexpr int kParts = 7, kPartSlots = 4, kRound = kParts * kPartSlots;
+constexpr int kPartAhead = 4;            // rounds whose loads are in flight
+constexpr int kSplitThreads = (kParts + 1) * 32;
+
+__global__ void __launch_bounds__(kSplitThreads, 2) k_batch_step_split(StepArgs A) {
+    extern __shared__ uint32_t sm[];
+    __shared__ float2 tile[2][kRound][32];                 // pre-decay traces of a round
+    __shared__ int s_unit;
+    __shared__ long long s_t;
+    const int tid = threadIdx.x, lane = tid & 31, part = tid >> 5;
+    float* relay = reinterpret_cast<float*>(sm + A.words_cap);
+
+    long long t = -1;
+    // the first unit is the CTA's own; what is left is taken in turn
+    for (int ui = blockIdx.x; ui < A.n_units;) {
+        const Unit U = A.units[ui];
+        const InstDev I = A.inst[U.inst];
+        const int h = I.field / 2;
+        const int col = U.cb0 * 32 + lane;
+        const bool on = col < I.cols;
+        const long long g = I.group_off + (long long)U.row0 * I.cblocks + U.cb0;
+        const int slots = A.group_slots[g];
+        const long long base = A.group_base[g];
+        const uint2* in = A.fc_in + base * 32 + lane;
+        float2* trp = A.fc_tr + base * 32 + lane;
+        uint2 x[kPartAhead][kPartSlots];
+        float2 y[kPartAhead][kPartSlots];
+        auto load_in = [&](int r, uint2 (&xx)[kPartSlots]) {
+            const int s = r * kRound + part * kPartSlots;
+#pragma unroll
+            for (int j = 0; j < kPartSlots; ++j)
+                if (on && s + j < slots) xx[j] = __ldg(in + (s + j) * 32);
+        };
+        auto load_tr = [&](int r, float2 (&yy)[kPartSlots]) {
+            const int s = r * kRound + part * kPartSlots;
+#pragma unroll
+            for (int j = 0; j < kPartSlots; ++j)
+                if (on && s + j < slots) yy[j] = trp[(s + j) * 32];
+        };
+        if (part < kParts) {
+#pragma unroll
+            for (int q = 0; q < kPartAhead; ++q) load_in(q, x[q]);
         }
+        if (t < 0) {
+            // the layout and the synapses do not change; the rest is the last step's
+            wait_for_previous();
+            if (tid == 0) s_t = *A.step;
+            __syncthreads();
+            t = s_t;
+        }
+        const uint32_t* words_in = A.words + (t & 1) * A.n_neurons;
+        uint32_t* words_out = A.words + ((t + 1) & 1) * A.n_neurons;
+        if (part < kParts) {
+#pragma unroll
+            for (int q = 0; q < kPartAhead; ++q) load_tr(q, y[q]);
+        }
+        stage_unit(I, U.row0, 1, t, words_in, sm, relay);
+        __syncthreads();
+        const int fc_rounds = (slots + kRound - 1) / kRound;
+        const int conv_rounds = (I.K + kRound - 1) / kRound;
+        if (part < kParts) {
+            // convergent relay -> Izhikevich, "add": AMPA (short) and NMDA (long)
+            const float* ew = A.conv_ew + g * I.K * 32 + lane;
+            float2* ct = A.conv_tr + g * I.K * 32 + lane;
+            int b = 0;
+            for (int r = 0; r < conv_rounds; ++r, b ^= 1) {
+                const int k0 = r * kRound + part * kPartSlots;
+                float weight[kPartSlots];
+                float2 c[kPartSlots];
+#pragma unroll
+                for (int j = 0; j < kPartSlots; ++j)
+                    if (on && k0 + j < I.K) {
+                        weight[j] = __ldg(ew + (k0 + j) * 32);
+                        c[j] = ct[(k0 + j) * 32];
+                    }
+#pragma unroll
+                for (int j = 0; j < kPartSlots; ++j)
+                    if (on && k0 + j < I.K) {
+                        const int kr = (k0 + j) / I.field, kc = k0 + j - kr * I.field;
+                        const float spike = relay[kr * I.cols + wrap1(col - h + kc, I.cols)];
+                        const float st = c[j].x + (spike * weight[j] * I.gconv);
+                        const float lt = c[j].y + (spike * weight[j] * I.gconv);
+                        tile[b][part * kPartSlots + j][lane] = make_float2(st, lt);
+                        ct[(k0 + j) * 32] = make_float2(st * kAmpaTau, lt * kNmdaTau);
+                    }
+                __syncthreads();
+            }
+            // recurrent fully connected, "sub": GABA-A (short) and GABA-B (long)
+            const float gf = I.gfc;
+            for (int r = 0; r < fc_rounds; r += kPartAhead) {
+#pragma unroll
+                for (int q = 0; q < kPartAhead; ++q) {
+                    if (r + q >= fc_rounds) break;
+                    const int s = (r + q) * kRound + part * kPartSlots;
+#pragma unroll
+                    for (int j = 0; j < kPartSlots; ++j)
+                        if (on && s + j < slots) {
+                            const uint32_t word = sm[x[q][j].x & 0x07FFFFFFu];
+                            const float spike = (float)((word << (x[q][j].x >> 27)) >> 31);
+                            const float weight = __uint_as_float(x[q][j].y);
+                            const float st = y[q][j].x + (spike * weight * gf);
+                            const float lt = y[q][j].y + (spike * weight * gf);
+                            tile[b][part * kPartSlots + j][lane] = make_float2(st, lt);
+                            trp[(s + j) * 32] = make_float2(st * kGabaaTau, lt * kGababTau);
+                        }
+                    load_in(r + q + kPartAhead, x[q]);
+                    load_tr(r + q + kPartAhead, y[q]);
+                    __syncthreads();
+                    b ^= 1;
+                }
+            }
+        } else {
+            float sum[4] = {};
+            int b = 0;
+            auto add = [&](int n, float& s0, float& s1) {
+                __syncthreads();
+                float2 v[kRound];
+#pragma unroll
+                for (int i = 0; i < kRound; ++i) v[i] = tile[b][i][lane];
+#pragma unroll
+                for (int i = 0; i < kRound; ++i)
+                    if (i < n) {
+                        s0 += v[i].x;
+                        s1 += v[i].y;
+                    }
+                b ^= 1;
+            };
+            for (int r = 0; r < conv_rounds; ++r) add(I.K - r * kRound, sum[0], sum[1]);
+            for (int r = 0; r < fc_rounds; ++r) add(slots - r * kRound, sum[2], sum[3]);
+            if (on)
+                batch_neuron(A, I, U.row0 * I.cols + col, sum[0], sum[1], sum[2], sum[3], sm, words_out);
+        }
+        if ((int)gridDim.x >= A.n_units) break;
+        if (tid == 0) s_unit = (int)gridDim.x + atomicAdd(A.ctr, 1);
+        __syncthreads();
+        ui = s_unit;
     }
+    if (tid == 0) batch_step_done(A, t);
 }
 
 // Group of warp-global index gw: its instance, image row and column.
@@ -612,28 +776,48 @@ class Batch {
         launches_ = 0;
     }
 
-    void set_tile(int tile_rows, int tile_cblocks) {
-        if (tile_rows < 1 || tile_cblocks < 1 || tile_rows * tile_cblocks * 32 > kMaxThreads)
-            throw SgError("batch: tile must have 1..8 warps");
-        tile_rows_ = tile_rows;
-        tile_cblocks_ = tile_cblocks;
-        threads_ = tile_rows * tile_cblocks * 32;
-        words_cap_ = (max_n_ + 3) / 4 * 4;
-        smem_ = (size_t)(words_cap_ + (tile_rows + max_field_ - 1) * max_cols_) * 4;
-        if ((int)smem_ > smem_optin_) throw SgError("batch: instance too large for shared memory");
+    // The units of every instance, unit_rows_ x unit_cblocks_ groups each.
+    void make_units() {
         units_h_.clear();
         for (size_t i = 0; i < inst_.size(); ++i) {
             const InstDev& I = inst_[i];
-            for (int r0 = 0; r0 < I.rows; r0 += tile_rows)
-                for (int c0 = 0; c0 < I.cblocks; c0 += tile_cblocks) {
+            for (int r0 = 0; r0 < I.rows; r0 += unit_rows_)
+                for (int c0 = 0; c0 < I.cblocks; c0 += unit_cblocks_) {
                     long long cost = 0;
-                    for (int r = r0; r < std::min(I.rows, r0 + tile_rows); ++r)
-                        for (int c = c0; c < std::min(I.cblocks, c0 + tile_cblocks); ++c)
+                    for (int r = r0; r < std::min(I.rows, r0 + unit_rows_); ++r)
+                        for (int c = c0; c < std::min(I.cblocks, c0 + unit_cblocks_); ++c)
                             cost += group_slots_h_[I.group_off + (long long)r * I.cblocks + c] + I.K;
                     cost += I.n / 32 + 1;
                     units_h_.push_back(Unit{(int)i, r0, c0, (int)std::min<long long>(cost, 1 << 30)});
                 }
         }
+    }
+
+    void set_tile(int tile_rows, int tile_cblocks) {
+        if (tile_rows < 1 || tile_cblocks < 1 || tile_rows * tile_cblocks * 32 > kMaxThreads)
+            throw SgError("batch: tile must have 1..8 warps");
+        tile_rows_ = tile_rows;
+        tile_cblocks_ = tile_cblocks;
+        words_cap_ = (max_n_ + 3) / 4 * 4;
+        unit_rows_ = tile_rows;
+        unit_cblocks_ = tile_cblocks;
+        make_units();
+        auto shared = [&](int rows) {
+            return (size_t)(words_cap_ + (rows + max_field_ - 1) * max_cols_) * 4;
+        };
+        if ((int)shared(tile_rows) > smem_optin_)
+            throw SgError("batch: instance too large for shared memory");
+        // no more units than SMs: one for each group, with several warps
+        cudaFuncAttributes fa;
+        SG_CUDA(cudaFuncGetAttributes(&fa, k_batch_step_split));
+        const bool split = (int)units_h_.size() <= num_sms_ &&
+                           (int)(shared(1) + fa.sharedSizeBytes) <= smem_optin_;
+        if (split) {
+            unit_rows_ = unit_cblocks_ = 1;
+            make_units();
+        }
+        threads_ = split ? kSplitThreads : tile_rows * tile_cblocks * 32;
+        smem_ = shared(unit_rows_);
         std::stable_sort(units_h_.begin(), units_h_.end(),
                          [](const Unit& a, const Unit& b) { return a.cost > b.cost; });
         if (!d_units_ || units_h_.size() > units_cap_) {
@@ -642,10 +826,9 @@ class Batch {
         }
         SG_CUDA(cudaMemcpyAsync(d_units_, units_h_.data(), units_h_.size() * sizeof(Unit),
                                 cudaMemcpyHostToDevice, stream_));
-        kernel_ = (int)units_h_.size() <= num_sms_ ? k_batch_step<16, 1> : k_batch_step<8, 2>;
+        kernel_ = split ? k_batch_step_split : k_batch_step;
         // the limit is the function's, shared by every batch of the process:
         // always the largest, or a smaller batch would lower it for a larger one
-        cudaFuncAttributes fa;
         SG_CUDA(cudaFuncGetAttributes(&fa, kernel_));
         SG_CUDA(cudaFuncSetAttribute(kernel_, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      smem_optin_ - (int)fa.sharedSizeBytes));
@@ -664,8 +847,8 @@ class Batch {
         a.inst = d_inst_;
         a.units = d_units_;
         a.n_units = (int)units_h_.size();
-        a.tile_rows = tile_rows_;
-        a.tile_cblocks = tile_cblocks_;
+        a.tile_rows = unit_rows_;
+        a.tile_cblocks = unit_cblocks_;
         a.words_cap = words_cap_;
         a.group_base = d_group_base_;
         a.group_slots = d_group_slots_;
@@ -684,14 +867,13 @@ class Batch {
     }
 
     void launch() {
-        kernel_<<<grid_, threads_, smem_, stream_>>>(args());
-        SG_LAUNCH_CHECK();
+        launch_dependent(kernel_, grid_, threads_, smem_, stream_, args());
     }
 
     void capture() {
         cudaGraph_t g;
         SG_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-        for (int i = 0; i < kGraphSteps; ++i) kernel_<<<grid_, threads_, smem_, stream_>>>(args());
+        for (int i = 0; i < kGraphSteps; ++i) launch();
         SG_CUDA(cudaStreamEndCapture(stream_, &g));
         cudaError_t e = cudaGraphInstantiate(&graph_, g, 0);
         cudaGraphDestroy(g);
@@ -741,6 +923,7 @@ class Batch {
     std::vector<Unit> units_h_;
     std::vector<TuneResult> tuning_;
     std::vector<void*> owned_;
+    int unit_rows_ = 1, unit_cblocks_ = 1;
     long long n_neurons_ = 0, n_groups_ = 0, slot_rows_ = 0, fc_synapses_ = 0;
     long long conv_synapses_ = 0, device_bytes_ = 0, steps_ = 0, launches_ = 0;
     int max_n_ = 0, max_cols_ = 0, max_rows_ = 0, max_field_ = 0, max_cblocks_ = 0, K_ = 0;

@@ -406,3 +406,29 @@ def test_one_pass_trace_activator(sg, sources, dests, model, opcode, learning):
               ("matrix", "c", "short term w"): draw(0.2, 0.8, n)}
     keys = [("matrix", "c", "short trace"), ("b", "voltage"), ("b", "input")]
     assert_equal(run_both(sg, net, inject, 4, keys, learning=learning))
+
+
+# a CTA a group of 32 destinations while the tile's units are no more than the SMs:
+# rounds of 28 slots, 112 of them in flight, convolutions of more and fewer positions
+# than a round, ragged groups, more groups than resident CTAs
+@pytest.mark.parametrize("sides", [[(5, 6)], [(7, 33), (16, 16)], [(31, 64), (9, 10), (48, 48)],
+                                   [(64, 64), (40, 96), (33, 65)]])
+@pytest.mark.parametrize("field", [3, 5, 7])
+def test_batch_split_groups(sg, sides, field):
+    from synaptogenesis_gb300 import batching
+    insts = [dict(batching.instance(r + c, 70 + i, rows=r, cols=c), conv_field=field)
+             for i, (r, c) in enumerate(sides)]
+    for inst in insts:
+        inst["input_rate"] = 0.1
+
+    def run(more, tile):
+        with sg.Batch(insts + more, tile=tile) as b:
+            b.step(37)
+            return [b.read(i, k).view(np.uint32) for i in range(len(insts))
+                    for k in ("voltage", "recovery", "output")], int(b.report().properties["threads"])
+
+    split, threads = run([], (8, 1))
+    assert threads == 256
+    # beside enough others the same instances take the tile's units
+    whole, _ = run([dict(batching.instance(96, 300 + i), conv_field=field) for i in range(24)], (2, 1))
+    assert all(np.array_equal(a, b) for a, b in zip(split, whole))
