@@ -70,10 +70,14 @@ __global__ void __launch_bounds__(256) k_activate_base(DGeom g, const uint32_t* 
 // words two chunks of kColsRows rows ahead into registers and leave the
 // products in shared memory by destination, one chunk ahead of the fifth warp,
 // which sums them (a lane per destination).  Rows past the end are products of
-// +0: they do not change a sum that started at +0.
+// +0: they do not change a sum that started at +0.  A whole chunk's adds are written
+// out, so that their loads run ahead of them.
 // Measured with cold caches: 4096 -> 4096 308 us with a thread per destination
 // reading its own weights, 29 us with one warp per band fetching (cp.async),
-// multiplying and adding, 22 us like this; 784 -> 500 58, 8.1 and 5.7 us.
+// multiplying and adding, 22 us like this; 784 -> 500 58, 8.1 and 5.7 us.  In a run,
+// whose 64 MB of weights come from both memory and cache, a step of 4096 -> 4096
+// takes 31.3 us in all; 33.1 with 16 rows' loads ahead of 16 rows' adds, and half
+// rows of 16-byte loads or other counts of producers change nothing (31.5 to 32).
 // ---------------------------------------------------------------------------
 constexpr int kColsRows = 256;
 constexpr int kColsProducers = 128;
@@ -144,24 +148,29 @@ __global__ void __launch_bounds__(kColsProducers + 32) k_activate_cols(
     for (int ch = 0; ch < nchunks; ++ch) {
         const float4* t = reinterpret_cast<const float4*>(
             &prod[ch & 1][(lane % kBand) * kColsPitch]);
-        const int groups = (min(kColsRows, nrows - ch * kColsRows) + 15) / 16;
-        float4 a[4];
+        const int quads = (min(kColsRows, nrows - ch * kColsRows) + 3) / 4;
+        if (lane < kBand) {               // (a 16-byte load by all lanes takes 4 passes)
+            if (quads == kColsRows / 4) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) a[q] = t[q];
-        for (int i = 1; i <= groups; ++i) {
-            float4 b[4];                                  // the next 16 while these are added
-#pragma unroll
-            for (int q = 0; q < 4; ++q) b[q] = t[(i < groups ? 4 * i : 0) + q];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                sum += a[q].x;
-                sum += a[q].y;
-                sum += a[q].z;
-                sum += a[q].w;
+                for (int q = 0; q < kColsRows / 4; ++q) {
+                    const float4 a = t[q];
+                    sum += a.x;
+                    sum += a.y;
+                    sum += a.z;
+                    sum += a.w;
+                }
+            } else {
+#pragma unroll 4
+                for (int q = 0; q < quads; ++q) {
+                    const float4 a = t[q];
+                    sum += a.x;
+                    sum += a.y;
+                    sum += a.z;
+                    sum += a.w;
+                }
             }
-#pragma unroll
-            for (int q = 0; q < 4; ++q) a[q] = b[q];
         }
+        __syncwarp();
         __syncthreads();
     }
     const int d = band * kBand + lane;

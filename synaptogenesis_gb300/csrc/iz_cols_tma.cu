@@ -495,13 +495,15 @@ __global__ void __launch_bounds__(kSmallProducers + 32) k_iz_cols_small(
         asm volatile("bar.sync %0, %1;" ::"r"(1 + ch), "n"(kSmallProducers + 32) : "memory");
         const float4* t = reinterpret_cast<const float4*>(col + ch * kSmallChunk);
         const int groups = (min(kSmallChunk, nrows - ch * kSmallChunk) + 15) / 16;
-        float4 a[4];
+        float4 a[4] = {};
 #pragma unroll
-        for (int q = 0; q < 4; ++q) a[q] = t[q];
+        for (int q = 0; q < 4; ++q)
+            if (mine) a[q] = t[q];
         for (int i = 1; i <= groups; ++i) {
-            float4 b[4];                                   // the next 16 while these are added
+            float4 b[4] = {};                              // the next 16 while these are added
 #pragma unroll
-            for (int q = 0; q < 4; ++q) b[q] = t[(i < groups ? 4 * i : 0) + q];
+            for (int q = 0; q < 4; ++q)
+                if (mine) b[q] = t[(i < groups ? 4 * i : 0) + q];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 acc += a[q].x;
