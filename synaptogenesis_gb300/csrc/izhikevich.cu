@@ -1273,7 +1273,6 @@ __global__ void __launch_bounds__(kWindowDests) k_spnet_activate_window(
     DGeom g, const uint32_t* __restrict__ src, int n_src, const int* __restrict__ first, int window,
     const uint32_t* __restrict__ packed, const float* __restrict__ w, float gc, int opcode,
     float* __restrict__ inputs) {
-    wait_for_previous();
     extern __shared__ uint32_t staged[];
     const unsigned d = blockIdx.x * kWindowDests + threadIdx.x;
     const int n = d < (unsigned)g.n_dest ? g.nz[d] : 0;
@@ -1282,7 +1281,7 @@ __global__ void __launch_bounds__(kWindowDests) k_spnet_activate_window(
     auto stage = [&] {
         for (int i = threadIdx.x; i < window; i += kWindowDests) {
             const int from = lo + i;
-            staged[i] = src[from < n_src ? from : from - n_src];
+            staged[i] = after_wait(src)[from < n_src ? from : from - n_src];
         }
         __syncthreads();
     };
@@ -1330,8 +1329,11 @@ __global__ void __launch_bounds__(kWindowDests) k_spnet_activate_window(
             }
         }
     };
+    // the words do not change, the weights with learning, which the setting of the
+    // registers at least has followed: before the wait
     load(0, 0);
     load(1, kSpnetAhead);
+    wait_for_previous();
     stage();
     for (int i = 0; i < nmax; i += 2 * kSpnetAhead) {
         add(0, i);
