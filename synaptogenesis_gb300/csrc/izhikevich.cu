@@ -267,11 +267,15 @@ __device__ __forceinline__ int conv_source_at(const DGeom& g, int2 base, int2 of
 // coalesced 128-byte row of the [k][destination] layout and each warp has
 // many independent loads in flight.  Pre-decay traces go to shared memory and
 // lanes of warps 0 / 1 add them in k order (the reference's sequential sum),
-// skipping positions outside a non-wrapping layer as the reference does.
+// skipping positions outside a non-wrapping layer as the reference does.  Bytes in
+// flight bound it (29 a synapse with two traces): 81 positions of 65,536 destinations
+// take 28 us with 5 CTAs to an SM (5.5 TB/s), 33 with 4, 30 to 36 with 6 or 8, which
+// spill or hold fewer loads, and took 38 with 4 and a sum that tested the wrap and
+// waited for shared memory at each term.
 constexpr int kConvMaxK = 128;
 
 template <int SR, bool LONG>
-__global__ void __launch_bounds__(256, 4) k_iz_activate_conv_tile(
+__global__ void __launch_bounds__(256, 5) k_iz_activate_conv_tile(
     DGeom g, int K, const uint32_t* __restrict__ src, const float* __restrict__ w,
     const float* __restrict__ stp_r, const float* __restrict__ stp_w, const uint8_t* __restrict__ delays,
     float* __restrict__ short_tr, float* __restrict__ long_tr, float gcond, float short_tau,
@@ -337,16 +341,19 @@ __global__ void __launch_bounds__(256, 4) k_iz_activate_conv_tile(
     }
     __syncthreads();
     if (!ok) return;
-    if (warp == 0) {
+    if (warp < (LONG ? 2 : 1)) {
+        const float (*terms)[32] = LONG && warp == 1 ? s_lt : s_st;
+        float* cond = LONG && warp == 1 ? long_cond : short_cond;
+        const float before = cond[d];
         float sum = 0.0f;
-        for (int k = 0; k < K; ++k)
-            if (g.wrap || conv_source_at(g, base, koff[k]) >= 0) sum += s_st[k][lane];
-        short_cond[d] += sum;
-    } else if (LONG && warp == 1) {
-        float sum = 0.0f;
-        for (int k = 0; k < K; ++k)
-            if (g.wrap || conv_source_at(g, base, koff[k]) >= 0) sum += s_lt[k][lane];
-        long_cond[d] += sum;
+        if (g.wrap) {
+#pragma unroll 16
+            for (int k = 0; k < K; ++k) sum += terms[k][lane];
+        } else {
+            for (int k = 0; k < K; ++k)
+                if (conv_source_at(g, base, koff[k]) >= 0) sum += terms[k][lane];
+        }
+        cond[d] = before + sum;
     }
 }
 
