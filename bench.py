@@ -921,13 +921,13 @@ def rate_line(args, world, r, wl, cb):
     c = RATE_CFG
     per_step = c["batch"] * c["steps"]
     achieved = r["fwd_bytes_per_timestep"] / (r["fwd_us_per_timestep"] * 1e-6) / 1e9
-    # kernel launches per forward + adjoint: forward = weight transpose, the
-    # multi-step forward kernel, outputs, loss; backward = weight transpose,
-    # dloss/dy, per segment the multi-step recompute, dW and its accumulation,
-    # dR and its accumulation, dtau partials, per timestep an adjoint step,
-    # and the dtau total
+    # kernel launches per forward + adjoint: forward = weight transpose, for each of
+    # 4 chunks of 25 steps (64 MiB of two layers' rates) every layer and the readout,
+    # the loss; backward = weight transpose, dloss/dy, per segment every layer twice
+    # (recompute and adjoint), dW, dR and their accumulation, then the gradients and
+    # dtau's two kernels
     nseg = -(-c["steps"] // c["checkpoint"])
-    launches = 4 + (2 + 6 * nseg + c["steps"] + 1)
+    launches = (2 + 4 * (c["layers"] + 1)) + (2 + nseg * (2 * c["layers"] + 3) + 3)
     return {
         "metric": "sequence-timesteps/s (rate forward + adjoint)",
         "value": r["units"] / r["dev_s"], "unit": wl["unit"], "n_gpus": world,

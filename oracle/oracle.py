@@ -131,7 +131,7 @@ def noise_cospi(x):
 
 
 def noise_draw(kind, seed, step, n, a, b, rates=None):
-    """One step of init-config noise for n neurons (the library's k_noise):
+    """One step of init-config noise for n neurons (the library's k_init_inputs):
     kind "uniform" (min a, max b), "normal" (mean a, std b), "poisson"
     (probability a or per-neuron rates; value b, returned as a mask and b)."""
     idx = (np.uint64(step) << np.uint64(32)) | np.arange(n, dtype=np.uint64)
