@@ -1606,9 +1606,9 @@ __global__ void __launch_bounds__(kSpnetLearnThreads) k_spnet_learn_sparse(DGeom
             dw = spnet_dw_full(dw0, f1, f2);
         }
         if (__float_as_uint(dw) != __float_as_uint(dw0)) dws[wi] = dw;
-        // dw + 0.01 in double; what is below 2^-60 is gone in it
+        // dw + 0.01 in double; what is at most 2^-60 is gone in it (a NaN is not)
         float weight_delta = S1;
-        if (fabsf(dw) > 8.673617379884035e-19f && !ff::add_const(dw, S1, S2, weight_delta))
+        if (!(fabsf(dw) <= 8.673617379884035e-19f) && !ff::add_const(dw, S1, S2, weight_delta))
             weight_delta = d2f_rn(__dadd_rn(f2d_exact(dw), 0.01));
         weight += lr * weight_delta;
         const float capped = (max_weight < weight) ? max_weight : weight;

@@ -432,3 +432,37 @@ def test_batch_split_groups(sg, sides, field):
     # beside enough others the same instances take the tile's units
     whole, _ = run([dict(batching.instance(96, 300 + i), conv_field=field) for i in range(24)], (2, 1))
     assert all(np.array_equal(a, b) for a, b in zip(split, whole))
+
+
+# derivatives, traces and weights that are not finite, as a float-valued source's words
+# read as spikes make them: a NaN derivative makes a NaN weight, in the sparse kernel as
+# in the dense one
+@pytest.mark.parametrize("sparse", [True, False])
+@pytest.mark.parametrize("source", ["spnet", "relay"])
+@pytest.mark.parametrize("opcode", ["add", "sub"])
+def test_spnet_learning_of_what_is_not_finite(sg, opcode, source, sparse):
+    sources, dests = 9, 130
+    n = sources * dests
+    net = network([layer("a", source, 1, sources, **({"params": "regular"} if source == "spnet" else {})),
+                   layer("b", "spnet", 1, dests, params="fast")],
+                  [connection("c", "a", "b", "fully connected", opcode=opcode, plastic=True, sparse=sparse,
+                              **{"weight config": {"type": "flat", "weight": 1.0}})])
+    odd = np.array([np.nan, np.inf, -np.inf, 3e38, -3e38, 0, 2.0**-60, 2.0**-61, 1e-40, 0.1], np.float32)
+    rng = np.random.default_rng(sources)
+    draw = lambda: np.where(rng.random(n) < 0.5, rng.choice(odd, n),         # noqa: E731
+                            rng.uniform(0, 1, n)).astype(np.float32)
+    # (a relay's own words as numbers; the destinations' as spikes, floats among them NaN)
+    words = rng.integers(0, 2**32, sources, dtype=np.uint64).astype(np.uint32)
+    inject = {("a", "output"): words if source == "spnet" else rng.choice(odd[5:], sources),
+              ("b", "output"): np.where(rng.random(dests) < 0.3, 0xFF800001,
+                                        rng.integers(0, 2**32, dests, dtype=np.uint64)).astype(np.uint32),
+              ("matrix", "c", "weights"): np.where(rng.random(n) < 0.2, odd[rng.integers(0, 10, n)],
+                                                   rng.uniform(0.1, 5, n)).astype(np.float32),
+              ("matrix", "c", "weight derivative"): draw(), ("matrix", "c", "presyn trace"): draw()}
+    keys = [("matrix", "c", k) for k in ("weights", "weight derivative", "presyn trace")]
+    results = run_both(sg, net, inject, 2, keys, learning=True)
+    for key, (got, want) in results.items():
+        g, w = got.view(np.float32), want.view(np.float32)
+        bad = np.flatnonzero((got != want) & ~(np.isnan(g) & np.isnan(w)))
+        assert bad.size == 0, (key, bad.size, g[bad[:3]], w[bad[:3]])
+    assert np.isnan(results[keys[0]][1].view(np.float32)).sum() > 20
