@@ -466,3 +466,37 @@ def test_spnet_learning_of_what_is_not_finite(sg, opcode, source, sparse):
         bad = np.flatnonzero((got != want) & ~(np.isnan(g) & np.isnan(w)))
         assert bad.size == 0, (key, bad.size, g[bad[:3]], w[bad[:3]])
     assert np.isnan(results[keys[0]][1].view(np.float32)).sum() > 20
+
+
+def rate_pass(net, p, y=None):
+    """Loss and gradients of a RateNetwork for arrays p, as numpy."""
+    import torch
+    t = {k: torch.tensor(np.asarray(v, np.float32), device="cuda") for k, v in p.items()}
+    loss, ws = net._forward(**t, y=y)
+    args = [t[k] for k in ("x", "weights", "readout", "tau", "target")]
+    grads = dict(zip(("x", "weights", "readout", "tau"), net._backward(ws, 1.0, *args)))
+    return {k: v.cpu().numpy() for k, v in dict(grads, loss=loss).items()}
+
+
+def test_rate_sigmoid(sg):
+    """One step from rest with tau 1 makes v the input; the readout picks single
+    neurons.  The exponential errs by at most 2 + 1.173 |v| units in the last place, the
+    sum with 1 and the reciprocal by half of one each; where the exponential overflows
+    (below -88.7) the sigmoid is less than 2^-128."""
+    import torch
+    batch, n = 65535, 16
+    net = sg.RateNetwork(layers=1, rows=1, cols=n, field=1, outputs=n, batch=batch, steps=1)
+    rng = np.random.default_rng(3)
+    v = rng.uniform(-100, 40, (1, batch, n)).astype(np.float32)
+    v[:, ::4] = rng.uniform(-89, -86, v[:, ::4].shape)
+    v[0, 0] = [0, -0.0, 1e-30, -1e-30, 88, 100, -88, -150, 3e38, -3e38, np.inf, -np.inf, 17, -17, 1, -1]
+    y = torch.empty((1, batch, n), device="cuda")
+    rate_pass(net, {"x": v, "weights": np.zeros((0, n, 1)), "readout": np.eye(n), "tau": [1.0],
+                    "target": np.zeros((batch, n))}, y)
+    got, x = y.cpu().numpy().astype(np.float64), v.astype(np.float64)
+    # an infinite neuron makes the zero weights' terms NaN only in its own batch element
+    got, x = np.delete(got, 0, 1), np.delete(x, 0, 1)
+    want = np.exp(np.minimum(x, 0)) / (1 + np.exp(-np.abs(x)))
+    bound = ((2 + 1.173 * np.abs(x)) + 1) * 2.0**-23 * want + 2.0**-127
+    bad = np.flatnonzero(~(np.abs(got - want) <= bound))
+    assert bad.size == 0, (bad.size, x.ravel()[bad[:4]], got.ravel()[bad[:4]], want.ravel()[bad[:4]])
