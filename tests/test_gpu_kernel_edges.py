@@ -500,3 +500,26 @@ def test_rate_sigmoid(sg):
     bound = ((2 + 1.173 * np.abs(x)) + 1) * 2.0**-23 * want + 2.0**-127
     bad = np.flatnonzero(~(np.abs(got - want) <= bound))
     assert bad.size == 0, (bad.size, x.ravel()[bad[:4]], got.ravel()[bad[:4]], want.ravel()[bad[:4]])
+
+
+def test_rate_adjoint_adds_kernel_rows(sg):
+    """Nine terms p of one kernel row beside +2^26 p and -2^26 p of the rows before and
+    after: the row's sum 9 p is added whole (to a multiple of the large one's spacing,
+    4 p to 8 p), where p by itself is less than half the spacing and would be lost."""
+    side, h = 9, 4
+    n = side * side
+    net = sg.RateNetwork(layers=2, rows=side, cols=side, field=9, outputs=1, batch=1, steps=2)
+    centre = h * side + h
+
+    def input_gradient(rows):
+        w = np.zeros((1, n, 81))
+        for (kr, kc), value in rows.items():           # the destination that reads the centre at (kr, kc)
+            w[0, (2 * h - kr) * side + 2 * h - kc, kr * 9 + kc] = value
+        # a time constant of 2^60 keeps layer 1 at rest whatever its input is
+        got = rate_pass(net, {"x": np.full((2, 1, n), 0.3), "weights": w, "readout": np.full((1, n), 0.37),
+                              "tau": [3.0, 2.0**60], "target": [[0.2]]})
+        return got["x"][0, 0, centre]
+
+    one = input_gradient({(4, 4): 1.0})
+    row = input_gradient({(0, 0): 2.0**26, (2, 0): -(2.0**26), **{(1, kc): 1.0 for kc in range(9)}})
+    assert 5.0 <= row / one <= 13.0, (row, one)
