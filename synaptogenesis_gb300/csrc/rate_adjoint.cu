@@ -840,17 +840,19 @@ __global__ void __launch_bounds__(256) k_rate_dtau_partial(Dims D, const float* 
     if (tid == 0) part[(long long)l * kTauBlocks + blockIdx.x] = sm[0];
 }
 
-// dtau_l = -(dt / tau_l^2) * sum of the layer's partials in block order.
+// dtau_l = -(dt / tau_l^2) * sum of the layer's partials in block order, in double: the
+// parts of one sign or the other cancel, and 64 float additions in a row err by more
+// than everything before them (25 % of the error of dtau).
 __global__ void __launch_bounds__(256) k_rate_dtau_final(Dims D, const float* __restrict__ tau,
                                                          const float* __restrict__ part,
                                                          float* __restrict__ dtau) {
     wait_for_previous();
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= D.L) return;
-    float s = 0.0f;
+    double s = 0.0;
     for (int q = 0; q < kTauBlocks; ++q) s += part[(long long)l * kTauBlocks + q];
     const float tv = __ldg(tau + l);
-    dtau[l] = s * (-D.dt / (tv * tv));
+    dtau[l] = (float)s * (-D.dt / (tv * tv));
 }
 
 // A segment's state of up to this many bytes stays in L2 and costs less than

@@ -502,6 +502,23 @@ def test_rate_sigmoid(sg):
     assert bad.size == 0, (bad.size, x.ravel()[bad[:4]], got.ravel()[bad[:4]], want.ravel()[bad[:4]])
 
 
+def test_rate_tau_gradient_of_equal_elements(sg):
+    """2^14 equal batch elements of one neuron: the loss is one element's, and every
+    quantity of the gradient is scaled by a power of two and added up to the same bits."""
+    rng = np.random.default_rng(5)
+    for _ in range(24):
+        steps = 4
+        x, tau = rng.normal(0, 1, (steps, 1, 1)), rng.uniform(2, 9, 1)
+        readout, target = rng.normal(0, 1, (1, 1)), rng.uniform(0, 1, (1, 1))
+        tau_grads = []
+        for batch in (1, 1 << 14):
+            net = sg.RateNetwork(layers=1, rows=1, cols=1, field=1, outputs=1, batch=batch, steps=steps)
+            got = rate_pass(net, {"x": np.repeat(x, batch, 1), "weights": np.zeros((0, 1, 1)), "readout": readout,
+                                  "tau": tau, "target": np.repeat(target, batch, 0)})
+            tau_grads.append(got["tau"][0])
+        assert tau_grads[0] == tau_grads[1], tau_grads
+
+
 def test_rate_adjoint_adds_kernel_rows(sg):
     """Nine terms p of one kernel row beside +2^26 p and -2^26 p of the rows before and
     after: the row's sum 9 p is added whole (to a multiple of the large one's spacing,
