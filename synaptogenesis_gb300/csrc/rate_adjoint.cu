@@ -952,11 +952,19 @@ Work carve(const Dims& D, void* base) {
 
 unsigned grid_of(long long n) { return (unsigned)((n + 255) / 256); }
 
-// Every launch of a pass is a programmatic dependent of the one before it.
+// Every launch of a pass is a programmatic dependent of the one before it, but for
+// k_rate_dw with few CTAs (below).
 template <class... P, class... A>
 void launch(void (*kernel)(P...), dim3 grid, int threads, cudaStream_t st, A... args) {
     launch_dependent(kernel, grid, dim3((unsigned)threads), 0, st, args...);
 }
+
+// CTAs of k_rate_dw are small and run long, a whole batch each.  Launched while the
+// adjoint's last wave ends they crowd onto the SMs that are free first, up to a dozen to
+// one, and the others stay empty: up to 8 CTAs to an SM wait for the launch before
+// (3 x 64x16, field 3, batch 256: 0.71 ms a training step, 1.28 as dependents; 6 x 16x16,
+// batch 256: 0.79 and 1.30; 2 x 256x256, batch 4, 9 CTAs to an SM: 0.44 and 0.43).
+bool crowds(const dim3& grid) { return (long long)grid.x * grid.y * grid.z <= 8 * 152; }
 
 void transpose_weights(const Dims& D, const float* w, const Work& W, cudaStream_t st) {
     if (D.L < 2) return;
@@ -1094,7 +1102,12 @@ void backward(const Dims& D, const float* x, const float* w, const float* wo, co
         if (D.L > 1) {
             SG_RATE_TILE(D, W, wide(D, (long long)(D.L - 1) * nt), ({
                 const dim3 grid(tiles(D, PY), (unsigned)(D.L - 1), (unsigned)nt);
-                launch(k_rate_dw<F, PY, V>, grid, kTileThreads, st, D, W.seg_P, W.seg_r, W.grad_part);
+                if (crowds(grid)) {
+                    k_rate_dw<F, PY, V><<<grid, kTileThreads, 0, st>>>(D, W.seg_P, W.seg_r, W.grad_part);
+                    SG_LAUNCH_CHECK();
+                } else {
+                    launch(k_rate_dw<F, PY, V>, grid, kTileThreads, st, D, W.seg_P, W.seg_r, W.grad_part);
+                }
             }));
                 }
         const int dwo_v = W.aligned && D.N % 4 == 0 ? 4 : 1, per = kReadoutThreads * dwo_v;
