@@ -78,6 +78,9 @@ __global__ void __launch_bounds__(256) k_activate_base(DGeom g, const uint32_t* 
 // whose 64 MB of weights come from both memory and cache, a step of 4096 -> 4096
 // takes 31.3 us in all; 33.1 with 16 rows' loads ahead of 16 rows' adds, and half
 // rows of 16-byte loads or other counts of producers change nothing (31.5 to 32).
+//
+// A CTA costs some 3.5 us before its first chunk is summed, whatever its rows, so many
+// destinations of few sources are left to k_activate_base, a thread each (cols_wins).
 // ---------------------------------------------------------------------------
 constexpr int kColsRows = 256;
 constexpr int kColsProducers = 128;
@@ -179,6 +182,17 @@ __global__ void __launch_bounds__(kColsProducers + 32) k_activate_cols(
     inputs[to] = aggregate(inputs[to], sum, opcode);
 }
 
+// Whether a dense matrix takes k_activate_cols.  Measured with 1 to 4096 sources (us a
+// step of relay -> rate layers, the columns' kernel / a thread a destination): they break
+// even near 50 sources for up to 4096 destinations (1024 destinations of 16 sources 4.9 /
+// 4.0, of 64 5.0 / 5.4), 130 for 8192, 350 for 16384 (256 sources 12.2 / 11.8, 512 15.9 /
+// 19.0) and 600 from 24000 to 65536 (512 sources 48 / 47, 1024 76 / 88); with 131072 and
+// more the thread kernel has the whole GPU busy and is faster throughout (2048 sources
+// 234 / 197; 4 sources of 10^6 destinations 269 / 18).
+static bool cols_wins(int sources, int dests) {
+    return dests <= 98304 && sources >= std::min(640, std::max(48, dests / 40 - 64));
+}
+
 void launch_base_activator(State& st, ConnState& cs, float* inputs, cudaStream_t s) {
     const Connection& c = *cs.conn;
     const uint32_t* src = st.dev_output(c.from, word_index(c.delay, c.from->output_type));
@@ -187,9 +201,9 @@ void launch_base_activator(State& st, ConnState& cs, float* inputs, cudaStream_t
     // a second-order host reads the copy of its weights the slaves modulated
     // (synapse_data.cpp:20-23)
     const float* w = cs.so_weights ? cs.so_weights->df() : cs.weights->df();
-    if (c.type == FULLY_CONNECTED || c.type == SUBSET) {
-        const bool subset = c.type == SUBSET;
-        const int nrows = subset ? c.subset.from_size() : c.from->size, op = (int)c.opcode;
+    const bool subset = c.type == SUBSET;
+    const int nrows = subset ? c.subset.from_size() : c.from->size, op = (int)c.opcode;
+    if ((subset || c.type == FULLY_CONNECTED) && cols_wins(nrows, cs.geom.n_dest)) {
         const unsigned bands = blocks_for(cs.geom.n_dest, kBand);
 #define SG_COLS(SRV)                                                                        \
     if (subset)                                                                              \

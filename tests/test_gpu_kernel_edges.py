@@ -540,3 +540,34 @@ def test_rate_adjoint_adds_kernel_rows(sg):
     one = input_gradient({(4, 4): 1.0})
     row = input_gradient({(0, 0): 2.0**26, (2, 0): -(2.0**26), **{(1, kc): 1.0 for kc in range(9)}})
     assert 5.0 <= row / one <= 13.0, (row, one)
+
+
+# either side of the line between the two kernels of dense matrices (48 sources for few
+# destinations, 186 for 10000, none for 98305), numbers and spikes
+@pytest.mark.parametrize("sources,dests", [(47, 900), (48, 900), (185, 10000), (186, 10000), (3, 98304), (700, 1500),
+                                           (50, 98305)])
+@pytest.mark.parametrize("model,delay", [("relay", 0), ("game_of_life", 7)])
+def test_dense_base_activators_by_size(sg, sources, dests, model, delay):
+    rng = np.random.default_rng(sources + dests)
+    net = network([layer("a", model, 1, sources), layer("b", "relay", 1, dests)],
+                  [connection("c", "a", "b", "fully connected", delay=delay, opcode="sub")])
+    words = rng.standard_normal(sources).astype(np.float32).view(np.uint32) if model == "relay" \
+        else rng.integers(0, 2**32, sources, dtype=np.uint64).astype(np.uint32)
+    inject = {("a", "output"): words,
+              ("matrix", "c", "weights"): rng.standard_normal(sources * dests).astype(np.float32)}
+    assert_equal(run_both(sg, net, inject, 1, [("b", "input"), ("b", "output")]))
+
+
+def test_dense_base_activators_of_windows(sg):
+    """Subset windows of few and of many sources, side by side with the dense form."""
+    rng = np.random.default_rng(4)
+    window = lambda k: {"subset config": {                                   # noqa: E731
+        "from row start": 1, "from row end": 1 + k, "from column start": 2, "from column end": 2 + k,
+        "to row start": 0, "to row end": 20, "to column start": 1, "to column end": 17}}
+    net = network([layer("a", "relay", 20, 17), layer("b", "relay", 20, 17)],
+                  [connection("few", "a", "b", "subset", **window(3)),
+                   connection("many", "a", "b", "subset", opcode="sub", **window(15))])
+    inject = {("a", "output"): rng.standard_normal(20 * 17).astype(np.float32).view(np.uint32)}
+    for name, k in (("few", 3), ("many", 15)):
+        inject[("matrix", name, "weights")] = rng.standard_normal(k * k * 320).astype(np.float32)
+    assert_equal(run_both(sg, net, inject, 1, [("b", "input")]))
