@@ -571,3 +571,26 @@ def test_dense_base_activators_of_windows(sg):
     for name, k in (("few", 3), ("many", 15)):
         inject[("matrix", name, "weights")] = rng.standard_normal(k * k * 320).astype(np.float32)
     assert_equal(run_both(sg, net, inject, 1, [("b", "input")]))
+
+
+# registers of all layers in launches of 16, a neuron a thread up to 2^18 neurons and eight
+# beyond; relay and rate layers of more than 8 blocks to an SM
+def test_input_registers_of_many_and_large_layers(sg):
+    from tests.golden.cases import Case
+    from tests.harness import compare, run_library, run_oracle
+    kinds = [None, {"type": "flat", "value": 0.75}, {"type": "uniform", "min": -1, "max": 2, "seed": 5},
+             {"type": "poisson", "rate": 200, "value": 1.5, "seed": 7},
+             {"type": "poisson", "rate": 300, "value": 2.5, "random": True, "seed": 8},
+             {"type": "normal", "mean": 0.5, "std dev": 0.2, "seed": 9}]
+    layers = [layer("l%d" % i, "relay", 1, 97 * i + 1, **({"init config": kinds[i % 6]} if kinds[i % 6] else {}))
+              for i in range(35)]
+    sizes = ((1 << 18) + 1, 311_297, 400_001)
+    layers += [layer("big%d" % i, "relay" if i else "rate_encoding", 1, n, **{"init config": kinds[2 + i]})
+               for i, n in enumerate(sizes)]
+    fed = ["l%d" % i for i in (0, 3, 7, 11, 16, 17, 32, 34)] + ["big2"]
+    final = [("neuron", "s", l["name"], k) for l in layers for k in ("input", "output")]
+    case = Case("registers", network(layers, []), 5, 3, final=final,
+                inputs={name: lambda rng, t, k: rng.standard_normal(k) for name in fed})
+    # (tanh may differ in the last bit between the GPU and the host's library)
+    problems = compare(run_library(case, sg), run_oracle(case), tol=1e-6, float_keys=("big0/output",))
+    assert not problems, problems[:3]
