@@ -1256,6 +1256,21 @@ class GameOfLifeModel : public Model {
     static int plane_mode(unsigned mask9) {
         return (mask9 & 0x1EFu) == 0x1EFu ? ((mask9 & 0x10u) ? 2 : 1) : 0;
     }
+    // Strips or tiles for a row that fits a warp.  Ragged widths have no other path but the
+    // per-step word kernel (strips / words: 0.40 / 5.0 us a step at 500 x 333, 0.58 / 33 at
+    // 1500 x 1500, 2.4 / 234 at 4096 x 4095), rows that fill the warp's words no better one.
+    // Other whole words (strips / tiles, 3 to 65,536 rows of 1 to 125 words): strips while
+    // an SM has one band, 6080 rows of the 2 a warp holds (0.46 / 0.58 at 512 x 256, 0.97 /
+    // 1.50 at 4096 x 992), but rows of at most 16 words leave most of the warp idle and the
+    // tiles win beyond (1.60 / 0.99 at 8192 x 256, 2.73 / 2.46 at 16384 x 512, 7.9 / 3.6 at
+    // 65536 x 64), from 4096 rows with at most 8 (0.69 / 0.72 at 4096 x 64, 0.82 / 0.73 at
+    // 6000).  Above 64 words a warp holds 4 rows, whose steps take 0.76 us however few there
+    // are: tiles up to 400 rows (0.76 / 0.58 at 3 x 2304, 1.07 / 1.12 at 1000).
+    static bool strips_win(int rows, int cols) {
+        const int W = cols / 32;
+        if (cols % 32 || W == 32 || W == 64 || W == 128) return true;
+        return W <= 8 ? rows <= 4096 : (W <= 16 ? rows <= 6080 : (W <= 64 || rows > 400));
+    }
     long advance_alone(State& st, LayerState& ls, long n, cudaStream_t s) const override {
         const Layer& l = *ls.layer;
         const ConnState& cs = *st.conn_state(l.inputs[0]);
@@ -1267,12 +1282,7 @@ class GameOfLifeModel : public Model {
         // the B3/S23 rule is its own instance of either kernel
         const int mode = plane_mode(mask9);
         const bool conway = smask == count_mask(2, 3) && bmask == count_mask(3, 3);
-        // Strips wherever a row fits a warp.  Time per step against the tile
-        // kernel (aligned widths): 0.40 / 0.52 us at 500 x 320, 0.58 / 0.92 at
-        // 1500 x 1504, 0.38 / 0.63 at 32 x 32; against the per-step word
-        // kernel, the only other path for ragged widths: 0.40 / 5.0 us at
-        // 500 x 333, 0.58 / 33 at 1500 x 1500, 0.78 / 15 at 300 x 3000.
-        const bool strips = mode != 0 && l.cols <= kStripCols;
+        const bool strips = mode != 0 && l.cols <= kStripCols && strips_win(l.rows, l.cols);
         const int W = (l.cols + 31) / 32, pitch = strips ? strip_pitch(l.cols) : W;
         const long long segs = (long long)l.rows * W;
         long launches = 0;

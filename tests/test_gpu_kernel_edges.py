@@ -594,3 +594,16 @@ def test_input_registers_of_many_and_large_layers(sg):
     # (tanh may differ in the last bit between the GPU and the host's library)
     problems = compare(run_library(case, sg), run_oracle(case), tol=1e-6, float_keys=("big0/output",))
     assert not problems, problems[:3]
+
+
+# whole words, either side of the lines between strips and tiles
+@pytest.mark.parametrize("rows,words", [(4096, 2), (4097, 8), (6080, 9), (6081, 16), (6081, 17), (400, 65), (401, 96),
+                                        (3, 127), (5, 128)])
+def test_gol_whole_runs_by_board(sg, rows, words):
+    cols = 32 * words
+    net = network([layer("b", "game_of_life", rows, cols, survival_min=2, survival_max=3, birth_min=3, birth_max=3)],
+                  [connection("c", "b", "b", "convergent", convolutional=True, **{
+                      "weight config": {"type": "flat", "weight": 1.0, "diagonal": False},
+                      "arborized config": {"field size": 3, "wrap": True}})])
+    board = np.random.default_rng(rows + cols).integers(0, 2**32, rows * cols, dtype=np.uint64).astype(np.uint32)
+    assert_equal(run_both(sg, net, {("b", "output"): board}, 14, [("b", "output"), ("b", "input")]))
