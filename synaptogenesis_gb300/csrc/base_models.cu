@@ -1157,9 +1157,10 @@ class GameOfLifeModel : public Model {
             swap->scratch = true;
             ls.internal["output swap"] = swap;
             const Connection& c = *l.inputs[0];
+            // 2 words a cell where rows are whole words, up to 64 in rows of one cell
             if (c.delay == 0 && c.arbor.wrap && (l.cols % 32 == 0 || l.cols <= kStripCols)) {
                 Array* planes = st.add_array(
-                    "planes", 'u',
+                    "planes", 'u', 0, LAYOUT_PLAIN, 1, 1,
                     (size_t)kPlaneRing * l.rows *
                         (l.cols <= kStripCols ? strip_pitch(l.cols) : l.cols / 32));
                 planes->scratch = true;

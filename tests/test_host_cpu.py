@@ -439,3 +439,26 @@ def test_randomized_divergent_overflow_is_refused(sg):
     n.build_state()
     assert not n.state
     assert "more than 9 sources" in sg.last_error()
+
+
+def test_life_boards_of_one_column_keep_their_size(sg):
+    """A board of 8 million cells in one column takes some 130 MB (words, inputs, the
+    other buffer's words): its bit planes, padded to a word a row, have no host copy."""
+    import subprocess
+    import sys
+    code = """
+import resource, sys
+from synaptogenesis_gb300 import syngen as sg
+sg.set_warnings(False)
+net = sg.Network({"structures": [{"name": "s", "layers": [
+    {"name": "b", "neural model": "game_of_life", "rows": 8_000_000, "columns": 1}]}],
+    "connections": [{"name": "c", "from layer": "b", "to layer": "b", "type": "convergent",
+                     "convolutional": True, "weight config": {"type": "flat", "weight": 1.0, "diagonal": False},
+                     "arborized config": {"field size": 3, "wrap": True}}]})
+before = resource.getrusage(resource.RUSAGE_SELF).ru_maxrss
+net.build_state()
+assert net.state, sg.last_error()
+print(resource.getrusage(resource.RUSAGE_SELF).ru_maxrss - before)
+"""
+    out = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, check=True)
+    assert int(out.stdout) < 400_000, out.stdout           # KiB; 2 GB with the planes
