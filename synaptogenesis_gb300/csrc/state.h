@@ -6,9 +6,9 @@
 // contiguous, src/core/state/weight_matrix.cpp:192-228).  Device copies live in
 // one arena allocation.  Like the reference (state.cpp:259-323), handing out
 // host pointers moves the state to the host, and the next run moves it back --
-// but only the arrays of which a host pointer was ever handed out: no caller can
-// read or change the others.  Once handed out an array always moves, since the
-// caller may keep the pointer.
+// but only the arrays of which a host pointer was ever handed out, by a getter or
+// to a weight or delay callback: no caller can read or change the others.  Once
+// handed out an array always moves, since the caller may keep the pointer.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -42,7 +42,7 @@ struct Array {
     size_t dev_offset = 0;
     bool scratch = false;    // device-only working buffer: never uploaded or downloaded
     bool on_device = false;  // uploaded, and no load() has replaced it since
-    bool exposed = false;    // a getter has handed out its host copy
+    bool exposed = false;    // its host copy has been handed out
 
     float* hf() { return reinterpret_cast<float*>(host.data()); }
     int32_t* hi() { return reinterpret_cast<int32_t*>(host.data()); }

@@ -212,6 +212,9 @@ void init_weights(State& st, ConnState& cs) {
 
     auto& cb = Callbacks::get();
     int id = cfg.get_int("id", 0);
+    // a callback may keep the pointers that it is given, as a getter's caller may
+    for (const char* key : {"callback", "indices callback", "distance callback", "delay callback"})
+        if (cfg.has(key)) cs.weights->exposed = true;
     if (cfg.has("callback"))
         Callbacks::find(cb.weight, cfg.get("callback"), "weight")(id, (int)n, w);
     if (cfg.has("indices callback")) {
@@ -236,6 +239,7 @@ void init_weights(State& st, ConnState& cs) {
             cs.delays = st.add_array("delays", 'i', n, matrix_layout(c), c.matrix_rows, c.matrix_cols);
             for (size_t i = 0; i < n; ++i) cs.delays->hi()[i] = c.delay;
         }
+        cs.delays->exposed = true;
         Callbacks::find(cb.delay, cfg.get("delay callback"), "delay")(id, (int)n, w, cs.delays->hi());
     }
     if (Props* m = cfg.child("circular mask")) circular_mask(c, *m, w);

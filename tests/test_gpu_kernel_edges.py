@@ -607,3 +607,38 @@ def test_gol_whole_runs_by_board(sg, rows, words):
                       "arborized config": {"field size": 3, "wrap": True}})])
     board = np.random.default_rng(rows + cols).integers(0, 2**32, rows * cols, dtype=np.uint64).astype(np.uint32)
     assert_equal(run_both(sg, net, {("b", "output"): board}, 14, [("b", "output"), ("b", "input")]))
+
+
+def test_arrays_kept_by_callbacks_move(sg):
+    """Arrays that a weight and a delay callback kept show what was learned and take
+    what the caller writes, like those of the getters."""
+    kept = {}
+
+    def weights(_, size, data):
+        kept["weights"] = sg.FloatArray(size, data).to_np_array()
+        kept["weights"][:] = np.linspace(0.1, 0.4, size, dtype=np.float32)
+
+    def delays(_, size, __, data):
+        kept["delays"] = sg.IntArray(size, data).to_np_array()
+        kept["delays"][:] = np.arange(size) % 5
+
+    sg.create_weight_callback("kept weights", weights)
+    sg.create_delay_weight_callback("kept delays", delays)
+    net = sg.Network(network(
+        [layer("a", "izhikevich", 6, 6, params="regular", **{"init config": {"type": "flat", "value": 20.0}}),
+         layer("b", "izhikevich", 6, 6, params="regular")],
+        [connection("c", "a", "b", "fully connected", plastic=True, **{
+            "learning rate": 0.1, "weight config": {"type": "flat", "weight": 0.5, "callback": "kept weights",
+                                                    "delay callback": "kept delays"}})]))
+    net.build_state()
+    first = kept["weights"].copy()
+    step = lambda: (net.run({"modules": []}, {"iterations": 20}),                # noqa: E731
+                    net.get_neuron_data("s", "b", "voltage").to_np_array().copy())
+    step()
+    assert not np.array_equal(kept["weights"], first)
+    kept["weights"][:] = 0.25
+    kept["delays"][:] = 3
+    step()
+    assert kept["weights"].max() < first.max()
+    assert np.array_equal(kept["weights"], net.get_weight_matrix("c").to_np_array())
+    assert np.array_equal(net.get_weight_matrix("c", "delays").to_np_array(), np.full(36 * 36, 3))
