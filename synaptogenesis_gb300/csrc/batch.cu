@@ -155,7 +155,7 @@ __device__ __forceinline__ void batch_step_done(const StepArgs& A, long long t) 
 // HBM bounds a batch that fills the GPU, so what counts is bytes in flight: 64
 // instances of 16..128 a side take 2.74 ms a step with 8 slots and 2 CTAs (6.0 TB/s
 // without padding), 2.97 with 16 and 1, 3.43 with 4 and 3, and took 3.41 with 4 slots
-// whose trace stores held back the next loads.  (With no more units than SMs:
+// whose trace stores held back the next loads.  (With few groups:
 // k_batch_step_split.)
 constexpr int kFcUnroll = 8;
 
@@ -281,7 +281,11 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_batch_step(StepArgs A) {
 // bounds the step (500 slots of 18 instructions in one warp, 6 cycles each) and then
 // its neurons' substeps.  12 instances of 16..48 take 29 us a step with 7 + 1 warps,
 // 32 with two groups of 3 + 1 in a CTA, 40 with 15 + 1, and took 41 with a warp a
-// group and 8 groups a CTA.
+// group and 8 groups a CTA.  Against the best tile of k_batch_step (us a step): 23 / 27 for
+// 512 groups of 32 x 32 instances, 37 / 37 for 768, 54 / 46 for 1024; 72 / 111, 109 / 118
+// and 145 / 132 for as many of 64 x 64, 61 / 70 for 768 of 48 x 48; 8.5 / 15.6 for 256
+// groups of 16 x 16, 21 / 15 for 640; 249 / 382 for the 512 of one 128 x 128 instance,
+// 1657 / 1064 for the 1152 of one 192 x 192, one CTA of which fills an SM.
 constexpr int kParts = 7, kPartSlots = 4, kRound = kParts * kPartSlots;
 constexpr int kPartAhead = 4;            // rounds whose loads are in flight
 constexpr int kSplitThreads = (kParts + 1) * 32;
@@ -793,6 +797,25 @@ class Batch {
         }
     }
 
+    // The most dynamic shared memory that `kernel` can be launched with.  The limit is
+    // the function's, shared by every batch of the process: always the largest, or a
+    // smaller batch would lower it for a larger one.
+    size_t allow_shared(void (*kernel)(StepArgs)) {
+        cudaFuncAttributes fa;
+        SG_CUDA(cudaFuncGetAttributes(&fa, kernel));
+        const int most = smem_optin_ - (int)fa.sharedSizeBytes;
+        SG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        return (size_t)most;
+    }
+    // CTAs of k_batch_step_split that the GPU holds, 0 if one does not fit.
+    long long split_places(size_t smem) {
+        if (smem > allow_shared(k_batch_step_split)) return 0;
+        int per_sm = 0;
+        SG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_step_split,
+                                                              kSplitThreads, smem));
+        return (long long)per_sm * num_sms_;
+    }
+
     void set_tile(int tile_rows, int tile_cblocks) {
         if (tile_rows < 1 || tile_cblocks < 1 || tile_rows * tile_cblocks * 32 > kMaxThreads)
             throw SgError("batch: tile must have 1..8 warps");
@@ -807,11 +830,11 @@ class Batch {
         };
         if ((int)shared(tile_rows) > smem_optin_)
             throw SgError("batch: instance too large for shared memory");
-        // no more units than SMs: one for each group, with several warps
-        cudaFuncAttributes fa;
-        SG_CUDA(cudaFuncGetAttributes(&fa, k_batch_step_split));
-        const bool split = (int)units_h_.size() <= num_sms_ &&
-                           (int)(shared(1) + fa.sharedSizeBytes) <= smem_optin_;
+        // several warps to a group, whatever the tile, up to three groups for each CTA that
+        // the GPU holds (two to an SM, fewer beside large instances), two where a group's
+        // slots are so few that a CTA's start outweighs them: k_batch_step_split
+        const int rounds = slot_rows_ >= 128 * n_groups_ ? 3 : 2;
+        const bool split = n_groups_ <= rounds * split_places(shared(1));
         if (split) {
             unit_rows_ = unit_cblocks_ = 1;
             make_units();
@@ -827,11 +850,7 @@ class Batch {
         SG_CUDA(cudaMemcpyAsync(d_units_, units_h_.data(), units_h_.size() * sizeof(Unit),
                                 cudaMemcpyHostToDevice, stream_));
         kernel_ = split ? k_batch_step_split : k_batch_step;
-        // the limit is the function's, shared by every batch of the process:
-        // always the largest, or a smaller batch would lower it for a larger one
-        SG_CUDA(cudaFuncGetAttributes(&fa, kernel_));
-        SG_CUDA(cudaFuncSetAttribute(kernel_, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     smem_optin_ - (int)fa.sharedSizeBytes));
+        allow_shared(kernel_);
         int per_sm = 0;
         SG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel_, threads_, smem_));
         if (per_sm < 1) throw SgError("batch: step kernel does not fit on an SM");

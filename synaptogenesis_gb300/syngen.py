@@ -553,7 +553,8 @@ class Batch:
     """Many independent Izhikevich instances advanced together (sg_batch_* in
     include/syngen.h).  ``instances`` is a sequence of dicts with the fields of
     ``BatchInstance``; ``tile`` = (rows, colblocks) fixes the step kernel's work
-    unit, None lets the autotuner choose."""
+    unit, None lets the autotuner choose.  Batches of few groups of 32 neurons take
+    a kernel whose unit is one group, whatever the tile."""
 
     def __init__(self, instances, tile=None):
         n = len(instances)

@@ -642,3 +642,29 @@ def test_arrays_kept_by_callbacks_move(sg):
     assert kept["weights"].max() < first.max()
     assert np.array_equal(kept["weights"], net.get_weight_matrix("c").to_np_array())
     assert np.array_equal(net.get_weight_matrix("c", "delays").to_np_array(), np.full(36 * 36, 3))
+
+
+# one form for a batch's number of groups, whatever the tile: 912 groups are three for
+# each CTA of several warps to a group that 152 SMs hold, 608 two (16 x 16, whose groups
+# have few slots), 456 three where an instance takes an SM
+@pytest.mark.parametrize("sides,split", [([(64, 64)] * 7 + [(8, 64)], True), ([(64, 64)] * 7 + [(9, 64)], False),
+                                         ([(128, 128)], True), ([(192, 192)], False), ([(16, 16)] * 38, True),
+                                         ([(16, 16)] * 39, False)])
+def test_batch_form_by_groups(sg, sides, split):
+    from synaptogenesis_gb300 import batching
+    insts = [batching.instance(r, 7 + i, rows=r, cols=c) for i, (r, c) in enumerate(sides)]
+    seen, first = set(), None
+    for tile in ((1, 1), (2, 2), (8, 1)):
+        with sg.Batch(insts, tile=tile) as b:
+            b.step(5)
+            words = np.concatenate([b.read(i, "output") for i in range(len(insts))])
+            report = b.report().properties
+        assert (report["units"] == report["groups"] and int(report["threads"]) == 256) == split, (tile, report)
+        first = words if first is None else first
+        assert np.array_equal(words, first)
+    # and the other form, beside enough others, gives the same
+    more = [batching.instance(96, 300 + i) for i in range(24)]
+    with sg.Batch(insts + more, tile=(2, 1)) as b:
+        b.step(5)
+        assert int(b.report().properties["threads"]) == 64
+        assert np.array_equal(np.concatenate([b.read(i, "output") for i in range(len(insts))]), first)
