@@ -119,7 +119,7 @@ constexpr float kBound5 = 1.136868377216160297e-13f;  // 2^-43
 // The rounding test of single-argument expressions, whose every float operand has
 // been compared with the double evaluation (tests/test_spnet_ff_cpu.py): hi + lo
 // with lo 2^-16 larger and smaller rounds to the same float.  Three operations
-// where rounds_to takes a dozen; rejects one operand in 30,000, and what is not
+// where rounds_to takes six; rejects one operand in 30,000, and what is not
 // finite.
 SG_FF bool decided(float hi, float lo, float& out) {
     out = fma(lo, 1.0000152587890625f, hi);
@@ -351,7 +351,8 @@ SG_FF bool short_term_w(float sw, bool spike, float& out) {
 // most u^2 (11 |P| + 10 S), P = 0.04 v v and S the largest partial sum, and
 // the reference's double roundings by less than 2^-53 (2 |P| + 5 S); the
 // bound used is 2^-43 (|P| + S), a factor of 2.9 above their sum.
-// iz_delta_v_sum gives the value as f + g, f = RN(f + g), and the bound.
+// iz_delta_v_sum gives the value as f + g, f = RN(f + g), and the bound; iz_delta_v
+// says whether f is the derivative's float.
 SG_FF void iz_delta_v_sum(float v, float recovery, float current, float& f, float& g, float& B) {
     constexpr double C = 0.04;
     constexpr float C1 = (float)C;
@@ -380,10 +381,14 @@ SG_FF void iz_delta_v_sum(float v, float recovery, float current, float& f, floa
     B = mul(add(absf(h2), smax), kBound5);
 }
 
+SG_FF bool iz_delta_v(float v, float recovery, float current, float& f, float& g, float& B) {
+    iz_delta_v_sum(v, recovery, current, f, g, B);
+    return rounds_to(f, g, B);
+}
+
 SG_FF bool iz_delta_v(float v, float recovery, float current, float& out) {
     float f, g, B;
-    iz_delta_v_sum(v, recovery, current, f, g, B);
-    if (!rounds_to(f, g, B)) return false;
+    if (!iz_delta_v(v, recovery, current, f, g, B)) return false;
     out = f;
     return true;
 }
@@ -473,16 +478,21 @@ SG_FF bool spnet_dw(float x, float p, float q, float& out) {
     return true;
 }
 
-// The voltage where the derivative's rounding test failed, which is where it is
-// small (a neuron near rest: the terms cancel, and the float nearest the sum is not
-// known).  Its float is within B of f + g, give or take its own rounding, and that
-// decides the voltage unless the step ends next to a rounding boundary: those are
-// 2^-24 |v| apart, the uncertainty 2^-43 of the cancelled terms.  Only a step past
-// the threshold needs the derivative itself.
+// The voltage from the derivative f + g (bound B) of iz_delta_v, `known` its answer.
+// Where it is not known, the derivative is small (a neuron near rest: the terms cancel,
+// and the float nearest the sum is not known).  Its float is within B of f + g, give or
+// take its own rounding, and that decides the voltage unless the step ends next to a
+// rounding boundary: those are 2^-24 |v| apart, the uncertainty 2^-43 of the cancelled
+// terms.  Only a step past the threshold needs the derivative itself.
 constexpr float kHalfUlp = 5.9604701e-8f;                 // a little above 2^-24
 
+SG_FF bool spnet_voltage_of(float v, float f, float g, float B, bool known, float& out) {
+    const float err = known ? 0.0f : add(B, mul(absf(f), kHalfUlp));
+    return spnet_voltage(v, f, out, known ? 0.0f : g, err) && (known || out <= 30.0f);
+}
+
 SG_FF bool spnet_voltage_near(float v, float f, float g, float B, float& out) {
-    return spnet_voltage(v, f, out, g, add(B, mul(absf(f), kHalfUlp))) && !(out > 30.0f);
+    return spnet_voltage_of(v, f, g, B, false, out);
 }
 
 // The same for iz_voltage: the Izhikevich drive is (delta_v + x) + y in float, x =
@@ -495,6 +505,16 @@ SG_FF void iz_drive_near(float f, float x, float y, float B, float& drive, float
     tail = add(tail, add(e, e2));
     // twice the roundings: the tail's own are far below
     err = add(B, mul(add(absf(f), add(absf(s), absf(drive))), 2.0f * kHalfUlp));
+}
+
+SG_FF bool iz_voltage_of(float v, float f, float g, float B, bool known, float x, float y, float d1,
+                         float d2, float rd, float& out) {
+    float drive = add(add(f, x), y), tail = 0.0f, err = 0.0f;
+    if (!known) {
+        tail = g;
+        iz_drive_near(f, x, y, B, drive, tail, err);
+    }
+    return iz_voltage(v, drive, d1, d2, rd, out, tail, err) && (known || out <= 30.0f);
 }
 
 // Recovery time constant of the substep that crosses the threshold

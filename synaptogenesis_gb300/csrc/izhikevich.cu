@@ -1391,14 +1391,6 @@ static void spnet_windows(State& st, ConnState& cs) {
     cs.sparse_packed->scratch = true;
 }
 
-// The substep's double expressions in double, where a rounding test fails.
-static __device__ __noinline__ float spnet_delta_double(float voltage, float recovery, float current) {
-    return (0.04 * voltage * voltage) + (5 * voltage) + 140 - recovery + current;
-}
-static __device__ __noinline__ float spnet_voltage_double(float voltage, float delta_v) {
-    return voltage + delta_v * 0.1;
-}
-
 // Neuron update (spnet_attributes.cpp:96-166), the layers of a step in one
 // launch: the double expressions in float-float with rounding tests.  FP64 bounds
 // it otherwise: 65,536 and 16,384 neurons took 21.5 us a launch in double, in two
@@ -1432,24 +1424,7 @@ __global__ void __launch_bounds__(256) k_spnet_update(SpnetUpdateGroup G) {
     wait_for_previous();
     if (blockIdx.x * blockDim.x + threadIdx.x >= G.start[G.n]) return;
     const float current = A.in[nid];
-    for (int i = 0; (i < 10) && (voltage < 30.0f); ++i) {
-        float delta_v, tail, bound, nv;
-        ff::iz_delta_v_sum(voltage, recovery, current, delta_v, tail, bound);
-        const bool known = ff::rounds_to(delta_v, tail, bound);
-        const float err = known ? 0.0f : ff::add(bound, ff::mul(fabsf(delta_v), ff::kHalfUlp));
-        if (!ff::spnet_voltage(voltage, delta_v, nv, known ? 0.0f : tail, err) ||
-            !(known || nv <= 30.0f)) {
-            if (!known) delta_v = spnet_delta_double(voltage, recovery, current);
-            nv = spnet_voltage_double(voltage, delta_v);
-        }
-        const float v0 = voltage, r0 = recovery;
-        voltage = (nv != nv) ? 30.0f : nv;
-        float adjusted_tau = (float)0.1;
-        if (voltage > 30.0f && !ff::iz_adjusted_tau(voltage, delta_v, adjusted_tau))
-            adjusted_tau = iz_tau_double(voltage, delta_v);
-        recovery += a * adjusted_tau * ((b * voltage) - recovery);
-        if (voltage == v0 && recovery == r0) break;          // at rest
-    }
+    spnet_integrate_ff(voltage, recovery, current, a, b);
     const uint32_t spike = voltage >= 30.0f;
     const uint32_t prev_bit = shift_bits(A.spikes, A.size, A.history, nid, spike);
     float np;
