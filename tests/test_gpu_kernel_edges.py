@@ -668,3 +668,40 @@ def test_batch_form_by_groups(sg, sides, split):
         b.step(5)
         assert int(b.report().properties["threads"]) == 64
         assert np.array_equal(np.concatenate([b.read(i, "output") for i in range(len(insts))]), first)
+
+
+# several segments of the backward pass and chunks of the forward one, the last of them
+# short: networks whose steps are too large for one segment (5 to 10 steps of 64 MB), for
+# every field, rows copied by 4 floats and one at a time, one row a thread and more
+@pytest.mark.parametrize("cfg", [
+    dict(layers=3, rows=300, cols=333, field=1, outputs=16, batch=2, steps=30),
+    dict(layers=2, rows=333, cols=301, field=3, outputs=16, batch=2, steps=21),
+    dict(layers=2, rows=250, cols=300, field=3, outputs=16, batch=1, steps=33),
+    dict(layers=2, rows=140, cols=255, field=5, outputs=16, batch=1, steps=40),
+    dict(layers=2, rows=140, cols=252, field=5, outputs=16, batch=1, steps=41),
+    dict(layers=2, rows=201, cols=255, field=5, outputs=16, batch=1, steps=31),
+    dict(layers=2, rows=170, cols=225, field=7, outputs=4, batch=1, steps=31),
+    dict(layers=2, rows=120, cols=224, field=7, outputs=4, batch=1, steps=45),
+    dict(layers=2, rows=101, cols=203, field=9, outputs=3, batch=1, steps=40),
+    dict(layers=2, rows=104, cols=200, field=9, outputs=3, batch=1, steps=43)],
+    ids=lambda c: "%(rows)dx%(cols)d-field%(field)d" % c)
+def test_rate_segments(cfg):
+    """Loss and gradients against the FP64 restatement, and bit for bit the same with
+    the smallest segments, somewhat larger ones and a single one."""
+    import torch
+    from oracle import rate_adjoint as ra
+    from synaptogenesis_gb300 import syngen
+    from tests.test_gpu_rate import close, gpu_grads, make
+    p = make(17, *(cfg[k] for k in ("layers", "rows", "cols", "field", "outputs", "batch", "steps")))
+    nets = [syngen.RateNetwork(checkpoint=k, **cfg) for k in (1, 13, cfg["steps"])]
+    assert len({net.workspace_bytes for net in nets}) == 3        # segments of three lengths
+    results = [gpu_grads(torch, syngen, net, p) for net in nets]
+    for other in results[1:]:
+        for a, b in zip(other, results[0]):
+            assert np.array_equal(np.asarray(a), np.asarray(b))
+    want = ra.adjoint(dict(cfg, checkpoint=1, dt=1.0), p["x"], p["weights"], p["readout"], p["tau"],
+                      p["target"])
+    assert abs(results[0][0] - want[0]) <= 1e-5 * abs(want[0])
+    for got, w in zip(results[0][1:], want[1:]):
+        ok, norm = close(got, w)
+        assert ok, norm
