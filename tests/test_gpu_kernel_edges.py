@@ -705,3 +705,21 @@ def test_rate_segments(cfg):
     for got, w in zip(results[0][1:], want[1:]):
         ok, norm = close(got, w)
         assert ok, norm
+
+
+def test_spnet_groups_of_layers_and_connections(sg):
+    """Eleven spnet layers and connections: neuron updates and time-since-spike updates go
+    in launches of eight, of sizes that share blocks."""
+    n = 11
+    layers = [layer("n%d" % i, "spnet", 1, 23 + 61 * i % 257, params="fast" if i % 3 else "regular", **{
+        "init config": {"type": "poisson", "rate": 150, "value": 25, "seed": 40 + i}}) for i in range(n)]
+    conns = [connection("c%d" % i, "n%d" % i, "n%d" % ((i * 4 + 1) % n), "fully connected",
+                        opcode="sub" if i % 4 == 3 else "add", plastic=True, sparse=i % 2 == 0,
+                        **{"weight config": {"type": "flat", "weight": 0.5 + 0.1 * i}, "delay": i})
+             for i in range(n)]
+    keys = [("n%d" % i, k) for i in range(n) for k in ("voltage", "recovery", "output", "post trace",
+                                                       "time since spike")]
+    keys += [("matrix", "c%d" % i, k) for i in range(n) for k in ("weights", "time since spike")]
+    results = run_both(sg, network(layers, conns), {}, 45, keys, learning=True)
+    assert_equal(results)
+    assert all((results[("n%d" % i, "output")][1] != 0).any() for i in range(n))
