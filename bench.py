@@ -89,7 +89,6 @@ def gol_workload(side=2048):
         "timestep_bytes": 3 * n // 8,
         "word_layout_timestep_bytes": 8 * n,
         "bytes_per_launch": GOL_STEPS_PER_LAUNCH * 3 * n // 8,
-        "state_bytes": 8 * n + 36,           # input + output + weights moved per e2e step
         "cpu_seconds": 12.0,
         "learning": False,
     }
@@ -175,7 +174,6 @@ def iz_plastic_workload():
         # delays from a byte copy (21 and 29 B per synapse)
         "moved_bytes": {"izhikevich.activate.subset": 21 * sub,
                         "izhikevich.activate.convergent": 29 * conv},
-        "state_bytes": None,                            # taken from the run report
         "cpu_seconds": 15.0,
         "learning": True,
     }
@@ -218,7 +216,6 @@ def iz_c0_workload():
         # array, delays as bytes
         "moved_bytes": {"izhikevich.activate.fully connected": 21 * fc},
         "l2_note": "34 MB per timestep: L2-resident within a bench step; flushed between steps",
-        "state_bytes": None,
         "cpu_seconds": 10.0,
         "learning": False,
     }
@@ -286,7 +283,6 @@ def spnet_sparse_workload(side=256):
         "kernel": "spnet.learn.sparse",
         "bytes_per_launch": None,                       # w, presyn trace, dw r+w, source index
         "bytes_per_timestep": None,
-        "state_bytes": None,
         "cpu_seconds": 8.0,
         "learning": True,
     })
@@ -659,17 +655,18 @@ def run_gb300(args, rank, world, local):
     # -- end to end through the public API with host buffers ----------------
     env = sg.Environment({"modules": []})
     wl["result"](net)                                      # state now lives on the host
-    state_bytes = wl["state_bytes"] or int(rep1.properties["state bytes"])
     e2e_steps = max(1, min(args.steps, 3))
 
     def e2e_step():
-        rep = net.run(env, dict(run_args, iterations=T))      # H2D of the state, then T timesteps
+        # H2D of the arrays that were handed out, then T timesteps
+        rep = net.run(env, dict(run_args, iterations=T))
         assert rep.obj is not None, sg.last_error()
-        res = wl["result"](net)                               # D2H of the state
+        res = wl["result"](net)                               # D2H of the same arrays
         _ = int(res.view("uint32")[0])
+        return int(rep.properties["moved bytes"])
 
     for _ in range(max(1, min(args.warmup, 2))):              # untimed, like the device leg
-        e2e_step()
+        e2e_bytes = e2e_step()
     t0 = time.perf_counter()
     for _ in range(e2e_steps):
         e2e_step()
@@ -683,7 +680,7 @@ def run_gb300(args, rank, world, local):
         "dev_s": dev_max, "units": units * world, "wall_s": t_wall, "launches": launches,
         "mean_us": mean_us, "profiled_us": profiled_us, "clocks": clk, "kernels": kern,
         "e2e_value": wl["units_per_timestep"] * T * e2e_steps * world / e2e_max,
-        "e2e_steps": e2e_steps, "wl": wl, "T": T, "state_bytes": state_bytes,
+        "e2e_steps": e2e_steps, "wl": wl, "T": T, "e2e_bytes": e2e_bytes,
     }
     return out
 
@@ -1111,7 +1108,7 @@ def main():
         "roofline": roofline,
         "cpu_baseline": cb,
         "e2e": {"value": r["e2e_value"], "unit": wl["unit"],
-                "h2d_bytes_per_step": r["state_bytes"], "d2h_bytes_per_step": r["state_bytes"],
+                "h2d_bytes_per_step": r["e2e_bytes"], "d2h_bytes_per_step": r["e2e_bytes"],
                 "steps": r["e2e_steps"]},
         "clocks": r["clocks"],
         "gpu_launches": r["launches"],

@@ -202,6 +202,13 @@ size_t State::host_bytes() const {
     return n;
 }
 
+size_t State::moved_bytes() const {
+    size_t n = 0;
+    for (auto& a : arrays_)
+        if (!a->scratch && a->exposed) n += std::min(a->count, a->dev_count) * 4;
+    return n;
+}
+
 void State::allocate_device() {
     size_t off = 0;
     for (auto& a : arrays_) {

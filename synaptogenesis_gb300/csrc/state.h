@@ -158,7 +158,8 @@ class State {
         return ls->output->du() + (size_t)word * l->size;
     }
     size_t device_bytes() const { return arena_bytes_; }
-    size_t host_bytes() const;
+    size_t host_bytes() const;               // every array with a host mirror
+    size_t moved_bytes() const;              // those handed out: an upload or download
 
     // Save / load in the reference's record format (state.cpp:365-447).
     void save(const std::string& path);

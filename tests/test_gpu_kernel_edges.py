@@ -723,3 +723,20 @@ def test_spnet_groups_of_layers_and_connections(sg):
     results = run_both(sg, network(layers, conns), {}, 45, keys, learning=True)
     assert_equal(results)
     assert all((results[("n%d" % i, "output")][1] != 0).any() for i in range(n))
+
+
+def test_report_of_moved_bytes(sg):
+    """The bytes that a run moves each way: those of the arrays handed out so far."""
+    net = sg.Network(network([layer("a", "relay", 5, 7), layer("b", "izhikevich", 3, 7, params="regular")],
+                             [connection("c", "a", "b", "fully connected")]))
+    net.build_state()
+
+    def moved():
+        return int(net.run({"modules": []}, {"iterations": 2}).properties["moved bytes"])
+
+    assert moved() == 0
+    net.get_neuron_data("s", "b", "voltage")
+    assert moved() == 4 * 21
+    net.get_neuron_data("s", "b", "voltage")
+    net.get_weight_matrix("c")
+    assert moved() == 4 * (21 + 35 * 21)
