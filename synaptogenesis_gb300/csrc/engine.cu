@@ -79,7 +79,8 @@ struct InputGroup {
 //
 // A thread sets one neuron's register, eight in layers of more than kInputFew, where what
 // a block costs to start outweighs its work: a layer of 4 million neurons took 15 us with
-// 256 neurons to a block, 4.2 with 2048.
+// 256 neurons to a block, 4.2 with 2048.  Steps without such a layer have their own
+// instance (0.6 us less of the 256 x 256 spnet network's 88).
 constexpr int kInputFew = 1 << 18;
 
 // One neuron's register at step t.
@@ -110,13 +111,15 @@ __device__ __forceinline__ void init_input(const InputArgs& A, unsigned long lon
     }
 }
 
+template <bool LARGE>
 __global__ void __launch_bounds__(256) k_init_inputs(InputGroup G) {
     wait_for_previous();
     __shared__ unsigned long long step;
     int c = 0;
     while (c + 1 < G.n && (int)blockIdx.x >= G.start[c + 1]) ++c;
     const InputArgs& A = G.C[c];
-    const int i0 = (int)(blockIdx.x - G.start[c]) * 256 * A.per + threadIdx.x;
+    const int per = LARGE ? A.per : 1;
+    const int i0 = (int)(blockIdx.x - G.start[c]) * 256 * per + threadIdx.x;
     const bool noise = A.kind < 3;
     unsigned long long counted = 0;
     if (noise) {
@@ -125,11 +128,11 @@ __global__ void __launch_bounds__(256) k_init_inputs(InputGroup G) {
         if (threadIdx.x == 0) counted = atomicAdd(A.ctr + 1, 1ull) + 1;
     }
     const unsigned long long t = noise ? step : 0;
-    if (A.per == 1) {
+    if (!LARGE) {
         if (i0 < A.n) init_input(A, t, i0);
     } else {
 #pragma unroll 8
-        for (int i = i0; i < min(A.n, i0 + 256 * A.per); i += 256) init_input(A, t, i);
+        for (int i = i0; i < min(A.n, i0 + 256 * per); i += 256) init_input(A, t, i);
     }
     if (counted == (unsigned long long)(G.start[c + 1] - G.start[c])) {
         A.ctr[0] = t + 1;
@@ -345,7 +348,10 @@ void Engine::enqueue_step(bool last) {
     auto flush = [&] {
         if (group.n == 0) return;
         timed("init", 1, [&] {
-            launch_dependent(k_init_inputs, group.start[group.n], 256, 0, stream_, group);
+            bool large = false;
+            for (int i = 0; i < group.n; ++i) large = large || group.C[i].per > 1;
+            launch_dependent(large ? k_init_inputs<true> : k_init_inputs<false>,
+                             group.start[group.n], 256, 0, stream_, group);
             SG_LAUNCH_CHECK();
         });
         ++launches_;
