@@ -341,6 +341,17 @@ void Engine::timed(const std::string& name, long kernels, F&& f) {
     p.launches += kernels;
 }
 
+// Kernels that load before they wait for the kernel before them (launch.cuh) rest on this
+// order.  The activators of trace models and sparse spnet connections load what learning
+// writes (weights, traces, short-term variables).  On one stream k_init_inputs stands
+// between: a layer of these models always has registers to set (none of them fuses an
+// input).  Where learning runs on the side stream, k_init_inputs does not follow it, and
+// what stands between is the connection's own time-since-spike kernel: a connection whose
+// learning is pending is left out of the prologue, so that activate() launches that kernel
+// after the wait for learn_ev_ and before the activator.  The neuron updates load their own
+// variables, which the last step's update wrote, with the registers and activations
+// between; the learning kernels load what activation and they themselves write, with the
+// updates between.
 void Engine::enqueue_step(bool last) {
     StepCtx ctx{stream_, last, &layer_io_, &launches_};
     // 1. input registers
@@ -498,7 +509,8 @@ void Engine::enqueue_step(bool last) {
     std::vector<Layer*> deferred;
     {
         // prologues of the connections whose activation waits on nothing,
-        // grouped by the model of their destination layer
+        // grouped by the model of their destination layer (pending ones keep
+        // their own, which their activators rely on: see above)
         std::vector<std::pair<const Model*, std::vector<ConnState*>>> pro;
         for (auto& lp : net_->layers) {
             const Model* m = find_model(lp->model);

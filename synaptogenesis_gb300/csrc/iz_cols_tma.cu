@@ -467,8 +467,9 @@ __global__ void __launch_bounds__(kSmallProducers + 32) k_iz_cols_small(
             }
             asm volatile("bar.arrive %0, %1;" ::"r"(1 + ch), "n"(kSmallProducers + 32) : "memory");
         };
-        // the synapses' variables are this kernel's and the learning one's, which the
-        // setting of the registers at least has followed: before the wait
+        // the synapses' variables are this kernel's and the learning one's, after which
+        // the registers or the times since spike at least are set: before the wait
+        // (Engine::enqueue_step)
         load(0, v[0]);
         load(1, v[1]);
         wait_for_previous();

@@ -308,8 +308,9 @@ __global__ void __launch_bounds__(256, 5) k_iz_activate_conv_tile(
             }
         }
     };
-    // the synapses' variables are this kernel's and the learning one's, which the
-    // setting of the registers at least has followed: before the wait
+    // the synapses' variables are this kernel's and the learning one's, after which the
+    // registers or the times since spike at least are set: before the wait
+    // (Engine::enqueue_step)
     load(warp);
     wait_for_previous();
     const uint32_t* words = after_wait(src);
@@ -1336,8 +1337,8 @@ __global__ void __launch_bounds__(kWindowDests) k_spnet_activate_window(
             }
         }
     };
-    // the words do not change, the weights with learning, which the setting of the
-    // registers at least has followed: before the wait
+    // the words do not change, the weights with learning, after which the registers or
+    // the times since spike at least are set: before the wait (Engine::enqueue_step)
     load(0, 0);
     load(1, kSpnetAhead);
     wait_for_previous();

@@ -23,8 +23,11 @@ __device__ __forceinline__ void wait_for_previous() {
 // p for loads after the wait that the compiler is not to move before it (read-only
 // ones, which no memory clobber holds), in kernels that load anything before it.
 // What may be loaded before it is what the kernel before does not write: the one
-// before that has completed, since the kernel before waited for it before it let
-// this one be launched.
+// before that has completed, its writes included, since the kernel before waited for
+// it before it let this one be launched.  So a kernel may load early what another one
+// writes only if a kernel that waits stands between the two in its stream, or an event
+// wait followed by such a kernel where the other one runs in another stream.  Nothing
+// checks that: Engine::enqueue_step says where its order provides it.
 template <class T>
 __device__ __forceinline__ T* after_wait(T* p) {
     asm volatile("" : "+l"(p));
