@@ -307,16 +307,6 @@ void launch_dendrite_fold(int n, float* src, float* dst, int opcode, float trail
     SG_LAUNCH_CHECK();
 }
 
-static int num_sms() {
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        SG_CUDA(cudaGetDevice(&dev));
-        SG_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
-        return n;
-    }();
-    return sms;
-}
-
 // relay_attributes.cpp:10-18 (the ramp is std::fmax on doubles, i.e. fmax)
 __global__ void k_relay(int size, int history, const float* __restrict__ in, float* out, int ramp) {
     wait_for_previous();
@@ -944,8 +934,7 @@ __global__ void __launch_bounds__(strip_max_warps(R) * 32) k_gol_strips_steps(
     // launched as a programmatic dependent of the previous advance: nothing
     // global is read before it has completed; the next advance may be
     // scheduled from here on
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    wait_for_previous();
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
         if (e == 0 ? warp != 0 : warp != nw - 1) continue;
@@ -1223,21 +1212,8 @@ class GameOfLifeModel : public Model {
             const int nw = (ty + 2 * K + rpw - 1) / rpw;
             const int grid = (rows + ty - 1) / ty;
             const size_t smem = strip_smem_bytes(nw, rpw, wpl);
-            // programmatic dependent launch: each launch may be scheduled
-            // while the previous one drains; it waits for it to complete
-            // (griddepcontrol.wait) before touching the planes
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)grid);
-            cfg.blockDim = dim3((unsigned)(nw * 32));
-            cfg.dynamicSmemBytes = smem;
-            cfg.stream = s;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[0].val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            SG_CUDA(cudaLaunchKernelEx(&cfg, kernel, rows, cols, ty, (long long)T, K, planes, smask,
-                                       bmask));
+            launch_dependent(kernel, (unsigned)grid, (unsigned)(nw * 32), smem, s, rows, cols, ty,
+                             (long long)T, K, planes, smask, bmask);
             ++launches;
             T += K;
         }

@@ -607,7 +607,7 @@ struct IzUpdateGroup {
 // A neuron is a chain of dependent substeps, so few neurons are spread a warp to a
 // CTA (a warp to a scheduler) before warps share one.
 static int update_threads(int neurons) {
-    return neurons <= 152 * 4 * 32 ? 32 : 128;
+    return neurons <= num_sms() * 4 * 32 ? 32 : 128;
 }
 
 __global__ void __launch_bounds__(256) k_iz_update(IzUpdateGroup G) {

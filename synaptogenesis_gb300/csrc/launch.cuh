@@ -34,6 +34,17 @@ __device__ __forceinline__ T* after_wait(T* p) {
     return p;
 }
 
+// SMs of the device, for rules on how many CTAs it holds.
+inline int num_sms() {
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        SG_CUDA(cudaGetDevice(&dev));
+        SG_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+        return n;
+    }();
+    return sms;
+}
+
 template <class... P, class... A>
 void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                       A&&... args) {

@@ -964,7 +964,7 @@ void launch(void (*kernel)(P...), dim3 grid, int threads, cudaStream_t st, A... 
 // one, and the others stay empty: up to 8 CTAs to an SM wait for the launch before
 // (3 x 64x16, field 3, batch 256: 0.71 ms a training step, 1.28 as dependents; 6 x 16x16,
 // batch 256: 0.79 and 1.30; 2 x 256x256, batch 4, 9 CTAs to an SM: 0.44 and 0.43).
-bool crowds(const dim3& grid) { return (long long)grid.x * grid.y * grid.z <= 8 * 152; }
+bool crowds(const dim3& grid) { return (long long)grid.x * grid.y * grid.z <= 8 * num_sms(); }
 
 void transpose_weights(const Dims& D, const float* w, const Work& W, cudaStream_t st) {
     if (D.L < 2) return;
@@ -978,7 +978,7 @@ unsigned tiles(const Dims& D, int py) {
     const int ty = py * kTileWarps;
     return (unsigned)(((D.rows + ty - 1) / ty) * ((D.cols + 31) / 32));
 }
-bool wide(const Dims& D, long long per_tile) { return tiles(D, tile_py(D.field)) * per_tile >= 152; }
+bool wide(const Dims& D, long long per_tile) { return tiles(D, tile_py(D.field)) * per_tile >= num_sms(); }
 
 // Pieces of 4 floats need rows that start on 16 bytes.
 #define SG_RATE_TILE_V(D_, WIDE, VV, CALL)                                                 \
@@ -1001,7 +1001,7 @@ bool wide(const Dims& D, long long per_tile) { return tiles(D, tile_py(D.field))
 // but a CTA for each of the 5 or more that an SM can hold comes first (3 x 64x64,
 // batch 64: 1.85 ms with one element to a CTA, 2.11 with two).
 int batch_group(const Dims& D, unsigned ntiles) {
-    return (int)std::max<long long>(1, (long long)ntiles * D.B / (5 * 152));
+    return (int)std::max<long long>(1, (long long)ntiles * D.B / (5 * num_sms()));
 }
 
 // Layer l through the steps c + 1 .. c + nt.
@@ -1042,7 +1042,7 @@ void forward(const Dims& D, const float* x, const float* w, const float* wo, con
         launch(W.aligned && D.N % 4 == 0 ? k_rate_readout<4> : k_rate_readout<1>,
                dim3((unsigned)((rows + kReadRows - 1) / kReadRows)), kBlock, st, D, c, nt,
                buf[(D.L - 1) & 1], D.BN, wo, target, W.y, W.loss_tb);
-        }
+    }
     launch(k_rate_loss, dim3(1), 256, st, D, W.loss_tb, loss);
     if (y_out)
         SG_CUDA(cudaMemcpyAsync(y_out, W.y, (size_t)D.T * D.B * D.O * sizeof(float),
@@ -1098,7 +1098,7 @@ void backward(const Dims& D, const float* x, const float* w, const float* wo, co
                     launch(k_rate_adjoint<F, PY, V>, grid, kTileThreads, st, D, l, A, W.wt, tau);
                 }));
             }
-                }
+        }
         if (D.L > 1) {
             SG_RATE_TILE(D, W, wide(D, (long long)(D.L - 1) * nt), ({
                 const dim3 grid(tiles(D, PY), (unsigned)(D.L - 1), (unsigned)nt);
@@ -1109,13 +1109,13 @@ void backward(const Dims& D, const float* x, const float* w, const float* wo, co
                     launch(k_rate_dw<F, PY, V>, grid, kTileThreads, st, D, W.seg_P, W.seg_r, W.grad_part);
                 }
             }));
-                }
+        }
         const int dwo_v = W.aligned && D.N % 4 == 0 ? 4 : 1, per = kReadoutThreads * dwo_v;
         launch(dwo_v == 4 ? k_rate_dwo<4> : k_rate_dwo<1>,
                dim3((unsigned)((D.N + per - 1) / per), (unsigned)nt), kReadoutThreads, st, D,
                W.gy + (long long)c * D.B * D.O, W.seg_r, W.grad_part + weights);
         launch(k_rate_acc, dim3(grid_of(D.G)), 256, st, D, nt, first, W.grad_part, W.grad);
-        }
+    }
     launch(k_rate_out, dim3(grid_of(D.G)), 256, st, D, W.grad, dw, dwo);
     launch(k_rate_dtau_partial, dim3(kTauBlocks, D.L), 256, st, D, W.lamd, W.tau_part);
     launch(k_rate_dtau_final, dim3((unsigned)((D.L + 255) / 256)), 256, st, D, tau, W.tau_part, dtau);
