@@ -43,7 +43,7 @@
 // registers.  The adjoint runs the same way from the last layer down.  Before, a
 // tile's layers ran step by step in one CTA with a barrier per step, recomputing
 // halos, and the adjoint took a launch per step: forward and adjoint of 3 x 64x64
-// layers, field 5, batch 64, 100 steps took 4.55 ms; 1.76 ms like this (4 x 30x45,
+// layers, field 5, batch 64, 100 steps took 4.55 ms; 1.83 ms like this (4 x 30x45,
 // batch 5, 37 steps: 0.56 and 0.34 ms).
 //
 // Layout on the device: the convergent weights are transposed once per call
@@ -104,10 +104,12 @@ __global__ void k_rate_transpose(Dims D, const float* __restrict__ w, float* __r
 // window rows it reads serve F x F terms of every one of them: (PY + F - 1) F
 // shared-memory reads for PY F F multiply-adds (0.6 per term at 5 x 5 and
 // PY = 2, where a neuron a thread needs 1).  Instruction issue is what bounds
-// these kernels, at half its rate for want of warps: at 5 x 5, two rows (72
+// these kernels, at half to 0.7 of its rate for want of warps: at 5 x 5, two rows (72
 // registers, 7 CTAs an SM) took 13.9 us a 10-step launch where four (151, 3 CTAs)
-// took 20.1, though four issue fewer instructions.  Everything else in the loop over items (batch element, timestep) is
-// kept short: offsets within a layer are 32-bit and worked out once, added to
+// took 20.1, though four issue fewer instructions (15.8 us with two rows since each
+// kernel row is summed by itself and the sigmoid's reciprocal is correctly rounded).
+// Everything else in the loop over items (batch element, timestep) is kept short:
+// offsets within a layer are 32-bit and worked out once, added to
 // bases that are the same for the whole CTA; windows (tile plus halo) come in
 // with cp.async, 16 bytes at a time where the layer's rows allow it (V = 4),
 // kTileDepth - 1 items ahead, and the part of a window outside the layer (a
@@ -120,8 +122,8 @@ constexpr int kTileDepth = 4;
 constexpr int tile_py(int field) { return field <= 3 ? 8 : (field <= 7 ? 2 : 1); }
 
 // CTAs an SM should hold of the forward kernel: up to 50 weights fit in 72
-// registers, and seven CTAs are one wave of 1024 (3 x 64x64, batch 64: 13.9 us a
-// 10-step launch against 14.9 with five).
+// registers, and seven CTAs are one wave of 1024 (3 x 64x64, batch 64, with one chain a
+// stencil: 13.9 us a 10-step launch against 14.9 with five).
 constexpr int tile_ctas(int field, int py) { return field * field * py <= 50 ? 7 : 1; }
 
 template <int F, int PY, int V>
@@ -842,17 +844,20 @@ __global__ void __launch_bounds__(256) k_rate_dtau_partial(Dims D, const float* 
 
 // dtau_l = -(dt / tau_l^2) * sum of the layer's partials in block order, in double: the
 // parts of one sign or the other cancel, and 64 float additions in a row err by more
-// than everything before them (25 % of the error of dtau).
+// than everything before them (they made dtau err by 2.15e-7 against 64 bits, 1.72e-7
+// like this; 7 networks, 60 seeds).
 __global__ void __launch_bounds__(256) k_rate_dtau_final(Dims D, const float* __restrict__ tau,
                                                          const float* __restrict__ part,
                                                          float* __restrict__ dtau) {
     wait_for_previous();
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= D.L) return;
-    double s = 0.0;
-    for (int q = 0; q < kTauBlocks; ++q) s += part[(long long)l * kTauBlocks + q];
+    double s[4] = {};                                        // (chains of slow additions)
+    for (int q = 0; q < kTauBlocks; q += 4)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s[u] += part[(long long)l * kTauBlocks + q + u];
     const float tv = __ldg(tau + l);
-    dtau[l] = (float)s * (-D.dt / (tv * tv));
+    dtau[l] = (float)((s[0] + s[1]) + (s[2] + s[3])) * (-D.dt / (tv * tv));
 }
 
 // A segment's state of up to this many bytes stays in L2 and costs less than
@@ -999,7 +1004,7 @@ bool wide(const Dims& D, long long per_tile) { return tiles(D, tile_py(D.field))
 
 // Batch elements a CTA takes one after the other: all of them share its weights,
 // but a CTA for each of the 5 or more that an SM can hold comes first (3 x 64x64,
-// batch 64: 1.85 ms with one element to a CTA, 2.11 with two).
+// batch 64: 2.11 ms a training step with two elements to a CTA, 1.85 with one then).
 int batch_group(const Dims& D, unsigned ntiles) {
     return (int)std::max<long long>(1, (long long)ntiles * D.B / (5 * num_sms()));
 }

@@ -611,7 +611,10 @@ class RateNetwork:
     field x field connections between consecutive layers, a readout of the
     last layer, per-layer learnable time constants.  ``loss`` is a
     torch.autograd-aware call whose backward pass is the library's hand-written
-    adjoint with a checkpoint every ``checkpoint`` steps."""
+    adjoint with a checkpoint every ``checkpoint`` steps, or fewer in small
+    networks: segments of up to 64 MB are not cut more finely, so the workspace
+    (``workspace_bytes``) holds at least as many steps as that whatever
+    ``checkpoint`` is."""
 
     def __init__(self, layers=3, rows=64, cols=64, field=5, outputs=10, batch=64, steps=100,
                  dt=1.0, checkpoint=10):
