@@ -656,16 +656,20 @@ long Engine::step(long n) {
     auto t0 = std::chrono::steady_clock::now();
     SG_CUDA(cudaEventRecord(ev0, stream_));
     long i = 0;
-    if (alone_ && n > 0) {
+    // in pieces, between which an interrupt is seen (a piece of a small board takes 30 ms,
+    // its conversions to planes and back 20 us)
+    constexpr long kAlonePiece = 1 << 16;
+    while (alone_ && i < n && !interrupt_flag) {
+        const long piece = std::min(kAlonePiece, n - i);
         for (auto& lp : net_->layers) {
             const Model* m = find_model(lp->model);
             long k = 0;
             const std::string group = std::string(lp->model) + ".advance";
-            timed(group, 0, [&] { k = m->advance_alone(*state_, *state_->layer_state(lp.get()), n, stream_); });
+            timed(group, 0, [&] { k = m->advance_alone(*state_, *state_->layer_state(lp.get()), piece, stream_); });
             launches_ += k;
             if (profile_) prof_[group].launches += k;
         }
-        i = n;
+        i += piece;
     }
     while (n == 0 || i < n) {
         if (interrupt_flag) break;

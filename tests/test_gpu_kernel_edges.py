@@ -740,3 +740,27 @@ def test_report_of_moved_bytes(sg):
     net.get_neuron_data("s", "b", "voltage")
     net.get_weight_matrix("c")
     assert moved() == 4 * (21 + 35 * 21)
+
+
+# a whole run of a board goes on in pieces between which an interrupt is seen, as it is
+# between single steps (20 million steps of the ragged board take some 10 s)
+@pytest.mark.parametrize("rows,cols", [(40, 33), (64, 64)])
+def test_interrupt_of_whole_runs(sg, rows, cols):
+    import threading
+    import time
+    net = sg.Network(network([layer("b", "game_of_life", rows, cols)],
+                             [connection("c", "b", "b", "convergent", convolutional=True, **{
+                                 "weight config": {"type": "flat", "weight": 1.0, "diagonal": False},
+                                 "arborized config": {"field size": 3, "wrap": True}})]))
+    net.build_state()
+    net.run({"modules": []}, {"iterations": 10})
+    steps = 20_000_000
+    timer = threading.Timer(0.5, sg.interrupt_engine)
+    timer.start()
+    before = time.perf_counter()
+    report = net.run({"modules": []}, {"iterations": steps})
+    seconds = time.perf_counter() - before
+    timer.join()
+    assert 0 < int(report.properties["iterations"]) < steps and seconds < 5, (report.properties, seconds)
+    # and the next run is whole again
+    assert int(net.run({"modules": []}, {"iterations": 100_000}).properties["iterations"]) == 100_000
