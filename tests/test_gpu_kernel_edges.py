@@ -764,3 +764,26 @@ def test_interrupt_of_whole_runs(sg, rows, cols):
     assert 0 < int(report.properties["iterations"]) < steps and seconds < 5, (report.properties, seconds)
     # and the next run is whole again
     assert int(net.run({"modules": []}, {"iterations": 100_000}).properties["iterations"]) == 100_000
+
+
+# a step's kernels as programmatic dependents inside graphs: dendritic trees and second
+# order (copies among the kernels), sparse connections, every model and kind of structure,
+# learning on one stream and on the side one
+@pytest.mark.parametrize("name", ["base_all_types", "iz_c0_8", "iz_plastic", "iz_subset_columns", "iz_opcodes",
+                                  "dendrites", "second_order", "sparse", "models", "spnet", "oscillator_som", "nvm",
+                                  "structures", "debug"])
+def test_graphs_equal_plain_launches(sg, name):
+    import copy
+    from tests.golden.cases import CASES, Case
+    from tests.harness import compare, float_like_keys, run_library
+    base = CASES[name]
+    net = copy.deepcopy(base.net)
+    for i, l in enumerate(l for s in net["structures"] for l in s["layers"]):
+        if l["name"] in base.inputs:           # driven by noise in the place of a callback
+            l["init config"] = {"type": "poisson", "rate": 200, "value": 15, "seed": 60 + i}
+    case = Case(name, net, 75, base.seed, inject=base.inject, final=base.final, learning=base.learning)
+    plain = run_library(case, sg, extra_args={"graphs": False, "overlap learning": False})
+    for more in ({"overlap learning": False}, {"overlap learning": True}, {"overlap learning": True, "graphs": False}):
+        problems = compare(run_library(case, sg, extra_args=dict({"graphs": True}, **more)), plain,
+                           nan_keys=float_like_keys(case))
+        assert not problems, (more, problems[:3])
